@@ -1038,7 +1038,7 @@ static void enq_force(MdbCp* ctx, bool energy)
         launch_force_fp64(s, ctx->M, ctx->N, ctx->p.half_neigh, energy, ctx->ncl_cap, ctx->cnt,
             ctx->cx, ctx->ty, ctx->cutforcesq, ctx->list, lks(ctx), lcs(ctx), ctx->numneigh,
             ctx->cf, ctx->partials);
-        if (energy) ctx->energy_blocks = mdb_blocks((long long)ctx->ncl_cap * 4, 128);
+        if (energy) ctx->energy_blocks = force_fp64_blocks(ctx->ncl_cap);
     }
 }
 

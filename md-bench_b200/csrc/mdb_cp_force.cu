@@ -28,12 +28,28 @@ int force_blocks(int ncl_cap)
 // index as the reference does; half lists subtract the reaction from local j
 // slots with atomics (the reference drops ghost reactions: without MPI its
 // reverse communication does nothing).
+// A quarter of the listed pairs lie inside the cutoff, in other places for
+// every thread of a warp, so a branch on the cutoff runs the force arithmetic
+// (the FP64 pipe's work) for nearly every listed pair. The threads therefore
+// first only test distances and queue the j slots inside the cutoff, in list
+// order, in shared memory, and then work off their queues together: 55 of the
+// 228 listed pairs each, with few idle threads. FP64_QUEUE entries hold one row
+// of nearly every atom at LJ density; longer rows go in several turns. 97 -> 54
+// us per launch at 73,656 atoms (full lists), 85 -> 41 us at 4,000, 190 -> 173
+// us at 256,000 (half lists), where the broadcast loads of j positions (8 cycles
+// each for 32 threads of 32 bytes) bound the distance loop.
+static constexpr int FP64_THREADS = 64;
+static constexpr int FP64_QUEUE   = 88;
+
+int force_fp64_blocks(int ncl_cap) { return mdb_blocks((long long)ncl_cap * CP_M, FP64_THREADS); }
+
 template <int M, int N, bool HALF, bool ENERGY>
-__global__ void __launch_bounds__(CP_FORCE_THREADS) k_force_fp64(const int* __restrict__ cnt,
+__global__ void __launch_bounds__(FP64_THREADS) k_force_fp64(const int* __restrict__ cnt,
     const double4* __restrict__ cx, Types ty, double cutforcesq, const int* __restrict__ list,
     int ks, int cs, const int* __restrict__ numneigh, double4* cf, double* epart)
 {
     __shared__ double s_se[MDB_MAX_TYPES], s_s3[MDB_MAX_TYPES];
+    __shared__ int s_queue[FP64_QUEUE][FP64_THREADS];
     if (threadIdx.x < MDB_MAX_TYPES) {
         s_se[threadIdx.x] = ty.sqrt_eps[threadIdx.x];
         s_s3[threadIdx.x] = ty.sigma3[threadIdx.x];
@@ -43,62 +59,114 @@ __global__ void __launch_bounds__(CP_FORCE_THREADS) k_force_fp64(const int* __re
     const int ncl  = cnt[CP_NCL];
     const int nloc = ncl * M; // local slots (= ncj * N)
     double epot    = 0.0;
-    if (s < nloc) {
-        const double4 pi = cx[s];
-        const int ti     = slot_type(pi);
-        if (ti >= 0) {
-            const int ci = s / M, a = s - ci * M;
-            const int ci_cj0 = ci / (N / M);
-            const int ai     = a + M * (ci % (N / M));
-            const double se_i = s_se[ti], s3_i = s_s3[ti];
-            double fx = 0.0, fy = 0.0, fz = 0.0;
-            const int nn = numneigh[ci];
-            for (int k = 0; k < nn; k++) {
-                const int cj = __ldg(&list[(size_t)k * ks + (size_t)ci * cs]);
-                double fix = 0.0, fiy = 0.0, fiz = 0.0;
+    int* queue     = &s_queue[0][threadIdx.x];
+    // slots past the locals and padding slots have an empty row
+    double4 pi = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (s < nloc) pi = cx[s];
+    const int ti    = s < nloc ? slot_type(pi) : -1;
+    const bool real = ti >= 0;
+    const int ci = real ? s / M : 0, a = s - (s / M) * M;
+    const int nn     = real ? numneigh[ci] : 0;
+    const int ci_cj0 = ci / (N / M);
+    const int ai     = a + M * (ci % (N / M));
+    const double se_i = s_se[real ? ti : 0], s3_i = s_s3[real ? ti : 0];
+    const int* row  = list + (size_t)ci * cs;
+    const int nmax  = __reduce_max_sync(0xffffffffu, nn);
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    double fix = 0.0, fiy = 0.0, fiz = 0.0; // the entry's sum
+    int cj_next = nn > 0 ? __ldg(row) : 0;
+    for (int k = 0; k < nmax;) {
+        int n = 0;
+        // distances of whole entries while every thread's queue has room
+        do {
+            if (k < nn) {
+                const int cj = cj_next;
+                if (k + 1 < nn) cj_next = __ldg(&row[(size_t)(k + 1) * ks]);
+                double4 pj[N];
+#pragma unroll
+                for (int b = 0; b < N; b++)
+                    pj[b] = ldg4(&cx[cj * N + b]);
+                int first = 0x80000000; // marks an entry's first queued slot
 #pragma unroll
                 for (int b = 0; b < N; b++) {
-                    const bool cond = HALF ? (ci_cj0 != cj || ai < b) : (ci_cj0 != cj || ai != b);
-                    if (!cond) continue;
-                    const int sj     = cj * N + b;
-                    const double4 pj = ldg4(&cx[sj]);
-                    const double delx = pi.x - pj.x;
-                    const double dely = pi.y - pj.y;
-                    const double delz = pi.z - pj.z;
+                    const double delx = pi.x - pj[b].x;
+                    const double dely = pi.y - pj[b].y;
+                    const double delz = pi.z - pj[b].z;
                     const double rsq  = delx * delx + dely * dely + delz * delz;
-                    if (rsq < cutforcesq) {
-                        int tj            = slot_type(pj);
-                        tj                = tj < 0 ? 0 : tj;
-                        const double sig6 = s3_i * s_s3[tj];
-                        const double eps  = se_i * s_se[tj];
-                        const double sr2  = 1.0 / rsq;
-                        const double sr6  = sr2 * sr2 * sr2 * sig6;
-                        const double force = 48.0 * sr6 * (sr6 - 0.5) * sr2 * eps;
-                        if (HALF && sj < nloc) {
-                            atomicAdd(&cf[sj].x, -(delx * force));
-                            atomicAdd(&cf[sj].y, -(dely * force));
-                            atomicAdd(&cf[sj].z, -(delz * force));
-                        }
-                        fix += delx * force;
-                        fiy += dely * force;
-                        fiz += delz * force;
-                        if (ENERGY) {
-                            double e = 4.0 * eps * sr6 * (sr6 - 1.0);
-                            epot += (HALF && sj < nloc) ? e : 0.5 * e;
-                        }
+                    const bool cond =
+                        HALF ? (ci_cj0 != cj || ai < b) : (ci_cj0 != cj || ai != b);
+                    if (cond && rsq < cutforcesq) {
+                        queue[n * FP64_THREADS] = (cj * N + b) | first;
+                        first                   = 0;
+                        n++;
                     }
                 }
-                fx += fix;
-                fy += fiy;
-                fz += fiz;
             }
-            if (HALF) {
-                atomicAdd(&cf[s].x, fx);
-                atomicAdd(&cf[s].y, fy);
-                atomicAdd(&cf[s].z, fz);
-            } else {
-                cf[s] = make_double4(fx, fy, fz, 0.0);
+            k++;
+        } while (k < nmax && !__any_sync(0xffffffffu, n > FP64_QUEUE - N));
+        // two queued pairs at a time: their square distances, divisions and
+        // products overlap, the sums stay in list order
+        for (int q = 0; q < n; q += 2) {
+            int v[2];
+            double4 pj[2];
+            double tx[2], ty[2], tz[2];
+            v[0] = queue[q * FP64_THREADS];
+            v[1] = q + 1 < n ? queue[(q + 1) * FP64_THREADS] : v[0];
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+                pj[u] = ldg4(&cx[v[u] & 0x7fffffff]);
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const double delx = pi.x - pj[u].x;
+                const double dely = pi.y - pj[u].y;
+                const double delz = pi.z - pj[u].z;
+                const double rsq  = delx * delx + dely * dely + delz * delz;
+                int tj            = slot_type(pj[u]);
+                tj                = tj < 0 ? 0 : tj;
+                const double sig6 = s3_i * s_s3[tj];
+                const double eps  = se_i * s_se[tj];
+                const double sr2  = 1.0 / rsq;
+                const double sr6  = sr2 * sr2 * sr2 * sig6;
+                const double force = 48.0 * sr6 * (sr6 - 0.5) * sr2 * eps;
+                tx[u] = delx * force;
+                ty[u] = dely * force;
+                tz[u] = delz * force;
+                if (ENERGY && q + u < n) {
+                    const double e = 4.0 * eps * sr6 * (sr6 - 1.0);
+                    epot += (HALF && (v[u] & 0x7fffffff) < nloc) ? e : 0.5 * e;
+                }
             }
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (q + u >= n) break;
+                const int sj = v[u] & 0x7fffffff;
+                if (HALF && sj < nloc) {
+                    atomicAdd(&cf[sj].x, -tx[u]);
+                    atomicAdd(&cf[sj].y, -ty[u]);
+                    atomicAdd(&cf[sj].z, -tz[u]);
+                }
+                if (v[u] < 0) {
+                    fx += fix;
+                    fy += fiy;
+                    fz += fiz;
+                    fix = fiy = fiz = 0.0;
+                }
+                fix += tx[u];
+                fiy += ty[u];
+                fiz += tz[u];
+            }
+        }
+    }
+    fx += fix;
+    fy += fiy;
+    fz += fiz;
+    if (real) {
+        if (HALF) {
+            atomicAdd(&cf[s].x, fx);
+            atomicAdd(&cf[s].y, fy);
+            atomicAdd(&cf[s].z, fz);
+        } else {
+            cf[s] = make_double4(fx, fy, fz, 0.0);
         }
     }
     if (ENERGY) {
@@ -112,7 +180,7 @@ static void run_fp64(cudaStream_t s, int blocks, const int* cnt, const double4* 
     const Types& ty, double cutforcesq, const int* list, int ks, int cs, const int* numneigh,
     double4* cf, double* epart)
 {
-    k_force_fp64<4, N, HALF, ENERGY><<<blocks, CP_FORCE_THREADS, 0, s>>>(cnt, cx, ty, cutforcesq,
+    k_force_fp64<4, N, HALF, ENERGY><<<blocks, FP64_THREADS, 0, s>>>(cnt, cx, ty, cutforcesq,
         list, ks, cs, numneigh, cf, epart);
 }
 
@@ -121,9 +189,9 @@ void launch_force_fp64(cudaStream_t s, int M, int N, int half, int energy, int n
     int ks, int cs, const int* numneigh, double4* cf, double* epart)
 {
     (void)M;
-    // one thread per slot: ncl_cap * 4 threads; energy partials sized by
-    // force_blocks (ncl_cap * 32 threads) cover it
-    int blocks = mdb_blocks((long long)ncl_cap * 4, CP_FORCE_THREADS);
+    // one thread per slot; the energy partials' size (force_blocks: ncl_cap * 32
+    // threads) covers the blocks
+    const int blocks = force_fp64_blocks(ncl_cap);
     if (N == 4) {
         if (half) energy ? run_fp64<4, true, true>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart)
                          : run_fp64<4, true, false>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart);

@@ -176,6 +176,8 @@ void launch_prune(cudaStream_t s, int M, int N, int ncl_cap, const int* cnt, con
 
 // force / integrate / thermo (mdb_cp_force.cu)
 int force_blocks(int ncl_cap);
+// blocks (= energy partials) of an FP64 force launch
+int force_fp64_blocks(int ncl_cap);
 void launch_force_fp64(cudaStream_t s, int M, int N, int half, int energy, int ncl_cap,
     const int* cnt, const double4* cx, const Types& ty, double cutforcesq, const int* list,
     int ks, int cs, const int* numneigh, double4* cf, double* epart);
