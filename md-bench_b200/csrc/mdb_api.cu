@@ -40,7 +40,7 @@ struct MdbCtx {
 
     BinGeom g;
     std::vector<int> stencil;
-    std::vector<int4> stencil4;
+    std::vector<int4> stencil_rows; // {flat offset of the middle bin, dy, dz, bins to a side}
     LJTable tab;
     LJTableF tabf;
     CellFrame cf;
@@ -60,11 +60,11 @@ struct MdbCtx {
     int *ghost_cnt = nullptr, *ghost_off = nullptr;
     int *atom_bin = nullptr, *atom_slot = nullptr;
     int *bin_count = nullptr, *bin_start = nullptr, *bin_atoms = nullptr;
-    double4* bin_x = nullptr; // positions in bin order, atom index bits in .w
-    float4* bin_xf = nullptr; // the same rounded to FP32 (list build prefilter)
+    int2* bin_jq = nullptr; // {atom index, cell} in bin order
+    float* binf  = nullptr; // FP32 positions in bin order: x, then y, then z
     int *bin_lcount = nullptr, *loc_start = nullptr; // locals per bin, their offsets
     int* local_order = nullptr; // local atoms bin by bin (the order sortAtom gives)
-    int4* stencil_d  = nullptr;                      // {flat offset, dx, dy, dz}
+    int4* rows_d = nullptr; // the stencil's runs of bins along x (stencil_rows)
     int *numneigh = nullptr, *neighbors = nullptr;
     int* counters = nullptr;
     int* scan_scratch = nullptr;
@@ -80,8 +80,7 @@ struct MdbCtx {
     int *eam_cutlist = nullptr, *eam_ncut = nullptr;
     double* stage  = nullptr; // 9 * nlocal doubles: AoS x, v, f for host transfers
     int* stage_t   = nullptr; // nlocal types
-    double *eam_frho = nullptr, *eam_rhor = nullptr, *eam_z2r = nullptr;
-    float* eam_frho32 = nullptr;
+    double4 *eam_frho = nullptr, *eam_rhor = nullptr, *eam_z2r = nullptr; // see EamDev
     float4 *eam_dens32 = nullptr, *eam_pair32 = nullptr;
     EamDev eam;
     double eam_cut = 0;
@@ -230,16 +229,19 @@ static int setup_bins(MdbCtx* ctx)
     if (mb > (1LL << 30)) return fail(ctx, MDB_ERR_ARG, "bin grid too large");
     g.mbins = (int)mb;
     ctx->stencil.clear();
-    ctx->stencil4.clear();
+    ctx->stencil_rows.clear();
     double cutsq = cut * cut;
     for (int k = -nextz; k <= nextz; k++)
-        for (int j = -nexty; j <= nexty; j++)
+        for (int j = -nexty; j <= nexty; j++) {
+            const int row = k * g.mbiny * g.mbinx + j * g.mbinx;
+            int side      = -1; // bindist grows with |i|: the run is -side..side
             for (int i = -nextx; i <= nextx; i++)
                 if (bindist(g, i, j, k) < cutsq) {
-                    int flat = k * g.mbiny * g.mbinx + j * g.mbinx + i;
-                    ctx->stencil.push_back(flat);
-                    ctx->stencil4.push_back(make_int4(flat, i, j, k));
+                    ctx->stencil.push_back(row + i);
+                    side = std::max(side, i);
                 }
+            if (side >= 0) ctx->stencil_rows.push_back(make_int4(row, j, k, side));
+        }
     g.nstencil = (int)ctx->stencil.size();
     if (g.nstencil > MDB_MAX_STENCIL) return fail(ctx, MDB_ERR_ARG, "stencil too large");
     g.xlo = fabs(0.0 - g.pad_x * g.binsizex) + 1e-9;
@@ -386,7 +388,7 @@ extern "C" int mdb_create(const MdbParams* params, MdbCtx** out)
             goto bad;
         }
         if ((e = dalloc(&ctx->counters, CNT_SLOTS)) != cudaSuccess ||
-            (e = dalloc(&ctx->stencil_d, ctx->g.nstencil)) != cudaSuccess ||
+            (e = dalloc(&ctx->rows_d, ctx->stencil_rows.size())) != cudaSuccess ||
             (e = dalloc(&ctx->bin_count, ctx->g.mbins)) != cudaSuccess ||
             (e = dalloc(&ctx->bin_start, ctx->g.mbins + 1)) != cudaSuccess ||
             (e = cudaMallocHost((void**)&ctx->h_counters, CNT_SLOTS * sizeof(int))) !=
@@ -400,7 +402,7 @@ extern "C" int mdb_create(const MdbParams* params, MdbCtx** out)
             goto bad;
         }
         cudaMemset(ctx->counters, 0, CNT_SLOTS * sizeof(int));
-        cudaMemcpy(ctx->stencil_d, ctx->stencil4.data(), sizeof(int4) * ctx->g.nstencil,
+        cudaMemcpy(ctx->rows_d, ctx->stencil_rows.data(), sizeof(int4) * ctx->stencil_rows.size(),
             cudaMemcpyHostToDevice);
         if ((e = cudaGetLastError()) != cudaSuccess) {
             rc = fail(ctx, MDB_ERR_CUDA, "setup copy", e);
@@ -434,8 +436,8 @@ static void free_atom_buffers(MdbCtx* ctx)
     dfree(ctx->atom_bin);
     dfree(ctx->atom_slot);
     dfree(ctx->bin_atoms);
-    dfree(ctx->bin_x);
-    dfree(ctx->bin_xf);
+    dfree(ctx->bin_jq);
+    dfree(ctx->binf);
     dfree(ctx->numneigh);
     dfree(ctx->neighbors);
     dfree(ctx->eam_cutlist);
@@ -458,7 +460,7 @@ extern "C" int mdb_destroy(MdbCtx* ctx)
     drop_graphs(ctx);
     free_atom_buffers(ctx);
     dfree(ctx->counters);
-    dfree(ctx->stencil_d);
+    dfree(ctx->rows_d);
     dfree(ctx->bin_count);
     dfree(ctx->bin_start);
     dfree(ctx->bin_lcount);
@@ -466,7 +468,6 @@ extern "C" int mdb_destroy(MdbCtx* ctx)
     dfree(ctx->eam_frho);
     dfree(ctx->eam_rhor);
     dfree(ctx->eam_z2r);
-    dfree(ctx->eam_frho32);
     dfree(ctx->eam_dens32);
     dfree(ctx->eam_pair32);
     if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
@@ -490,29 +491,33 @@ static int alloc_ghost_sized(MdbCtx* ctx, int ghost_cap)
     drop_graphs(ctx);
     int nall = ctx->nlocal + ghost_cap;
     double4* nx;
-    CK(dalloc(&nx, nall));
+    CK(dalloc(&nx, (size_t)nall + 1));
     if (ctx->x) {
         CK(cudaMemcpyAsync(nx, ctx->x, sizeof(double4) * ctx->nlocal, cudaMemcpyDeviceToDevice, s));
         CK(cudaStreamSynchronize(s));
     }
     dfree(ctx->x);
     ctx->x = nx;
+    const double4 far64 = make_double4(MDB_FAR, MDB_FAR, MDB_FAR, 0.0); // the dummy atom
+    CK(cudaMemcpyAsync(nx + nall, &far64, sizeof far64, cudaMemcpyHostToDevice, s));
     if (ctx->mixed) {
         if ((long long)nall > (long long)MDB_IDX_MASK)
             return fail(ctx, MDB_ERR_ARG, "mixed path limited to 2^25 atoms including ghosts");
         // cells and relative positions are recomputed by every rebuild
         dfree(ctx->xr);
         dfree(ctx->qcell);
-        CK(dalloc(&ctx->xr, nall));
+        CK(dalloc(&ctx->xr, (size_t)nall + 1));
         CK(dalloc(&ctx->qcell, nall));
+        const float4 far32 = make_float4((float)MDB_FAR, (float)MDB_FAR, (float)MDB_FAR, 0.0f);
+        CK(cudaMemcpyAsync(ctx->xr + nall, &far32, sizeof far32, cudaMemcpyHostToDevice, s));
     }
     dfree(ctx->border_map);
     dfree(ctx->pbc_code);
     dfree(ctx->atom_bin);
     dfree(ctx->atom_slot);
     dfree(ctx->bin_atoms);
-    dfree(ctx->bin_x);
-    dfree(ctx->bin_xf);
+    dfree(ctx->bin_jq);
+    dfree(ctx->binf);
     dfree(ctx->fp);
     dfree(ctx->xe);
     CK(dalloc(&ctx->border_map, ghost_cap));
@@ -521,8 +526,8 @@ static int alloc_ghost_sized(MdbCtx* ctx, int ghost_cap)
     CK(dalloc(&ctx->atom_bin, nall));
     CK(dalloc(&ctx->atom_slot, nall));
     CK(dalloc(&ctx->bin_atoms, nall));
-    CK(dalloc(&ctx->bin_x, nall));
-    CK(dalloc(&ctx->bin_xf, nall));
+    CK(dalloc(&ctx->bin_jq, nall));
+    CK(dalloc(&ctx->binf, 3 * (size_t)bin_stride(nall)));
     if (ctx->p.force_field == MDB_FF_EAM) CK(dalloc(&ctx->fp, nall));
     if (ctx->p.force_field == MDB_FF_EAM && ctx->mixed) CK(dalloc(&ctx->xe, nall));
     ctx->ghost_cap   = ghost_cap;
@@ -538,7 +543,7 @@ static int alloc_list(MdbCtx* ctx, int maxneighs)
     drop_graphs(ctx);
     dfree(ctx->neighbors);
     dfree(ctx->eam_cutlist);
-    CK(dalloc(&ctx->neighbors, (size_t)maxneighs * ctx->ld));
+    CK(dalloc(&ctx->neighbors, list_ints(maxneighs, ctx->ld)));
     if (ctx->p.force_field == MDB_FF_EAM && ctx->mixed)
         CK(dalloc(&ctx->eam_cutlist, (size_t)maxneighs * ctx->ld));
     ctx->maxneighs = maxneighs;
@@ -610,7 +615,7 @@ extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const dou
         ctx->scan_scratch_n = nscan;
         CK(dalloc(&ctx->scan_scratch, nscan));
         ctx->npart = std::max(std::max(force_partial_blocks(cap), ke_partial_blocks(cap)),
-            eam_mixed_blocks(cap));
+            ctx->p.force_field == MDB_FF_EAM ? eam_fp64_blocks(cap) : 1);
         CK(dalloc(&ctx->partials, 3 * (size_t)ctx->npart));
         ctx->nred_slots = 64;
         CK(dalloc(&ctx->red, 4 * (size_t)ctx->nred_slots));
@@ -717,7 +722,7 @@ static void enq_force(MdbCtx* ctx, bool energy)
                 ctx->eam_cutlist, ctx->eam_ncut, ctx->fp, ctx->xe, ctx->fx, ctx->fy, ctx->fz, ep0,
                 ep1);
         } else {
-            launch_eam_fp64(s, energy, n, ctx->ghost_cap, nullptr,ctx->x,
+            launch_eam_fp64(s, energy, n, ctx->ghost_cap, ctx->x,
                 ctx->numneigh, ctx->neighbors, ctx->ld, ctx->cutforcesq, ctx->eam,
                 ctx->border_map, ctx->counters, ctx->fp, ctx->fx, ctx->fy, ctx->fz, ep0, ep1);
         }
@@ -730,10 +735,10 @@ static void enq_force(MdbCtx* ctx, bool energy)
     }
     if (ctx->mixed)
         launch_lj_mixed(s, ctx->p.precision == MDB_PREC_MIXED_COMP, ctx->p.half_neigh, energy, n,
-            nullptr, ctx->xr, ctx->shift, ctx->numneigh, ctx->neighbors, ctx->ld,
+            ctx->xr, ctx->shift, ctx->numneigh, ctx->neighbors, ctx->ld,
             (float)ctx->cutforcesq, ctx->tabf, ctx->fx, ctx->fy, ctx->fz, ep0);
     else
-        launch_lj_fp64(s, ctx->p.half_neigh, energy, n, nullptr, ctx->x, ctx->numneigh,
+        launch_lj_fp64(s, ctx->p.half_neigh, energy, n, ctx->x, ctx->numneigh,
             ctx->neighbors, ctx->ld, ctx->cutforcesq, ctx->tab, ctx->fx, ctx->fy, ctx->fz, ep0);
 }
 
@@ -768,14 +773,13 @@ static void enq_list(MdbCtx* ctx)
     scan_exclusive(ctx->bin_lcount, ctx->loc_start, ctx->g.mbins, ctx->scan_scratch, s);
     launch_bin_scatter(s, ctx->nlocal, ctx->nall_cap, ctx->atom_bin, ctx->atom_slot,
         ctx->bin_start, ctx->bin_atoms, ctx->counters);
-    launch_bin_sort(s, ctx->g.mbins, ctx->bin_start, ctx->bin_atoms, ctx->loc_start,
-        ctx->local_order);
-    launch_bin_positions(s, ctx->nall_cap, ctx->g.mbins, ctx->x, ctx->bin_start, ctx->bin_atoms,
-        ctx->bin_x, ctx->bin_xf);
-    launch_build_list(s, ctx->nlocal, ctx->x, ctx->g, ctx->stencil_d, ctx->atom_bin,
-        ctx->bin_start, ctx->bin_x, ctx->bin_xf, ctx->cutneighsq, ctx->list_margin,
-        ctx->p.half_neigh, ctx->maxneighs, ctx->ld, ctx->neighbors, ctx->numneigh,
-        ctx->counters, ctx->mixed ? ctx->qcell : nullptr);
+    launch_bin_order(s, ctx->nlocal, ctx->nall_cap, ctx->g.mbins, ctx->x, ctx->atom_bin,
+        ctx->bin_start, ctx->bin_atoms, ctx->loc_start, ctx->mixed ? ctx->qcell : nullptr,
+        ctx->bin_jq, ctx->binf, ctx->local_order);
+    launch_build_list(s, ctx->nlocal, ctx->nall_cap, ctx->local_order, ctx->loc_start, ctx->x,
+        ctx->g, (int)ctx->stencil_rows.size(), ctx->rows_d, ctx->atom_bin, ctx->bin_start, ctx->bin_jq,
+        ctx->binf, ctx->cutneighsq, ctx->list_margin, ctx->p.half_neigh, ctx->maxneighs, ctx->ld,
+        ctx->neighbors, ctx->numneigh, ctx->counters, ctx->mixed ? ctx->qcell : nullptr);
 }
 
 static void clear_rebuild_counters(MdbCtx* ctx)
@@ -897,8 +901,8 @@ static int sort_atoms(MdbCtx* ctx)
     scan_exclusive(ctx->bin_lcount, ctx->loc_start, ctx->g.mbins, ctx->scan_scratch, s);
     launch_bin_scatter(s, n, ctx->nall_cap, ctx->atom_bin, ctx->atom_slot, ctx->bin_start,
         ctx->bin_atoms, ctx->counters);
-    launch_bin_sort(s, ctx->g.mbins, ctx->bin_start, ctx->bin_atoms, ctx->loc_start,
-        ctx->local_order);
+    launch_bin_order(s, n, ctx->nall_cap, ctx->g.mbins, ctx->x, ctx->atom_bin, ctx->bin_start,
+        ctx->bin_atoms, ctx->loc_start, nullptr, ctx->bin_jq, ctx->binf, ctx->local_order);
     // stage: 9 n doubles; positions as double4 [0, 4n), velocities [4n, 7n)
     double4* sx = reinterpret_cast<double4*>(ctx->stage);
     double* sv  = ctx->stage + 4 * (size_t)n;
@@ -1045,10 +1049,9 @@ static void enq_thermo(MdbCtx* ctx, int slot, bool with_pe)
         ctx->partials + 2 * (size_t)ctx->npart);
     launch_reduce_partials(s, nke, ctx->partials + 2 * (size_t)ctx->npart, r + 0);
     if (with_pe) {
-        // the mixed EAM passes write eam_mixed_blocks partials, the rest one
-        // per block of the force kernels
-        int nf = ctx->p.force_field == MDB_FF_EAM && ctx->mixed ? eam_mixed_blocks(owned(ctx))
-                                                               : force_partial_blocks(owned(ctx));
+        const int nf = ctx->p.force_field != MDB_FF_EAM ? force_partial_blocks(owned(ctx))
+                       : ctx->mixed                     ? eam_mixed_blocks(owned(ctx))
+                                                        : eam_fp64_blocks(owned(ctx));
         launch_reduce_partials(s, nf, ctx->partials, r + 1);
         if (ctx->p.force_field == MDB_FF_EAM)
             launch_reduce_partials(s, nf, ctx->partials + ctx->npart, r + 2);
@@ -1126,11 +1129,10 @@ extern "C" int mdb_set_neighbor_list(MdbCtx* ctx, const int* numneigh, const int
         int rc = alloc_list(ctx, maxn);
         if (rc) return rc;
     }
-    // k-major on the device: entry k of atom i at k * ld + i
-    std::vector<int> all((size_t)ctx->maxneighs * ctx->ld, 0);
+    std::vector<int> all(list_ints(ctx->maxneighs, ctx->ld), ctx->nall_cap); // the dummy atom
     for (int i = 0; i < n; i++)
         for (int k = 0; k < numneigh[i]; k++)
-            all[(size_t)k * ctx->ld + i] = neighbors[(size_t)i * ld + k];
+            all[list_at(k, ctx->ld, i)] = neighbors[(size_t)i * ld + k];
     CK(cudaStreamSynchronize(ctx->s));
     CK(cudaMemcpy(ctx->neighbors, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ctx->numneigh, numneigh, sizeof(int) * n, cudaMemcpyHostToDevice));
@@ -1302,48 +1304,41 @@ extern "C" int mdb_set_eam(MdbCtx* ctx, const MdbEamTables* t)
     CK(cudaSetDevice(ctx->dev));
     CK(cudaStreamSynchronize(ctx->s));
     drop_graphs(ctx);
-    auto relayout = [](const double* src, int n, int tot, std::vector<double>& d,
-                        std::vector<float>& f) {
-        int rows = std::min(n + 1, tot / 7);
-        d.assign((size_t)(n + 1) * 8, 0.0);
-        f.assign((size_t)(n + 1) * 8, 0.0f);
-        for (int m = 0; m < rows; m++)
-            for (int c = 0; c < 7; c++) {
-                d[(size_t)m * 8 + c] = src[(size_t)m * 7 + c];
-                f[(size_t)m * 8 + c] = (float)src[(size_t)m * 7 + c];
-            }
+    // rows of a table of n grid points (1-based, 7 coefficients each, see EamDev)
+    auto relayout = [](const double* src, int n, int tot) {
+        std::vector<double4> d(2 * ((size_t)n + 1), make_double4(0.0, 0.0, 0.0, 0.0));
+        for (int m = 0; m < std::min(n + 1, tot / 7); m++) {
+            const double* c     = src + (size_t)m * 7;
+            d[2 * (size_t)m]     = make_double4(c[3], c[4], c[5], c[6]);
+            d[2 * (size_t)m + 1] = make_double4(c[0], c[1], c[2], 0.0);
+        }
+        return d;
     };
-    std::vector<double> fr, rr, zr;
-    std::vector<float> fr32, rr32, zr32;
-    relayout(t->frho_spline, t->nrho, t->nrho_tot, fr, fr32);
-    relayout(t->rhor_spline, t->nr, t->nr_tot, rr, rr32);
-    relayout(t->z2r_spline, t->nr, t->nr_tot, zr, zr32);
+    const std::vector<double4> fr = relayout(t->frho_spline, t->nrho, t->nrho_tot);
+    const std::vector<double4> rr = relayout(t->rhor_spline, t->nr, t->nr_tot);
+    const std::vector<double4> zr = relayout(t->z2r_spline, t->nr, t->nr_tot);
     // the mixed passes' rows (see EamDev)
     const size_t nrow = (size_t)t->nr + 1;
     std::vector<float4> dens32(nrow), pair32(2 * nrow);
     for (size_t m = 0; m < nrow; m++) {
-        const float* r = &rr32[m * 8];
-        const float* z = &zr32[m * 8];
-        dens32[m]         = make_float4(r[3], r[4], r[5], r[6]);
-        pair32[2 * m]     = make_float4(z[3], z[4], z[5], z[6]);
-        pair32[2 * m + 1] = make_float4(r[0], r[1], r[2], z[0]);
+        const double4 &r = rr[2 * m], &rd = rr[2 * m + 1], &z = zr[2 * m], &zd = zr[2 * m + 1];
+        dens32[m]         = make_float4((float)r.x, (float)r.y, (float)r.z, (float)r.w);
+        pair32[2 * m]     = make_float4((float)z.x, (float)z.y, (float)z.z, (float)z.w);
+        pair32[2 * m + 1] = make_float4((float)rd.x, (float)rd.y, (float)rd.z, (float)zd.x);
     }
     dfree(ctx->eam_frho);
     dfree(ctx->eam_rhor);
     dfree(ctx->eam_z2r);
-    dfree(ctx->eam_frho32);
     dfree(ctx->eam_dens32);
     dfree(ctx->eam_pair32);
     CK(dalloc(&ctx->eam_frho, fr.size()));
     CK(dalloc(&ctx->eam_rhor, rr.size()));
     CK(dalloc(&ctx->eam_z2r, zr.size()));
-    CK(dalloc(&ctx->eam_frho32, fr32.size()));
     CK(dalloc(&ctx->eam_dens32, dens32.size()));
     CK(dalloc(&ctx->eam_pair32, pair32.size()));
-    CK(cudaMemcpy(ctx->eam_frho, fr.data(), fr.size() * 8, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->eam_rhor, rr.data(), rr.size() * 8, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->eam_z2r, zr.data(), zr.size() * 8, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->eam_frho32, fr32.data(), fr32.size() * 4, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(ctx->eam_frho, fr.data(), fr.size() * sizeof(double4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(ctx->eam_rhor, rr.data(), rr.size() * sizeof(double4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(ctx->eam_z2r, zr.data(), zr.size() * sizeof(double4), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ctx->eam_dens32, dens32.data(), dens32.size() * sizeof(float4),
         cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ctx->eam_pair32, pair32.data(), pair32.size() * sizeof(float4),
@@ -1355,7 +1350,6 @@ extern "C" int mdb_set_eam(MdbCtx* ctx, const MdbEamTables* t)
     ctx->eam.frho   = ctx->eam_frho;
     ctx->eam.rhor   = ctx->eam_rhor;
     ctx->eam.z2r    = ctx->eam_z2r;
-    ctx->eam.frho32 = ctx->eam_frho32;
     ctx->eam.dens32 = ctx->eam_dens32;
     ctx->eam.pair32 = ctx->eam_pair32;
     ctx->have_eam   = true;
@@ -1418,24 +1412,19 @@ extern "C" int mdb_get_neighbor_list(MdbCtx* ctx, int* numneigh, int* neighbors,
 {
     NEED_ATOMS();
     if (!ctx->have_list) return fail(ctx, MDB_ERR_STATE, "no neighbour list");
-    // row i (column i of the k-major list) belongs to atom i. Mixed-path
-    // entries carry a cell-offset code above the index bits, masked off here.
     int n = ctx->nlocal;
-    std::vector<int> nn(n), order(n);
+    std::vector<int> nn(n);
     CK(cudaStreamSynchronize(ctx->s));
     CK(cudaMemcpy(nn.data(), ctx->numneigh, sizeof(int) * n, cudaMemcpyDeviceToHost));
-    for (int t = 0; t < n; t++)
-        order[t] = t;
-    if (numneigh)
-        for (int t = 0; t < n; t++)
-            numneigh[order[t]] = nn[t];
+    if (numneigh) std::copy(nn.begin(), nn.end(), numneigh);
     if (neighbors) {
-        const int mask = ctx->mixed ? MDB_IDX_MASK : -1;
-        std::vector<int> all((size_t)ctx->maxneighs * ctx->ld);
+        const int shift = ctx->mixed ? MDB_CODE_BITS : 0; // past the cell-offset code
+        std::vector<int> all(list_ints(ctx->maxneighs, ctx->ld));
         CK(cudaMemcpy(all.data(), ctx->neighbors, sizeof(int) * all.size(), cudaMemcpyDeviceToHost));
-        for (int t = 0; t < n; t++)
-            for (int k = 0; k < nn[t] && k < ld && k < ctx->maxneighs; k++)
-                neighbors[(size_t)order[t] * ld + k] = all[(size_t)k * ctx->ld + t] & mask;
+        for (int i = 0; i < n; i++)
+            for (int k = 0; k < nn[i] && k < ld && k < ctx->maxneighs; k++)
+                neighbors[(size_t)i * ld + k] =
+                    (int)((unsigned)all[list_at(k, ctx->ld, i)] >> shift);
     }
     return MDB_OK;
 }

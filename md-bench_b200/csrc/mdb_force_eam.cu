@@ -3,9 +3,9 @@
 // (2) fp copied to the ghosts through the ghost map (the mid-step halo),
 // (3) pair forces from rho', phi' and fp_i + fp_j.
 //
-// Thread t handles atom t (or order[t]). Spline tables are re-laid out as rows of 8
-// coefficients (one 64-byte row per grid point instead of 56 bytes) so a row
-// is two aligned sectors.
+// Thread t handles atom t. Spline tables are re-laid out as rows of 8
+// coefficients, 3..6 (the value) then 0..2 (the derivative), so each half is one
+// aligned sector in one 256-bit load.
 // FP64 path: -fmad=false, bit-identical to the reference's strict build.
 // Mixed path: pair terms and spline rows in FP32 on cell-relative FP32
 // positions (see mdb_force_lj.cu); the density (embedding) sum, F'(rho) and
@@ -26,21 +26,43 @@ __device__ __forceinline__ void ldg_row32(const float4* p, float4& a, float4& b)
 }
 static constexpr int EUNROLL     = 4;
 
+// FP64 passes: a row's sums must add its pairs one after the other, in list
+// order, for bit-identical results, but everything else of a pair is
+// independent. So 8 threads share an atom, one entry of a tile each, and leave
+// their terms in shared memory, where one thread per sum adds them up in order.
+// (One thread per atom spent its time waiting on its own chain of dependent
+// square roots, divisions and table rows, at 31 blocks for 4,000 atoms.)
+// A pair outside the cutoff adds an exact zero. Both passes: 85 -> 20 us at 3,960
+// atoms, 302 -> 211 us at 131,072, where the scattered table rows bound them (one
+// 32-byte load per half row; 307 us with eight-byte loads of the coefficients).
+static constexpr int EAM64_ATOMS = EAM_THREADS / MDB_TILE; // atoms per block
+
+int eam_fp64_blocks(int nlocal) { return mdb_blocks(nlocal, EAM64_ATOMS); }
+
 template <bool ENERGY>
 __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_fp64(int nlocal,
-    const int* __restrict__ order, const double4* __restrict__ x,
-    const int* __restrict__ numneigh, const int* __restrict__ neighbors, int ld,
-    double cutforcesq, EamDev e, double* __restrict__ fp, double* __restrict__ epart)
+    const double4* __restrict__ x, const int* __restrict__ numneigh,
+    const int* __restrict__ neighbors, int ld, double cutforcesq, EamDev e,
+    double* __restrict__ fp, double* __restrict__ epart)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double s_term[EAM64_ATOMS][MDB_TILE + 1];
+    const int g = threadIdx.x / MDB_TILE, u = threadIdx.x % MDB_TILE;
+    const int i = blockIdx.x * EAM64_ATOMS + g;
     double eng  = 0.0;
-    if (t < nlocal) {
-        const int i      = order ? order[t] : t;
-        const double4 xi = x[i];
-        const int n      = numneigh[t];
-        const int* nb    = neighbors + t;
-        double rhoi      = 0.0;
-        auto pair        = [&](const double4& xj) {
+    const int ia     = i < nlocal ? i : 0;
+    const double4 xi = x[ia];
+    const int n      = i < nlocal ? numneigh[ia] : 0;
+    const int* nb    = neighbors + list_at(0, ld, ia) + u;
+    const int nmax   = __reduce_max_sync(0xffffffffu, n);
+    double rhoi      = 0.0;
+    int j            = n > 0 ? __ldcs(nb) : -1;
+    for (int k = 0; k < nmax; k += MDB_TILE) {
+        double term = 0.0;
+        const int jn = k + MDB_TILE < n
+                           ? __ldcs(nb + (size_t)(k / MDB_TILE + 1) * ld * MDB_TILE)
+                           : -1;
+        if (j >= 0) {
+            const double4 xj = ldg4(x + j);
             double delx = xi.x - xj.x;
             double dely = xi.y - xj.y;
             double delz = xi.z - xj.z;
@@ -51,35 +73,30 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_fp64(int nlocal,
                 m        = m < e.nr - 1 ? m : e.nr - 1;
                 p -= m;
                 p               = p < 1.0 ? p : 1.0;
-                const double* c = e.rhor + 8 * m;
-                rhoi += ((__ldg(c + 3) * p + __ldg(c + 4)) * p + __ldg(c + 5)) * p + __ldg(c + 6);
+                const double4 c = ldg4(e.rhor + 2 * m);
+                term            = ((c.x * p + c.y) * p + c.z) * p + c.w;
             }
-        };
-        int k = 0;
-        for (; k + EUNROLL <= n; k += EUNROLL) {
-            int j[EUNROLL];
-            double4 xj[EUNROLL];
-#pragma unroll
-            for (int u = 0; u < EUNROLL; u++)
-                j[u] = __ldcs(nb + (size_t)(k + u) * ld);
-#pragma unroll
-            for (int u = 0; u < EUNROLL; u++)
-                xj[u] = ldg4(x + j[u]);
-#pragma unroll
-            for (int u = 0; u < EUNROLL; u++)
-                pair(xj[u]);
         }
-        for (; k < n; k++)
-            pair(ldg4(x + __ldcs(nb + (size_t)k * ld)));
+        s_term[g][u] = term;
+        __syncwarp();
+        if (u == 0) {
+#pragma unroll
+            for (int q = 0; q < MDB_TILE; q++)
+                rhoi += s_term[g][q];
+        }
+        __syncwarp();
+        j = jn;
+    }
+    if (u == 0 && i < nlocal) {
         double p = 1.0 * rhoi * e.rdrho + 1.0;
         int m    = (int)(p);
         m        = m < e.nrho - 1 ? m : e.nrho - 1;
         m        = m > 1 ? m : 1;
         p -= m;
         p               = p < 1.0 ? p : 1.0;
-        const double* c = e.frho + 8 * m;
-        fp[i]           = (__ldg(c + 0) * p + __ldg(c + 1)) * p + __ldg(c + 2);
-        if (ENERGY) eng = ((__ldg(c + 3) * p + __ldg(c + 4)) * p + __ldg(c + 5)) * p + __ldg(c + 6);
+        const double4 c = ldg4(e.frho + 2 * m), d = ldg4(e.frho + 2 * m + 1);
+        fp[i]           = (d.x * p + d.y) * p + d.z;
+        if (ENERGY) eng = ((c.x * p + c.y) * p + c.z) * p + c.w;
     }
     if (ENERGY) {
         double s = block_sum(eng);
@@ -97,21 +114,30 @@ __global__ void k_eam_fp_ghost(int nlocal, double* __restrict__ fp,
 
 template <bool ENERGY>
 __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_fp64(int nlocal,
-    const int* __restrict__ order, const double4* __restrict__ x,
-    const int* __restrict__ numneigh, const int* __restrict__ neighbors, int ld,
-    double cutforcesq, EamDev e, const double* __restrict__ fp, double* __restrict__ fx,
-    double* __restrict__ fy, double* __restrict__ fz, double* __restrict__ epart)
+    const double4* __restrict__ x, const int* __restrict__ numneigh,
+    const int* __restrict__ neighbors, int ld, double cutforcesq, EamDev e,
+    const double* __restrict__ fp, double* __restrict__ fx, double* __restrict__ fy,
+    double* __restrict__ fz, double* __restrict__ epart)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double s_term[EAM64_ATOMS][3][MDB_TILE + 1];
+    const int g = threadIdx.x / MDB_TILE, u = threadIdx.x % MDB_TILE;
+    const int i = blockIdx.x * EAM64_ATOMS + g;
     double eng  = 0.0;
-    if (t < nlocal) {
-        const int i      = order ? order[t] : t;
-        const double4 xi = x[i];
-        const int n      = numneigh[t];
-        const int* nb    = neighbors + t;
-        const double fpi = fp[i];
-        double fix = 0.0, fiy = 0.0, fiz = 0.0;
-        auto pair = [&](int j, const double4& xj) {
+    const int ia     = i < nlocal ? i : 0;
+    const double4 xi = x[ia];
+    const int n      = i < nlocal ? numneigh[ia] : 0;
+    const int* nb    = neighbors + list_at(0, ld, ia) + u;
+    const int nmax   = __reduce_max_sync(0xffffffffu, n);
+    const double fpi = fp[ia];
+    double sum       = 0.0; // threads 0, 1, 2: the x, y, z force
+    int j            = n > 0 ? __ldcs(nb) : -1;
+    for (int k = 0; k < nmax; k += MDB_TILE) {
+        double tx = 0.0, ty = 0.0, tz = 0.0;
+        const int jn = k + MDB_TILE < n
+                           ? __ldcs(nb + (size_t)(k / MDB_TILE + 1) * ld * MDB_TILE)
+                           : -1;
+        if (j >= 0) {
+            const double4 xj = ldg4(x + j);
             double delx = xi.x - xj.x;
             double dely = xi.y - xj.y;
             double delz = xi.z - xj.z;
@@ -123,45 +149,35 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_fp64(int nlocal,
                 m        = m < e.nr - 1 ? m : e.nr - 1;
                 p -= m;
                 p                = p < 1.0 ? p : 1.0;
-                const double* cr = e.rhor + 8 * m;
-                const double* cz = e.z2r + 8 * m;
-                double rhoip     = (__ldg(cr + 0) * p + __ldg(cr + 1)) * p + __ldg(cr + 2);
-                double z2p       = (__ldg(cz + 0) * p + __ldg(cz + 1)) * p + __ldg(cz + 2);
-                double z2 = ((__ldg(cz + 3) * p + __ldg(cz + 4)) * p + __ldg(cz + 5)) * p +
-                            __ldg(cz + 6);
+                const double4 cr = ldg4(e.rhor + 2 * m + 1);
+                const double4 cz = ldg4(e.z2r + 2 * m), cd = ldg4(e.z2r + 2 * m + 1);
+                double rhoip     = (cr.x * p + cr.y) * p + cr.z;
+                double z2p       = (cd.x * p + cd.y) * p + cd.z;
+                double z2        = ((cz.x * p + cz.y) * p + cz.z) * p + cz.w;
                 double recip = 1.0 / r;
                 double phi   = z2 * recip;
                 double phip  = z2p * recip - phi * recip;
                 double psip  = fpi * rhoip + __ldg(fp + j) * rhoip + phip;
                 double fpair = -psip * recip;
-                fix += delx * fpair;
-                fiy += dely * fpair;
-                fiz += delz * fpair;
+                tx = delx * fpair;
+                ty = dely * fpair;
+                tz = delz * fpair;
                 if (ENERGY) eng += 0.5 * phi;
             }
-        };
-        int k = 0;
-        for (; k + EUNROLL <= n; k += EUNROLL) {
-            int j[EUNROLL];
-            double4 xj[EUNROLL];
-#pragma unroll
-            for (int u = 0; u < EUNROLL; u++)
-                j[u] = __ldcs(nb + (size_t)(k + u) * ld);
-#pragma unroll
-            for (int u = 0; u < EUNROLL; u++)
-                xj[u] = ldg4(x + j[u]);
-#pragma unroll
-            for (int u = 0; u < EUNROLL; u++)
-                pair(j[u], xj[u]);
         }
-        for (; k < n; k++) {
-            int j = __ldcs(nb + (size_t)k * ld);
-            pair(j, ldg4(x + j));
+        s_term[g][0][u] = tx;
+        s_term[g][1][u] = ty;
+        s_term[g][2][u] = tz;
+        __syncwarp();
+        if (u < 3) {
+#pragma unroll
+            for (int q = 0; q < MDB_TILE; q++)
+                sum += s_term[g][u][q];
         }
-        fx[i] = fix;
-        fy[i] = fiy;
-        fz[i] = fiz;
+        __syncwarp();
+        j = jn;
     }
+    if (i < nlocal && u < 3) (u == 0 ? fx : u == 1 ? fy : fz)[i] = sum;
     if (ENERGY) {
         double s = block_sum(eng);
         if (threadIdx.x == 0) epart[blockIdx.x] = s;
@@ -194,14 +210,14 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_mixed(int nlocal,
     if (i < nlocal) {
         const float4 pi = xr[i];
         const int n     = numneigh[i];
-        const int* nb   = neighbors + i;
+        const int* nb   = neighbors + list_at(0, ld, i);
         int* out        = cut + i;
         int c           = 0;
         double rhoi     = 0.0; // FP64 embedding (density) sum
         const float rdr = (float)e.rdr;
         auto pair       = [&](int en, const float4& pj) {
             float dx, dy, dz;
-            cell_delta(pi, pj, (unsigned)en >> MDB_IDX_BITS, cg, dx, dy, dz);
+            cell_delta(pi, pj, en, cg, dx, dy, dz);
             float rsq = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
             if (rsq < cutforcesq) {
                 float p = __fmaf_rn(sqrtf(rsq), rdr, 1.0f);
@@ -215,23 +231,16 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_mixed(int nlocal,
                 c++;
             }
         };
-        int k = 0;
-        for (; k + EUNROLL <= n; k += EUNROLL) {
-            int en[EUNROLL];
-            float4 pj[EUNROLL];
+        for (int k = 0; k < n; k += MDB_TILE, nb += (size_t)ld * MDB_TILE) {
+            int en[MDB_TILE];
+            float4 pj[MDB_TILE];
+            ld_tile(nb, en);
 #pragma unroll
-            for (int v = 0; v < EUNROLL; v++)
-                en[v] = __ldcs(nb + (size_t)(k + v) * ld);
+            for (int v = 0; v < MDB_TILE; v++)
+                pj[v] = __ldg(xr + entry_index(en[v]));
 #pragma unroll
-            for (int v = 0; v < EUNROLL; v++)
-                pj[v] = __ldg(xr + (en[v] & MDB_IDX_MASK));
-#pragma unroll
-            for (int v = 0; v < EUNROLL; v++)
+            for (int v = 0; v < MDB_TILE; v++)
                 pair(en[v], pj[v]);
-        }
-        for (; k < n; k++) {
-            const int en = __ldcs(nb + (size_t)k * ld);
-            pair(en, __ldg(xr + (en & MDB_IDX_MASK)));
         }
         ncut[i]   = c;
         double p = 1.0 * rhoi * e.rdrho + 1.0;
@@ -240,11 +249,11 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_mixed(int nlocal,
         m        = m > 1 ? m : 1;
         p -= m;
         p                = p < 1.0 ? p : 1.0;
-        const double* cf = e.frho + 8 * m;
-        const double fpi = (__ldg(cf + 0) * p + __ldg(cf + 1)) * p + __ldg(cf + 2);
+        const double4 cf = ldg4(e.frho + 2 * m), df = ldg4(e.frho + 2 * m + 1);
+        const double fpi = (df.x * p + df.y) * p + df.z;
         fp[i]            = fpi;
         xe[i]            = make_float4(pi.x, pi.y, pi.z, (float)fpi);
-        if (ENERGY) eng = ((__ldg(cf + 3) * p + __ldg(cf + 4)) * p + __ldg(cf + 5)) * p + __ldg(cf + 6);
+        if (ENERGY) eng = ((cf.x * p + cf.y) * p + cf.z) * p + cf.w;
     }
     if (ENERGY) {
         double s = block_sum(eng);
@@ -275,7 +284,6 @@ __global__ void __launch_bounds__(2 * EAM_THREADS) k_eam_rho_mixed2(int nlocal,
     const int ia    = act ? i : 0;
     const float4 pi = act ? xr[ia] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int n     = act ? numneigh[ia] : 0;
-    const int* nb   = neighbors + ia;
     int* out        = cut + ia;
     int c           = 0;     // entries appended so far (both lanes)
     double rhoi     = 0.0;   // this lane's FP64 partial density
@@ -286,7 +294,7 @@ __global__ void __launch_bounds__(2 * EAM_THREADS) k_eam_rho_mixed2(int nlocal,
         bool in = false;
         if (valid) {
             float dx, dy, dz;
-            cell_delta(pi, pj, (unsigned)en >> MDB_IDX_BITS, cg, dx, dy, dz);
+            cell_delta(pi, pj, en, cg, dx, dy, dz);
             const float rsq = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
             in              = rsq < cutforcesq;
             if (in) {
@@ -314,19 +322,19 @@ __global__ void __launch_bounds__(2 * EAM_THREADS) k_eam_rho_mixed2(int nlocal,
 #pragma unroll
         for (int v = 0; v < EUNROLL; v++) {
             const int kk = k + 2 * v + u;
-            en[v]        = kk < n ? __ldcs(nb + (size_t)kk * ld) : 0;
+            en[v]        = kk < n ? __ldcs(neighbors + list_at(kk, ld, ia)) : 0;
         }
 #pragma unroll
         for (int v = 0; v < EUNROLL; v++)
-            pj[v] = k + 2 * v + u < n ? __ldg(xr + (en[v] & MDB_IDX_MASK)) : pi;
+            pj[v] = k + 2 * v + u < n ? __ldg(xr + entry_index(en[v])) : pi;
 #pragma unroll
         for (int v = 0; v < EUNROLL; v++)
             pair(en[v], pj[v], k + 2 * v + u < n);
     }
     for (; k < nmax; k += 2) {
         const bool valid = k + u < n;
-        const int en     = valid ? __ldcs(nb + (size_t)(k + u) * ld) : 0;
-        pair(en, valid ? __ldg(xr + (en & MDB_IDX_MASK)) : pi, valid);
+        const int en     = valid ? __ldcs(neighbors + list_at(k + u, ld, ia)) : 0;
+        pair(en, valid ? __ldg(xr + entry_index(en)) : pi, valid);
     }
     rhoi += __shfl_xor_sync(0xffffffffu, rhoi, 1);
     if (act && u == 0) {
@@ -337,11 +345,11 @@ __global__ void __launch_bounds__(2 * EAM_THREADS) k_eam_rho_mixed2(int nlocal,
         m        = m > 1 ? m : 1;
         p -= m;
         p                = p < 1.0 ? p : 1.0;
-        const double* cf = e.frho + 8 * m;
-        const double fpi = (__ldg(cf + 0) * p + __ldg(cf + 1)) * p + __ldg(cf + 2);
+        const double4 cf = ldg4(e.frho + 2 * m), df = ldg4(e.frho + 2 * m + 1);
+        const double fpi = (df.x * p + df.y) * p + df.z;
         fp[i]            = fpi;
         xe[i]            = make_float4(pi.x, pi.y, pi.z, (float)fpi);
-        if (ENERGY) eng = ((__ldg(cf + 3) * p + __ldg(cf + 4)) * p + __ldg(cf + 5)) * p + __ldg(cf + 6);
+        if (ENERGY) eng = ((cf.x * p + cf.y) * p + cf.z) * p + cf.w;
     }
     if (ENERGY) {
         double s = block_sum(eng);
@@ -396,7 +404,7 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_mixed(int nlocal,
         };
         auto pair = [&](int en, const float4& pj) {
             float dx, dy, dz;
-            cell_delta(pi, pj, (unsigned)en >> MDB_IDX_BITS, cg, dx, dy, dz);
+            cell_delta(pi, pj, en, cg, dx, dy, dz);
             const float rsq = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
             const float r   = sqrtf(rsq);
             float p         = __fmaf_rn(r, rdr, 1.0f);
@@ -430,14 +438,14 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_mixed(int nlocal,
                 en[v] = __ldcs(nb + (size_t)(k + v) * ld);
 #pragma unroll
             for (int v = 0; v < EUNROLL; v++)
-                pj[v] = __ldg(xe + (en[v] & MDB_IDX_MASK));
+                pj[v] = __ldg(xe + entry_index(en[v]));
 #pragma unroll
             for (int v = 0; v < EUNROLL; v++)
                 pair(en[v], pj[v]);
         }
         for (; k < n; k++) {
             const int en = __ldcs(nb + (size_t)k * ld);
-            pair(en, __ldg(xe + (en & MDB_IDX_MASK)));
+            pair(en, __ldg(xe + entry_index(en)));
         }
         fx[i] = (double)fix + (double)cx;
         fy[i] = (double)fiy + (double)cy;
@@ -458,26 +466,26 @@ static void fp_ghost(cudaStream_t s, int nlocal, int ghost_cap, double* fp,
     g_launches++;
 }
 
-void launch_eam_fp64(cudaStream_t s, int energy, int nlocal, int ghost_cap, const int* order,
+void launch_eam_fp64(cudaStream_t s, int energy, int nlocal, int ghost_cap,
     const double4* x, const int* numneigh, const int* neighbors, int ld, double cutforcesq,
     EamDev eam, const int* border_map, const int* counters, double* fp, double* fx,
     double* fy, double* fz, double* epart_rho, double* epart_pair)
 {
     if (nlocal <= 0) return;
-    int nb = mdb_blocks(nlocal, EAM_THREADS);
+    const int nb = eam_fp64_blocks(nlocal);
     if (energy)
-        k_eam_rho_fp64<true><<<nb, EAM_THREADS, 0, s>>>(nlocal, order, x, numneigh, neighbors,
+        k_eam_rho_fp64<true><<<nb, EAM_THREADS, 0, s>>>(nlocal, x, numneigh, neighbors,
             ld, cutforcesq, eam, fp, epart_rho);
     else
-        k_eam_rho_fp64<false><<<nb, EAM_THREADS, 0, s>>>(nlocal, order, x, numneigh, neighbors,
+        k_eam_rho_fp64<false><<<nb, EAM_THREADS, 0, s>>>(nlocal, x, numneigh, neighbors,
             ld, cutforcesq, eam, fp, epart_rho);
     g_launches++;
     fp_ghost(s, nlocal, ghost_cap, fp, border_map, counters);
     if (energy)
-        k_eam_force_fp64<true><<<nb, EAM_THREADS, 0, s>>>(nlocal, order, x, numneigh,
+        k_eam_force_fp64<true><<<nb, EAM_THREADS, 0, s>>>(nlocal, x, numneigh,
             neighbors, ld, cutforcesq, eam, fp, fx, fy, fz, epart_pair);
     else
-        k_eam_force_fp64<false><<<nb, EAM_THREADS, 0, s>>>(nlocal, order, x, numneigh,
+        k_eam_force_fp64<false><<<nb, EAM_THREADS, 0, s>>>(nlocal, x, numneigh,
             neighbors, ld, cutforcesq, eam, fp, fx, fy, fz, epart_pair);
     g_launches++;
 }

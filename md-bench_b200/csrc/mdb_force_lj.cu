@@ -1,34 +1,31 @@
 // Lennard-Jones forces over Verlet lists (computeForceLJFullNeigh /
 // computeForceLJHalfNeigh, verletlist/force_lj.c:17-206).
 //
-// Thread t handles atom i = t (or order[t] when an order is given) and reads
-// row t of the list. The list is k-major, so each step of the k loop is one 128-byte coalesced
-// read per warp; neighbour positions are 32-byte (FP64) or 16-byte (mixed)
-// gathers that mostly hit L1/L2. The k loop is unrolled by UNROLL with all
-// list reads and gathers of a batch issued before any arithmetic, which keeps
-// enough bytes in flight for the HBM-bound list stream. Pairs are summed in
-// list order.
+// Thread t handles atom t and its row of the list, a tile of 8 entries at a
+// time (one 256-bit load, 1 KB coalesced per warp); neighbour positions are
+// 32-byte (FP64) or 16-byte (mixed) gathers that mostly hit L1/L2. All gathers
+// of a tile are issued before any arithmetic, which keeps enough bytes in
+// flight. Pairs are summed in list order.
 //
 // FP64 path: -fmad=false keeps every product and sum rounded as the
 // reference's strict build rounds them, so full-list forces are bit-identical.
 // Mixed path: FP32 positions relative to the centre of each atom's cell (edge
 // G, a power of two) plus the cell offset of the pair (-1, 0, +1 per axis,
 // 2-bit fields of the list entry): dx = (p_i - p_j) - offset * G, the offset
-// decoded into an exact float with integer bit operations. No int->float
+// decoded into an exact float with one integer bit operation. No int->float
 // conversions, no shared-memory table, one approximate reciprocal per pair;
 // FP32 force sums (or two-sum compensated sums), FP64 energy sums.
+#include "mdb_cp_f2.cuh"
 #include "mdb_internal.cuh"
 
 namespace mdb {
 
 static constexpr int LJ_THREADS = 128;
-static constexpr int UNROLL     = 8;
 
 int force_partial_blocks(int n) { return mdb_blocks(n > 0 ? n : 1, LJ_THREADS); }
 
 template <bool HALF, bool UNIFORM, bool ENERGY>
-__global__ void __launch_bounds__(LJ_THREADS) k_lj_fp64(int nlocal,
-    const int* __restrict__ order, const double4* __restrict__ x,
+__global__ void __launch_bounds__(LJ_THREADS) k_lj_fp64(int nlocal, const double4* __restrict__ x,
     const int* __restrict__ numneigh, const int* __restrict__ neighbors, int ld,
     double cutforcesq, LJTable tab, double* __restrict__ fx, double* __restrict__ fy,
     double* __restrict__ fz, double* __restrict__ epart)
@@ -46,11 +43,11 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_fp64(int nlocal,
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     double epot = 0.0;
     if (t < nlocal) {
-        const int i      = order ? order[t] : t;
+        const int i      = t;
         const double4 xi = x[i];
         const int ti     = type_of(xi);
-        const int n      = numneigh[t];
-        const int* nb    = neighbors + t;
+        const int n      = numneigh[i];
+        const int* nb    = neighbors + list_at(0, ld, i);
         double fix = 0.0, fiy = 0.0, fiz = 0.0;
         const double eps0 = tab.eps[0], sig0 = tab.sig6[0];
 
@@ -84,23 +81,16 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_fp64(int nlocal,
             }
         };
 
-        int k = 0;
-        for (; k + UNROLL <= n; k += UNROLL) {
-            int j[UNROLL];
-            double4 xj[UNROLL];
+        for (int k = 0; k < n; k += MDB_TILE, nb += (size_t)ld * MDB_TILE) {
+            int j[MDB_TILE];
+            double4 xj[MDB_TILE];
+            ld_tile(nb, j);
 #pragma unroll
-            for (int u = 0; u < UNROLL; u++)
-                j[u] = __ldcs(nb + (size_t)(k + u) * ld);
-#pragma unroll
-            for (int u = 0; u < UNROLL; u++)
+            for (int u = 0; u < MDB_TILE; u++)
                 xj[u] = ldg4(x + j[u]);
 #pragma unroll
-            for (int u = 0; u < UNROLL; u++)
+            for (int u = 0; u < MDB_TILE; u++)
                 pair(j[u], xj[u]);
-        }
-        for (; k < n; k++) {
-            int j = __ldcs(nb + (size_t)k * ld);
-            pair(j, ldg4(x + j));
         }
         if (HALF) {
             atomicAdd(&fx[i], fix);
@@ -119,8 +109,7 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_fp64(int nlocal,
 }
 
 template <bool HALF, bool UNIFORM, bool ENERGY, bool COMP>
-__global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal,
-    const int* __restrict__ order, const float4* __restrict__ xr, CellShift sh,
+__global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal, const float4* __restrict__ xr, CellShift sh,
     const int* __restrict__ numneigh, const int* __restrict__ neighbors, int ld,
     float cutforcesq, LJTableF tab, double* __restrict__ fx, double* __restrict__ fy,
     double* __restrict__ fz, double* __restrict__ epart)
@@ -139,11 +128,11 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal,
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     double epot = 0.0;
     if (t < nlocal) {
-        const int i     = order ? order[t] : t;
+        const int i     = t;
         const float4 pi = xr[i];
         const int ti    = __float_as_int(pi.w);
-        const int n     = numneigh[t];
-        const int* nb   = neighbors + t;
+        const int n     = numneigh[i];
+        const int* nb   = neighbors + list_at(0, ld, i);
         float fix = 0.f, fiy = 0.f, fiz = 0.f;
         float cx = 0.f, cy = 0.f, cz = 0.f; // compensation terms
         const float eps0 = tab.eps[0], sig0 = tab.sig6[0];
@@ -165,9 +154,9 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal,
         };
 
         auto pair = [&](int e, const float4& pj) {
-            const int j = e & MDB_IDX_MASK;
+            const int j = entry_index(e);
             float delx, dely, delz;
-            cell_delta(pi, pj, (unsigned)e >> MDB_IDX_BITS, cg, delx, dely, delz);
+            cell_delta(pi, pj, e, cg, delx, dely, delz);
             float rsq = __fmaf_rn(delx, delx, __fmaf_rn(dely, dely, delz * delz));
             float sigma6 = sig0, epsilon = eps0;
             if (!UNIFORM) {
@@ -175,17 +164,7 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal,
                 sigma6  = s_sig6[tij];
                 epsilon = s_eps[tij];
             }
-            if (UNIFORM && !HALF && !ENERGY && !COMP) {
-                // one type, full lists: no branch; pairs outside the cutoff
-                // add exact zeros (the same sums as the branch)
-                const float sr2 = __fdividef(1.0f, rsq);
-                const float s3  = sr2 * sr2 * sr2;
-                float force     = sr2 * s3 * __fmaf_rn(cA, s3, -cB);
-                force           = rsq < cutforcesq ? force : 0.0f;
-                fix             = __fmaf_rn(delx, force, fix);
-                fiy             = __fmaf_rn(dely, force, fiy);
-                fiz             = __fmaf_rn(delz, force, fiz);
-            } else if (rsq < cutforcesq) {
+            if (rsq < cutforcesq) {
                 float sr2 = __fdividef(1.0f, rsq);
                 float sr6, force;
                 if (UNIFORM) {
@@ -211,27 +190,84 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal,
             }
         };
 
-        int k = 0;
-        for (; k + UNROLL <= n; k += UNROLL) {
-            int e[UNROLL];
-            float4 pj[UNROLL];
+        double rx = 0.0, ry = 0.0, rz = 0.0;
+        if (UNIFORM && !HALF && !COMP) {
+            // One type, full lists: two entries per packed instruction and no
+            // branch; a pair outside the cutoff adds an exact zero (the same
+            // forces with and without the energy). Even and odd
+            // entries of a tile sum apart in FP32, the tiles in FP64 (6 instructions
+            // in 8 pairs; a row's sum then rounds less than pair by pair in FP32).
+            // 168 -> 132 us per launch at 1M atoms (155 with tiles alone): half
+            // the instructions per pair, the gathers' latency and L1 bound it.
+            using namespace cp;
+            const f2 G0 = f2_pack(-cg, -cg), G1 = f2_pack(-0.25f * cg, -0.25f * cg),
+                     G2 = f2_pack(-0.0625f * cg, -0.0625f * cg);
+            const f2 B0 = f2_pack(CELL_BIAS(0), CELL_BIAS(0)),
+                     B1 = f2_pack(CELL_BIAS(1), CELL_BIAS(1)),
+                     B2 = f2_pack(CELL_BIAS(2), CELL_BIAS(2));
+            const f2 A2 = f2_pack(cA, cA), mB2 = f2_pack(-cB, -cB);
+            for (int k = 0; k < n; k += MDB_TILE, nb += (size_t)ld * MDB_TILE) {
+                int e[MDB_TILE];
+                float4 pj[MDB_TILE];
+                ld_tile(nb, e);
 #pragma unroll
-            for (int u = 0; u < UNROLL; u++)
-                e[u] = __ldcs(nb + (size_t)(k + u) * ld);
+                for (int u = 0; u < MDB_TILE; u++)
+                    pj[u] = __ldg(xr + entry_index(e[u]));
+                f2 tx = 0, ty = 0, tz = 0;
 #pragma unroll
-            for (int u = 0; u < UNROLL; u++)
-                pj[u] = __ldg(xr + (e[u] & MDB_IDX_MASK));
+                for (int u = 0; u < MDB_TILE; u += 2) {
+                    const float4 &a = pj[u], &b = pj[u + 1];
+                    const f2 dx = f2_fma(
+                        f2_sub(f2_pack(cell_field(e[u], 0), cell_field(e[u + 1], 0)), B0), G0,
+                        f2_pack(pi.x - a.x, pi.x - b.x));
+                    const f2 dy = f2_fma(
+                        f2_sub(f2_pack(cell_field(e[u], 1), cell_field(e[u + 1], 1)), B1), G1,
+                        f2_pack(pi.y - a.y, pi.y - b.y));
+                    const f2 dz = f2_fma(
+                        f2_sub(f2_pack(cell_field(e[u], 2), cell_field(e[u + 1], 2)), B2), G2,
+                        f2_pack(pi.z - a.z, pi.z - b.z));
+                    const f2 rsq = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+                    float r0, r1;
+                    f2_unpack(rsq, r0, r1);
+                    const float u0 = rcp_approx(r0), u1 = rcp_approx(r1);
+                    const f2 U  = f2_pack(r0 < cutforcesq ? u0 : 0.0f, r1 < cutforcesq ? u1 : 0.0f);
+                    const f2 U2 = f2_mul(U, U);
+                    const f2 U3 = f2_mul(U2, U);
+                    const f2 F  = f2_mul(f2_mul(U2, U2), f2_fma(A2, U3, mB2));
+                    if (ENERGY) {
+                        float s0, s1;
+                        f2_unpack(f2_mul(U3, f2_pack(sig0, sig0)), s0, s1);
+                        epot += 0.5 * (double)(4.0f * eps0 * s0 * (s0 - 1.0f));
+                        epot += 0.5 * (double)(4.0f * eps0 * s1 * (s1 - 1.0f));
+                    }
+                    tx = u ? f2_fma(dx, F, tx) : f2_mul(dx, F);
+                    ty = u ? f2_fma(dy, F, ty) : f2_mul(dy, F);
+                    tz = u ? f2_fma(dz, F, tz) : f2_mul(dz, F);
+                }
+                float t0, t1;
+                f2_unpack(tx, t0, t1);
+                rx += (double)(t0 + t1);
+                f2_unpack(ty, t0, t1);
+                ry += (double)(t0 + t1);
+                f2_unpack(tz, t0, t1);
+                rz += (double)(t0 + t1);
+            }
+        } else {
+            for (int k = 0; k < n; k += MDB_TILE, nb += (size_t)ld * MDB_TILE) {
+                int e[MDB_TILE];
+                float4 pj[MDB_TILE];
+                ld_tile(nb, e);
 #pragma unroll
-            for (int u = 0; u < UNROLL; u++)
-                pair(e[u], pj[u]);
+                for (int u = 0; u < MDB_TILE; u++)
+                    pj[u] = __ldg(xr + entry_index(e[u]));
+#pragma unroll
+                for (int u = 0; u < MDB_TILE; u++)
+                    pair(e[u], pj[u]);
+            }
         }
-        for (; k < n; k++) {
-            int e = __ldcs(nb + (size_t)k * ld);
-            pair(e, __ldg(xr + (e & MDB_IDX_MASK)));
-        }
-        double rx = (double)fix + (double)cx;
-        double ry = (double)fiy + (double)cy;
-        double rz = (double)fiz + (double)cz;
+        rx += (double)fix + (double)cx;
+        ry += (double)fiy + (double)cy;
+        rz += (double)fiz + (double)cz;
         if (HALF) {
             atomicAdd(&fx[i], rx);
             atomicAdd(&fy[i], ry);
@@ -249,19 +285,19 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal,
 }
 
 template <bool HALF, bool UNIFORM>
-static void lj64(cudaStream_t s, int energy, int nb, int nlocal, const int* order,
+static void lj64(cudaStream_t s, int energy, int nb, int nlocal,
     const double4* x, const int* numneigh, const int* neighbors, int ld, double cut,
     const LJTable& tab, double* fx, double* fy, double* fz, double* epart)
 {
     if (energy)
-        k_lj_fp64<HALF, UNIFORM, true><<<nb, LJ_THREADS, 0, s>>>(nlocal, order, x, numneigh,
+        k_lj_fp64<HALF, UNIFORM, true><<<nb, LJ_THREADS, 0, s>>>(nlocal, x, numneigh,
             neighbors, ld, cut, tab, fx, fy, fz, epart);
     else
-        k_lj_fp64<HALF, UNIFORM, false><<<nb, LJ_THREADS, 0, s>>>(nlocal, order, x, numneigh,
+        k_lj_fp64<HALF, UNIFORM, false><<<nb, LJ_THREADS, 0, s>>>(nlocal, x, numneigh,
             neighbors, ld, cut, tab, fx, fy, fz, epart);
 }
 
-void launch_lj_fp64(cudaStream_t s, int half, int energy, int nlocal, const int* order,
+void launch_lj_fp64(cudaStream_t s, int half, int energy, int nlocal,
     const double4* x, const int* numneigh, const int* neighbors, int ld, double cutforcesq,
     const LJTable& tab, double* fx, double* fy, double* fz, double* epart)
 {
@@ -269,50 +305,50 @@ void launch_lj_fp64(cudaStream_t s, int half, int energy, int nlocal, const int*
     int nb = force_partial_blocks(nlocal);
     if (half) {
         if (tab.uniform)
-            lj64<true, true>(s, energy, nb, nlocal, order, x, numneigh, neighbors, ld,
+            lj64<true, true>(s, energy, nb, nlocal, x, numneigh, neighbors, ld,
                 cutforcesq, tab, fx, fy, fz, epart);
         else
-            lj64<true, false>(s, energy, nb, nlocal, order, x, numneigh, neighbors, ld,
+            lj64<true, false>(s, energy, nb, nlocal, x, numneigh, neighbors, ld,
                 cutforcesq, tab, fx, fy, fz, epart);
     } else {
         if (tab.uniform)
-            lj64<false, true>(s, energy, nb, nlocal, order, x, numneigh, neighbors, ld,
+            lj64<false, true>(s, energy, nb, nlocal, x, numneigh, neighbors, ld,
                 cutforcesq, tab, fx, fy, fz, epart);
         else
-            lj64<false, false>(s, energy, nb, nlocal, order, x, numneigh, neighbors, ld,
+            lj64<false, false>(s, energy, nb, nlocal, x, numneigh, neighbors, ld,
                 cutforcesq, tab, fx, fy, fz, epart);
     }
     g_launches++;
 }
 
 template <bool HALF, bool UNIFORM, bool COMP>
-static void ljmx(cudaStream_t s, int energy, int nb, int nlocal, const int* order,
+static void ljmx(cudaStream_t s, int energy, int nb, int nlocal,
     const float4* xr, const CellShift& sh, const int* numneigh, const int* neighbors, int ld,
     float cut, const LJTableF& tab, double* fx, double* fy, double* fz, double* epart)
 {
     if (energy)
-        k_lj_mixed<HALF, UNIFORM, true, COMP><<<nb, LJ_THREADS, 0, s>>>(nlocal, order, xr, sh,
+        k_lj_mixed<HALF, UNIFORM, true, COMP><<<nb, LJ_THREADS, 0, s>>>(nlocal, xr, sh,
             numneigh, neighbors, ld, cut, tab, fx, fy, fz, epart);
     else
-        k_lj_mixed<HALF, UNIFORM, false, COMP><<<nb, LJ_THREADS, 0, s>>>(nlocal, order, xr, sh,
+        k_lj_mixed<HALF, UNIFORM, false, COMP><<<nb, LJ_THREADS, 0, s>>>(nlocal, xr, sh,
             numneigh, neighbors, ld, cut, tab, fx, fy, fz, epart);
 }
 
 template <bool HALF, bool COMP>
-static void ljmx_u(cudaStream_t s, int energy, int nb, int nlocal, const int* order,
+static void ljmx_u(cudaStream_t s, int energy, int nb, int nlocal,
     const float4* xr, const CellShift& sh, const int* numneigh, const int* neighbors, int ld,
     float cut, const LJTableF& tab, double* fx, double* fy, double* fz, double* epart)
 {
     if (tab.uniform)
-        ljmx<HALF, true, COMP>(s, energy, nb, nlocal, order, xr, sh, numneigh, neighbors, ld,
+        ljmx<HALF, true, COMP>(s, energy, nb, nlocal, xr, sh, numneigh, neighbors, ld,
             cut, tab, fx, fy, fz, epart);
     else
-        ljmx<HALF, false, COMP>(s, energy, nb, nlocal, order, xr, sh, numneigh, neighbors, ld,
+        ljmx<HALF, false, COMP>(s, energy, nb, nlocal, xr, sh, numneigh, neighbors, ld,
             cut, tab, fx, fy, fz, epart);
 }
 
 void launch_lj_mixed(cudaStream_t s, int comp, int half, int energy, int nlocal,
-    const int* order, const float4* xr, const CellShift& sh, const int* numneigh,
+    const float4* xr, const CellShift& sh, const int* numneigh,
     const int* neighbors, int ld, float cutforcesq, const LJTableF& tab, double* fx,
     double* fy, double* fz, double* epart)
 {
@@ -320,17 +356,17 @@ void launch_lj_mixed(cudaStream_t s, int comp, int half, int energy, int nlocal,
     int nb = force_partial_blocks(nlocal);
     if (half) {
         if (comp)
-            ljmx_u<true, true>(s, energy, nb, nlocal, order, xr, sh, numneigh, neighbors, ld,
+            ljmx_u<true, true>(s, energy, nb, nlocal, xr, sh, numneigh, neighbors, ld,
                 cutforcesq, tab, fx, fy, fz, epart);
         else
-            ljmx_u<true, false>(s, energy, nb, nlocal, order, xr, sh, numneigh, neighbors, ld,
+            ljmx_u<true, false>(s, energy, nb, nlocal, xr, sh, numneigh, neighbors, ld,
                 cutforcesq, tab, fx, fy, fz, epart);
     } else {
         if (comp)
-            ljmx_u<false, true>(s, energy, nb, nlocal, order, xr, sh, numneigh, neighbors, ld,
+            ljmx_u<false, true>(s, energy, nb, nlocal, xr, sh, numneigh, neighbors, ld,
                 cutforcesq, tab, fx, fy, fz, epart);
         else
-            ljmx_u<false, false>(s, energy, nb, nlocal, order, xr, sh, numneigh, neighbors, ld,
+            ljmx_u<false, false>(s, energy, nb, nlocal, xr, sh, numneigh, neighbors, ld,
                 cutforcesq, tab, fx, fy, fz, epart);
     }
     g_launches++;

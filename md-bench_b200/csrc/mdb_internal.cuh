@@ -1,18 +1,25 @@
 // Internal declarations shared by the libmdb translation units.
 // Device data layout (HBM), per context:
-//   x        double4[nall_cap]  positions of locals then ghosts; .w holds the type
-//                               id as raw int bits (never used arithmetically)
-//   xr       float4[nall_cap]   mixed path: position relative to the centre of the
+//   x        double4[nall_cap + 1]  positions of locals then ghosts; .w holds the type
+//                               id as raw int bits (never used arithmetically); last
+//                               the dummy atom (MDB_FAR), which pads rows of the list
+//   xr       float4[nall_cap + 1]  mixed path: position relative to the centre of the
 //                               atom's cell (cells of edge G, a power of two, fixed at
 //                               each rebuild), .w type bits
 //   qcell    int[nall_cap]      mixed path: the cell of each atom, 10 bits per axis
 //   vx,vy,vz / fx,fy,fz         SoA doubles over locals
-//   neighbors int32 [maxneighs][ld]  SoA (k-major), row t belongs to atom
-//                               local_order[t] (atoms of one bin are adjacent rows);
-//                               mixed path: bits 0-24 index, bits 25-31 cell-offset code
-//   numneigh  int32 [nlocal]    indexed by row t
-//   bins: CSR (bin_start[mbins+1], bin_atoms[nall]) with atoms of a bin in
-//         ascending index order, so lists come out in the reference order
+//   neighbors int32 [ceil(maxneighs / 8)][ld][8]  tiles of 8 consecutive entries of
+//                               a row: entry k of atom i at list_at(k, ld, i). A warp
+//                               of consecutive atoms reads a tile as 1 KB, and a row
+//                               is written in whole 32-byte sectors. Entries of a
+//                               row's last tile past numneigh[i] name the dummy atom
+//                               nall_cap, which is out of every atom's reach.
+//                               Mixed path: the atom index above MDB_CODE_BITS bits
+//                               of the pair's cell-offset code
+//   numneigh  int32 [nlocal]    entries of atom i
+//   bins: CSR (bin_start[mbins+1]) with atoms of a bin in ascending index order,
+//         so lists come out in the reference order; their FP32 positions as three
+//         arrays (binf, [3][bin_stride(nall_cap)]) and {index, cell} (bin_jq)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -22,8 +29,12 @@
 
 #define MDB_MAX_TYPES   8
 #define MDB_MAX_STENCIL 1331 /* (2*5+1)^3 */
-#define MDB_IDX_BITS    26   /* mixed-path list entries: index bits (6 code bits above) */
-#define MDB_IDX_MASK    ((1 << MDB_IDX_BITS) - 1)
+#define MDB_CODE_BITS   6    /* mixed-path list entries: cell-offset code below the index */
+#define MDB_IDX_MASK    ((1 << (32 - MDB_CODE_BITS)) - 1)
+#define MDB_CODE_SAME   0x15 /* the code of two atoms in one cell */
+#define MDB_FAR         1.0e18 /* coordinates of the dummy atom */
+
+#define MDB_TILE        8 /* list entries of one row in one 32-byte sector */
 
 // device counters (int slots)
 enum {
@@ -62,7 +73,7 @@ struct LJTableF {
 // Mixed-path cells: edge G, the smallest power of two >= cutneigh, so the
 // cells of a listed pair differ by -1, 0 or +1 per axis and offset * G is
 // exact in FP32. A list entry stores the three offsets + 1 as 2-bit fields
-// above the index bits.
+// below the index bits.
 struct CellFrame {
     double g;
     double ginv;
@@ -72,31 +83,37 @@ struct CellShift {
     float g;
 };
 
-// cell offset (-1, 0 or +1) of 2-bit field f, as an exact float without an
-// int->float conversion: 0x4B400000 is 1.5 * 2^23, so OR-ing f into the
-// mantissa gives 12582912 + f exactly
-__device__ __forceinline__ float cell_offset(unsigned f)
+// atom index of a mixed-path entry
+__device__ __forceinline__ int entry_index(int e) { return (int)((unsigned)e >> MDB_CODE_BITS); }
+
+// Field a of an entry's cell-offset code as an exact float, 4^a (offset + 1)
+// above 1.5 * 2^23, without a shift or an int->float conversion: the field
+// stays where it is in the mantissa. Less CELL_BIAS(a) that is 4^a * offset,
+// which times G / 4^a (exact, powers of two) is offset * G.
+__device__ __forceinline__ float cell_field(int e, int a)
 {
-    return __int_as_float(0x4B400000 | (int)f) - 12582913.0f;
+    return __int_as_float(0x4B400000 | (e & (3 << (2 * a))));
 }
+#define CELL_BIAS(a) (12582912.0f + (float)(1 << (2 * (a))))
 
 // pair difference p_i - p_j - offset * G on the mixed path; a fused multiply-add
 // with the exact product offset * G rounds once
-__device__ __forceinline__ void cell_delta(const float4& pi, const float4& pj, unsigned code,
-    float g, float& dx, float& dy, float& dz)
+__device__ __forceinline__ void cell_delta(const float4& pi, const float4& pj, int e, float g,
+    float& dx, float& dy, float& dz)
 {
-    dx = __fmaf_rn(-cell_offset(code & 3u), g, pi.x - pj.x);
-    dy = __fmaf_rn(-cell_offset((code >> 2) & 3u), g, pi.y - pj.y);
-    dz = __fmaf_rn(-cell_offset((code >> 4) & 3u), g, pi.z - pj.z);
+    dx = __fmaf_rn(CELL_BIAS(0) - cell_field(e, 0), g, pi.x - pj.x);
+    dy = __fmaf_rn(CELL_BIAS(1) - cell_field(e, 1), 0.25f * g, pi.y - pj.y);
+    dz = __fmaf_rn(CELL_BIAS(2) - cell_field(e, 2), 0.0625f * g, pi.z - pj.z);
 }
 
 struct EamDev {
     int nrho, nr;
     double rdr, rdrho;
-    const double* frho; // rows of 8 doubles (coefficients 0..6 + pad)
-    const double* rhor;
-    const double* z2r;
-    const float* frho32;
+    // two double4 per grid point: coefficients 3..6 (the value's cubic), then
+    // 0..2 (its derivative's quadratic)
+    const double4* frho;
+    const double4* rhor;
+    const double4* z2r;
     // mixed path, FP32 rows: dens32[m] = rho coefficients 3..6 (the density
     // pass); pair32[2m], pair32[2m + 1] = z2r coefficients 3..6, then rho
     // coefficients 0..2 and z2r coefficient 0 (the force pass: z2r 1 and 2
@@ -138,6 +155,32 @@ __device__ __forceinline__ float4 rel_position(const double4& p, int q, const Ce
     r.z = (float)(p.z - ((double)cell_axis(q, 2) + 0.5) * cf.g);
     r.w = __int_as_float(type_of(p));
     return r;
+}
+
+// entry k of row i of a tiled list
+__host__ __device__ __forceinline__ size_t list_at(int k, int ld, int i)
+{
+    return ((size_t)(k / MDB_TILE) * ld + i) * MDB_TILE + k % MDB_TILE;
+}
+
+// floats of one coordinate of the bin-ordered positions: 16-byte aligned
+// loads, which may reach 7 entries past the binned atoms
+__host__ __device__ __forceinline__ int bin_stride(int nall_cap) { return (nall_cap + 11) & ~3; }
+
+// ints of a tiled list of rows of up to maxneighs entries
+__host__ __device__ __forceinline__ size_t list_ints(int maxneighs, int ld)
+{
+    return (size_t)((maxneighs + MDB_TILE - 1) / MDB_TILE) * ld * MDB_TILE;
+}
+
+// one tile (32-byte aligned) in one 256-bit load that leaves L1 to the
+// gathered positions
+__device__ __forceinline__ void ld_tile(const int* p, int (&e)[MDB_TILE])
+{
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(e[0]), "=r"(e[1]), "=r"(e[2]), "=r"(e[3]), "=r"(e[4]), "=r"(e[5]),
+                   "=r"(e[6]), "=r"(e[7])
+                 : "l"(p));
 }
 
 // block-wide sum; the result is valid in thread 0 (all threads must call)
@@ -204,34 +247,36 @@ void launch_bin_count(cudaStream_t s, int nlocal, int nall_cap, const double4* x
     int* atom_bin, int* atom_slot, int* bin_count, int* bin_lcount, int* counters);
 void launch_bin_scatter(cudaStream_t s, int nlocal, int nall_cap, const int* atom_bin,
     const int* atom_slot, const int* bin_start, int* bin_atoms, const int* counters);
-void launch_bin_sort(cudaStream_t s, int mbins, const int* bin_start, int* bin_atoms,
-    const int* loc_start, int* local_order);
-// stencil entries: {flat bin offset, dx, dy, dz}; qcell non-null packs cell codes
-// positions of the binned atoms in bin order (atom index bits in .w), FP64
-// and rounded to FP32
-void launch_bin_positions(cudaStream_t s, int nall_cap, int mbins, const double4* x,
-    const int* bin_start, const int* bin_atoms, double4* bin_x, float4* bin_xf);
-// the Verlet list from the bin-ordered positions; margin bounds the FP32
-// prefilter's rsq error (only candidates within it take the exact FP64 test)
-void launch_build_list(cudaStream_t s, int nlocal, const double4* x, BinGeom g,
-    const int4* stencil, const int* atom_bin, const int* bin_start,
-    const double4* bin_x, const float4* bin_xf, double cutneighsq, float margin, int half,
-    int maxneighs, int ld, int* neighbors, int* numneigh, int* counters, const int* qcell);
+// the atoms of each bin in index order: {index, cell} and FP32 positions in bin
+// order (binf: x, then y, then z, bin_stride(nall_cap) each), and the locals
+// bin by bin (local_order); qcell null: cells 0
+void launch_bin_order(cudaStream_t s, int nlocal, int nall_cap, int mbins, const double4* x,
+    const int* atom_bin, const int* bin_start, const int* bin_atoms, const int* loc_start,
+    const int* qcell, int2* bin_jq, float* binf, int* local_order);
+// the Verlet list from the bin-ordered positions; rows: the stencil's runs of
+// bins along x, {flat offset of the middle bin, dy, dz, bins to either side};
+// margin bounds the FP32 prefilter's rsq error (only candidates within it take
+// the exact FP64 test)
+void launch_build_list(cudaStream_t s, int nlocal, int nall_cap, const int* local_order,
+    const int* loc_start, const double4* x, BinGeom g, int nrows, const int4* rows, const int* atom_bin,
+    const int* bin_start, const int2* bin_jq, const float* binf, double cutneighsq,
+    float margin, int half, int maxneighs, int ld, int* neighbors, int* numneigh, int* counters,
+    const int* qcell);
 int ke_partial_blocks(int n);
 void launch_ke_partial(cudaStream_t s, int n, const double* vx, const double* vy,
     const double* vz, double mass, double* partials);
 void launch_reduce_partials(cudaStream_t s, int nparts, const double* partials, double* out);
 
-// forces (mdb_force_lj.cu, mdb_force_eam.cu); thread t handles atom order[t]
+// forces (mdb_force_lj.cu, mdb_force_eam.cu)
 int force_partial_blocks(int n);
-void launch_lj_fp64(cudaStream_t s, int half, int energy, int nlocal, const int* order,
+void launch_lj_fp64(cudaStream_t s, int half, int energy, int nlocal,
     const double4* x, const int* numneigh, const int* neighbors, int ld, double cutforcesq,
     const LJTable& tab, double* fx, double* fy, double* fz, double* epart);
 void launch_lj_mixed(cudaStream_t s, int comp, int half, int energy, int nlocal,
-    const int* order, const float4* xr, const CellShift& sh, const int* numneigh,
+    const float4* xr, const CellShift& sh, const int* numneigh,
     const int* neighbors, int ld, float cutforcesq, const LJTableF& tab, double* fx,
     double* fy, double* fz, double* epart);
-void launch_eam_fp64(cudaStream_t s, int energy, int nlocal, int ghost_cap, const int* order,
+void launch_eam_fp64(cudaStream_t s, int energy, int nlocal, int ghost_cap,
     const double4* x, const int* numneigh, const int* neighbors, int ld, double cutforcesq,
     EamDev eam, const int* border_map, const int* counters, double* fp, double* fx,
     double* fy, double* fz, double* epart_rho, double* epart_pair);
@@ -244,7 +289,9 @@ int launch_eam_mixed(cudaStream_t s, int energy, int comp, int rho_lanes, int nl
     float cutforcesq, EamDev eam, const int* border_map, const int* counters, int* cut,
     int* ncut, double* fp, float4* xe, double* fx, double* fy, double* fz, double* epart_rho,
     double* epart_pair);
+// blocks (= energy partials per pass) of the EAM kernels
 int eam_mixed_blocks(int nlocal);
+int eam_fp64_blocks(int nlocal);
 
 // domain-decomposed runs: positions of atoms idx[0..n) plus a shift, AoS
 // triples (the halo another domain receives); and the positions of halo
