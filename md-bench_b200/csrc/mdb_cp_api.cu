@@ -101,19 +101,17 @@ struct MdbCp {
     bool snap_valid    = false;
     long long rebuilds_sched = 0, rebuilds_check = 0;
     // the check decided on the device (default; "check_on_host" 1: the host
-    // reads the flag every step): one graph per step with conditional nodes
-    // that rebuild when the flag is up, and skip the force and every later
-    // step of the call once such a rebuild overflowed a buffer (the host
-    // grows it, replays that build and resumes). dstate: {stopped, steps
-    // run, rebuilds} on the device, h_dstate its pinned copy
+    // reads the flag every step): one graph per step with a conditional node
+    // that rebuilds when the flag goes up; once such a rebuild overflowed a
+    // buffer no later step of the call moves an atom (the host grows it,
+    // replays that build and resumes). dstate: {stopped, steps run, rebuilds}
+    // on the device, h_dstate its pinned copy
     bool check_host    = false;
     int* dstate        = nullptr;
     int* h_dstate      = nullptr;
-    cudaStream_t s_cap[2] = {nullptr, nullptr}; // capture streams of the bodies
+    cudaStream_t s_cap = nullptr; // capture stream of the rebuild
     CpGraph g_chk;
-    // kernels of the checked step graph's parts, for the launch count: the
-    // step's fixed part, the ghost update, the rebuild, the force
-    long long chk_k[4] = {0, 0, 0, 0};
+    long long chk_k[2] = {0, 0}; // kernels of the checked step graph: a step's, a rebuild's
     long long chk_steps = 0, chk_replays = 0; // graph steps run, overflowed rebuilds replayed
     // pair-list force path of the mixed scheme (force_path 1, mdb_cp_pairs.cu):
     // codes per (i pair, chunk), their counts, the positions they were
@@ -481,8 +479,7 @@ extern "C" int mdb_cp_destroy(MdbCp* ctx)
     drop_graph(ctx);
     free_all(ctx);
     if (ctx->s) cudaStreamDestroy(ctx->s);
-    for (cudaStream_t c : ctx->s_cap)
-        if (c) cudaStreamDestroy(c);
+    if (ctx->s_cap) cudaStreamDestroy(ctx->s_cap);
     delete ctx;
     return MDB_OK;
 }
@@ -1013,28 +1010,29 @@ static float pair_qlim2(const MdbCp* ctx)
     return (float)(q * q);
 }
 
-static void enq_force(MdbCp* ctx, bool energy)
+// the half-list force slots of the local clusters' capacity to zero
+static void enq_zero_forces(MdbCp* ctx)
+{
+    const size_t n = (size_t)ctx->ncl_cap * ctx->M;
+    if (f32_slots(ctx)) cudaMemsetAsync(ctx->cf32, 0, sizeof(float4) * n, ctx->s);
+    else cudaMemsetAsync(ctx->cf, 0, sizeof(double4) * n, ctx->s);
+}
+
+// zeroed: the integrator cleared the half-list force slots (zero_in_integrator)
+static void enq_force(MdbCp* ctx, bool energy, bool zeroed = false)
 {
     cudaStream_t s = ctx->s;
-    const int nloc_slots = ctx->ncl_cap * ctx->M;
+    if (ctx->p.half_neigh && !zeroed) enq_zero_forces(ctx);
     if (pair_path(ctx)) {
-        if (ctx->p.half_neigh && ctx->comp)
-            cudaMemsetAsync(ctx->cf, 0, sizeof(double4) * (size_t)nloc_slots, s);
-        else if (ctx->p.half_neigh)
-            cudaMemsetAsync(ctx->cf32, 0, sizeof(float4) * (size_t)nloc_slots, s);
         enq_derive(ctx, 0);
         const int nb = enq_force_pairs(ctx, energy);
         if (energy) ctx->energy_blocks = nb;
     } else if (ctx->mixed) {
-        if (ctx->p.half_neigh)
-            cudaMemsetAsync(ctx->cf32, 0, sizeof(float4) * (size_t)nloc_slots, s);
         const int nb = launch_force_mixed(s, ctx->N, ctx->p.half_neigh, energy, ctx->ncl_cap,
             ctx->cnt, ctx->xr, ctx->anchor, ctx->ty, (float)ctx->cutforcesq, ctx->list, lks(ctx),
             lcs(ctx), ctx->numneigh, ctx->cf32, ctx->partials);
         if (energy) ctx->energy_blocks = nb;
     } else {
-        if (ctx->p.half_neigh)
-            cudaMemsetAsync(ctx->cf, 0, sizeof(double4) * (size_t)nloc_slots, s);
         launch_force_fp64(s, ctx->M, ctx->N, ctx->p.half_neigh, energy, ctx->ncl_cap, ctx->cnt,
             ctx->cx, ctx->ty, ctx->cutforcesq, ctx->list, lks(ctx), lcs(ctx), ctx->numneigh,
             ctx->cf, ctx->partials);
@@ -1048,14 +1046,28 @@ static const double4* check_xb(const MdbCp* ctx)
     return ctx->disp_max > 0.0 && ctx->snap_valid ? ctx->xbuild : nullptr;
 }
 
-static void enq_initial(MdbCp* ctx)
+// an initial integration's other work; ghosts: the images follow (setupPbc has
+// run); zero: the force slots are cleared for the force evaluation of this step
+static CpInitial initial_args(const MdbCp* ctx, bool ghosts, bool zero)
 {
-    const bool pq = pair_path(ctx);
+    CpInitial in;
+    if (ghosts) {
+        in.gstart = ctx->gstart, in.pbc = ctx->pbc;
+        in.xprd = ctx->g.xprd, in.yprd = ctx->g.yprd, in.zprd = ctx->g.zprd;
+    }
+    in.zero = zero;
+    in.xb   = check_xb(ctx);
+    in.lim2 = ctx->disp_max * ctx->disp_max;
+    in.flag = ctx->dflag;
+    if (pair_path(ctx)) in.xq = ctx->xq, in.qlim2 = pair_qlim2(ctx), in.qflag = ctx->qflag;
+    return in;
+}
+
+static void enq_initial(MdbCp* ctx, bool ghosts)
+{
     launch_cp_initial(ctx->s, ctx->M, ctx->N, ctx->ncl_cap, ctx->cnt, ctx->p.dtforce, ctx->p.dt,
         ctx->cx, ctx->cv, ctx->cf, f32_slots(ctx), ctx->anchor,
-        ctx->mixed ? ctx->xr : nullptr, xr_mode(ctx), check_xb(ctx),
-        ctx->disp_max * ctx->disp_max, ctx->dflag, pq ? ctx->xq : nullptr, pair_qlim2(ctx),
-        pq ? ctx->qflag : nullptr);
+        ctx->mixed ? ctx->xr : nullptr, xr_mode(ctx), initial_args(ctx, ghosts, false));
 }
 
 static void enq_final(MdbCp* ctx)
@@ -1064,14 +1076,11 @@ static void enq_final(MdbCp* ctx)
         ctx->cf, f32_slots(ctx));
 }
 
-static void enq_final_initial(MdbCp* ctx)
+static void enq_final_initial(MdbCp* ctx, const CpInitial& in)
 {
-    const bool pq = pair_path(ctx);
     launch_cp_final_initial(ctx->s, ctx->M, ctx->N, ctx->ncl_cap, ctx->cnt, ctx->p.dtforce,
         ctx->p.dt, ctx->cx, ctx->cv, ctx->cf, f32_slots(ctx), ctx->anchor,
-        ctx->mixed ? ctx->xr : nullptr, xr_mode(ctx), check_xb(ctx),
-        ctx->disp_max * ctx->disp_max, ctx->dflag, pq ? ctx->xq : nullptr, pair_qlim2(ctx),
-        pq ? ctx->qflag : nullptr);
+        ctx->mixed ? ctx->xr : nullptr, xr_mode(ctx), in);
 }
 
 static void enq_ghost_update(MdbCp* ctx)
@@ -1264,7 +1273,7 @@ extern "C" int mdb_cp_initial_integrate(MdbCp* ctx)
     NEED_ATOMS();
     if (!ctx->have_clusters) return fail(ctx, MDB_ERR_STATE, "buildClusters not run");
     long long m = mark();
-    enq_initial(ctx);
+    enq_initial(ctx, false);
     account(ctx, m);
     ctx->force_current = false;
     return MDB_OK;
@@ -1352,13 +1361,19 @@ extern "C" int mdb_cp_setup(MdbCp* ctx)
     return compute_force(ctx, false);
 }
 
+// the integrator of a plain step clears the half-list force slots
+static bool zero_in_integrator(const MdbCp* ctx)
+{
+    return ctx->p.half_neigh && ctx->ncl_cap * ctx->M <= CP_ZERO_SLOTS;
+}
+
 // A plain step whose predecessor left its final integration pending:
-// finalIntegrate(n-1) + initialIntegrate(n), updatePbc, force.
+// finalIntegrate(n-1) + initialIntegrate(n) + updatePbc, then the force.
 static void enq_plain_step(MdbCp* ctx)
 {
-    enq_final_initial(ctx);
-    enq_ghost_update(ctx);
-    enq_force(ctx, false);
+    const bool zero = zero_in_integrator(ctx);
+    enq_final_initial(ctx, initial_args(ctx, true, zero));
+    enq_force(ctx, false, zero);
 }
 
 static int capture_plain(MdbCp* ctx)
@@ -1378,29 +1393,23 @@ static int capture_plain(MdbCp* ctx)
 }
 
 // ---- displacement check decided on the device --------------------------------
-// dstate = {stopped, steps run, rebuilds}: a step's graph opens with a gate
-// (the step runs unless a rebuild earlier in the call overflowed a buffer),
-// rebuilds when the integrator raised the displacement flag, and runs the
-// force unless that rebuild overflowed.
+// dstate = {stopped, steps run, rebuilds}: a step's graph runs unless a rebuild
+// earlier in the call overflowed a buffer.
+// after a rebuild inside a step graph: what eval_build would grow (or reject)
+// stops the call
+__global__ void k_chk_built(const int* cnt, int ngc_cap, int maxneighs, int* st)
+{
+    st[2]++;
+    if (cnt[CP_BADBIN] > 0 || cnt[CP_NGC_TOTAL] > ngc_cap || cnt[CP_MAXNEED] >= maxneighs)
+        st[0] = 1;
+}
+
+// the gates of the ensemble's step graph
 __global__ void k_chk_gate(cudaGraphConditionalHandle h, int* st)
 {
     const bool go = st[0] == 0;
     if (go) st[1]++;
     cudaGraphSetConditional(h, go ? 1u : 0u);
-}
-
-__global__ void k_chk_reb(cudaGraphConditionalHandle h, const int* dflag, int* st)
-{
-    const bool reb = *dflag != 0;
-    if (reb) st[2]++;
-    cudaGraphSetConditional(h, reb ? 1u : 0u);
-}
-
-// what eval_build would grow (or reject) stops the call
-__global__ void k_chk_built(const int* cnt, int ngc_cap, int maxneighs, int* st)
-{
-    if (cnt[CP_BADBIN] > 0 || cnt[CP_NGC_TOTAL] > ngc_cap || cnt[CP_MAXNEED] >= maxneighs)
-        st[0] = 1;
 }
 
 __global__ void k_chk_force(cudaGraphConditionalHandle h, const int* st)
@@ -1436,98 +1445,69 @@ static cudaError_t cap_handle(cudaStream_t s, cudaGraphConditionalHandle* h)
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamGetCaptureInfo(s, &st, nullptr, &g, nullptr, nullptr);
     if (e != cudaSuccess) return e;
-    return cudaGraphConditionalHandleCreate(h, g, 0, 0);
+    return cudaGraphConditionalHandleCreate(h, g, 0, cudaGraphCondAssignDefault);
 }
 
-// One checked step as a graph: finalIntegrate(n-1) + initialIntegrate(n) with
-// the displacement test, then either updateAtoms + the whole rebuild (an atom
-// moved past the limit) or updatePbc, then the force; all of it only while no
-// rebuild of this call has overflowed a buffer. The bodies are captured on two
-// further streams (enq_* enqueue on ctx->s, which points at the capturing one).
+// One checked step as a graph: finalIntegrate(n-1) + initialIntegrate(n) +
+// updatePbc with the displacement test, an "if" node with updateAtoms + the
+// whole rebuild when the integrator found an atom past the limit and set the
+// node's condition (0 at each launch), then the force. After a rebuild of this
+// call has overflowed a buffer the integrator does nothing, so no later step
+// moves an atom; the force is evaluated all the same (every read stays inside
+// the clamped lists and ghosts) and replaced when the host replays the rebuild.
+// One conditional node and no gate kernels: a checked step took 70 us with
+// three nodes and four single-thread kernels on a 45,356-atom system whose
+// plain step takes 25 us. The body is captured on a further stream (enq_*
+// enqueue on ctx->s, which points at the capturing one).
 static int capture_chk(MdbCp* ctx)
 {
     cudaError_t e = cudaSuccess;
-    for (cudaStream_t& c : ctx->s_cap)
-        if (!c && (e = cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking)) != cudaSuccess)
-            return fail(ctx, MDB_ERR_CUDA, "capture stream", e);
-    const cudaStream_t s0 = ctx->s, s1 = ctx->s_cap[0], s2 = ctx->s_cap[1];
+    if (!ctx->s_cap && (e = cudaStreamCreateWithFlags(&ctx->s_cap, cudaStreamNonBlocking)) !=
+                           cudaSuccess)
+        return fail(ctx, MDB_ERR_CUDA, "capture stream", e);
+    const cudaStream_t s0 = ctx->s, s1 = ctx->s_cap;
     const cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
-    cudaGraphConditionalHandle h_step = 0, h_reb = 0, h_force = 0;
-    cudaGraph_t step[1] = {nullptr}, reb[2] = {nullptr, nullptr}, frc[1] = {nullptr};
-    cudaGraph_t graph = nullptr;
+    const bool zero = zero_in_integrator(ctx);
+    CpInitial in    = initial_args(ctx, true, zero);
+    in.stop         = ctx->dstate;
+    in.ran          = ctx->dstate + 1;
+    cudaGraph_t body = nullptr, graph = nullptr;
     const long long m0 = mark();
-    long long* k = ctx->chk_k;
-    bool cap1 = false, cap2 = false;
-    auto body2 = [&](cudaGraph_t g, int what) -> cudaError_t {
-        // one body of the inner conditionals, captured on s2
-        cudaError_t r = cudaStreamBeginCaptureToGraph(s2, g, nullptr, nullptr, 0, mode);
-        if (r != cudaSuccess) return r;
-        cap2 = true;
-        ctx->s = s2;
-        long long m = mark();
-        if (what == 0) {
-            enq_gather(ctx, 1);
-            enq_build(ctx);
-            k_chk_built<<<1, 1, 0, s2>>>(ctx->cnt, ctx->ngc_cap, ctx->maxneighs, ctx->dstate);
-            cudaMemcpyAsync(ctx->xbuild, ctx->cx, sizeof(double4) * ctx->ncl_cap * ctx->M,
-                cudaMemcpyDeviceToDevice, s2);
-            cudaMemsetAsync(ctx->dflag, 0, sizeof(int), s2);
-            k[2] = mark() - m + 1;
-        } else if (what == 1) {
-            enq_ghost_update(ctx);
-            k[1] = mark() - m;
-        } else {
-            enq_force(ctx, false);
-            k[3] = mark() - m;
-        }
-        ctx->s = s1;
-        r = cudaGetLastError();
-        cudaGraph_t out = nullptr;
-        cudaError_t r2 = cudaStreamEndCapture(s2, &out);
-        cap2 = false;
-        return r != cudaSuccess ? r : r2;
-    };
+    long long* k       = ctx->chk_k;
     e = cudaStreamBeginCapture(s0, mode);
-    if (e == cudaSuccess) e = cap_handle(s0, &h_step);
+    if (e != cudaSuccess) return fail(ctx, MDB_ERR_CUDA, "checked step graph", e);
+    e = cap_handle(s0, &in.cond);
     if (e == cudaSuccess) {
-        k_chk_gate<<<1, 1, 0, s0>>>(h_step, ctx->dstate);
+        enq_final_initial(ctx, in);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cap_conditional(s0, h_step, 1, step);
-    if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(s1, step[0], nullptr, nullptr, 0, mode);
+    if (e == cudaSuccess) e = cap_conditional(s0, in.cond, 1, &body);
+    if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(s1, body, nullptr, nullptr, 0, mode);
     if (e == cudaSuccess) {
-        cap1   = true;
-        ctx->s = s1;
-        long long m = mark();
-        enq_final_initial(ctx);
-        k[0] = mark() - m + 2;
-        e = cap_handle(s1, &h_reb);
-    }
-    if (e == cudaSuccess) {
-        k_chk_reb<<<1, 1, 0, s1>>>(h_reb, ctx->dflag, ctx->dstate);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cap_conditional(s1, h_reb, 2, reb);
-    if (e == cudaSuccess) e = body2(reb[0], 0);
-    if (e == cudaSuccess) e = body2(reb[1], 1);
-    if (e == cudaSuccess) e = cap_handle(s1, &h_force);
-    if (e == cudaSuccess) {
-        k_chk_force<<<1, 1, 0, s1>>>(h_force, ctx->dstate);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cap_conditional(s1, h_force, 1, frc);
-    if (e == cudaSuccess) e = body2(frc[0], 2);
-    ctx->s = s0;
-    mdb::g_launches = m0;
-    if (cap2) {
-        cudaGraph_t g2 = nullptr;
-        cudaStreamEndCapture(s2, &g2);
-    }
-    if (cap1) {
-        cudaGraph_t g1       = nullptr;
-        const cudaError_t e1 = cudaStreamEndCapture(s1, &g1);
+        ctx->s            = s1;
+        const long long m = mark();
+        enq_gather(ctx, 1);
+        enq_build(ctx);
+        k_chk_built<<<1, 1, 0, s1>>>(ctx->cnt, ctx->ngc_cap, ctx->maxneighs, ctx->dstate);
+        cudaMemcpyAsync(ctx->xbuild, ctx->cx, sizeof(double4) * ctx->ncl_cap * ctx->M,
+            cudaMemcpyDeviceToDevice, s1);
+        cudaMemsetAsync(ctx->dflag, 0, sizeof(int), s1);
+        if (zero) // the slots hold other atoms now
+            enq_zero_forces(ctx);
+        k[1]   = mark() - m + 1;
+        ctx->s = s0;
+        e      = cudaGetLastError();
+        cudaGraph_t out      = nullptr;
+        const cudaError_t e1 = cudaStreamEndCapture(s1, &out);
         if (e == cudaSuccess) e = e1;
     }
+    if (e == cudaSuccess) {
+        const long long m = mark();
+        enq_force(ctx, false, zero);
+        k[0] = mark() - m + 1;
+        e    = cudaGetLastError();
+    }
+    mdb::g_launches      = m0;
     const cudaError_t e0 = cudaStreamEndCapture(s0, &graph);
     if (e == cudaSuccess) e = e0;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&ctx->g_chk.exec, graph, 0);
@@ -1558,8 +1538,7 @@ static int chk_resolve(MdbCp* ctx, std::vector<int>& launched, int* resume)
     ctx->rebuilds_check += reb;
     ctx->chk_steps += ran;
     ctx->chk_replays += stopped ? 1 : 0;
-    ctx->launches += (long long)launched.size() + ran * k[0] + (ran - reb) * k[1] + reb * k[2] +
-                     (ran - stopped) * k[3];
+    ctx->launches += (long long)launched.size() * k[0] + reb * k[1];
     if (stopped) {
         if (ran < 1 || ran > (int)launched.size())
             return fail(ctx, MDB_ERR_CUDA, "checked steps: inconsistent device record");
@@ -1625,12 +1604,14 @@ static int run_checked(MdbCp* ctx, int first_step, int nsteps, MdbThermo* sample
             }
         }
         const bool had = ctx->snap_valid;
+        bool reneigh   = sched || !had;
         long long m    = mark();
-        if (pending_final) enq_final_initial(ctx);
-        else enq_initial(ctx);
+        // (pruning reads the ghosts of the last step, as the reference's does)
+        const bool ghosts = !reneigh && !prune;
+        if (pending_final) enq_final_initial(ctx, initial_args(ctx, ghosts, false));
+        else enq_initial(ctx, ghosts);
         pending_final = false;
         account(ctx, m);
-        bool reneigh = sched || !had;
         if (!reneigh) {
             CK(cudaMemcpyAsync(ctx->h_dflag, ctx->dflag, sizeof(int), cudaMemcpyDeviceToHost,
                 ctx->s));
@@ -1646,9 +1627,9 @@ static int run_checked(MdbCp* ctx, int first_step, int nsteps, MdbThermo* sample
             account(ctx, m);
             int rc = do_build(ctx);
             if (rc) return rc;
-        } else {
+        } else if (prune) {
             m = mark();
-            if (prune) enq_prune(ctx);
+            enq_prune(ctx);
             enq_ghost_update(ctx);
             account(ctx, m);
         }
@@ -1733,8 +1714,10 @@ extern "C" int mdb_cp_run(MdbCp* ctx, int first_step, int nsteps, MdbThermo* sam
             continue;
         }
         long long m = mark();
-        if (pending_final) enq_final_initial(ctx);
-        else enq_initial(ctx);
+        // (pruning reads the ghosts of the last step, as the reference's does)
+        const bool ghosts = !reneigh && !prune;
+        if (pending_final) enq_final_initial(ctx, initial_args(ctx, ghosts, false));
+        else enq_initial(ctx, ghosts);
         pending_final = false;
         account(ctx, m);
         if (reneigh) {
@@ -1744,9 +1727,9 @@ extern "C" int mdb_cp_run(MdbCp* ctx, int first_step, int nsteps, MdbThermo* sam
             account(ctx, m);
             int rc = do_build(ctx);
             if (rc) return rc;
-        } else {
+        } else if (prune) {
             m = mark();
-            if (prune) enq_prune(ctx);
+            enq_prune(ctx);
             enq_ghost_update(ctx);
             account(ctx, m);
         }
@@ -1994,8 +1977,8 @@ struct MdbCpEnsemble {
     CpForceMember* d_force = nullptr;
     int2* d_bmap           = nullptr;
     size_t bmap_cap        = 0;
-    int nb_integ = 0, nb_ghost = 0;
-    size_t off_integ = 0, off_ghost = 0;
+    int nb_integ     = 0;
+    size_t off_integ = 0;
     // batched rebuild: member table, block map per stage, counters of all members
     CpBuildMember* d_build = nullptr;
     int nb_stage[CB_COUNT]     = {};
@@ -2016,7 +1999,7 @@ struct MdbCpEnsemble {
     int* d_rebcnt   = nullptr; // per member: checked rebuilds on the device
     int* h_rebcnt   = nullptr;
     cudaStream_t s_cap[2] = {nullptr, nullptr};
-    long long chk_k[4]    = {0, 0, 0, 0}; // kernels: fixed part, ghost update, rebuild, force
+    long long chk_k[3]    = {0, 0, 0}; // kernels: fixed part, rebuild, force
     long long chk_steps = 0, chk_replays = 0;
     // per member {M, N, force group, i-clusters per warp, force threads}, for
     // the block maps that a rebuild inside the checked step graph refreshes
@@ -2030,12 +2013,11 @@ struct MdbCpEnsemble {
         int nblocks;
         size_t off, off_dyn;
     };
-    // block maps of the integrator, the ghost update and the force groups that
-    // cover only the members' current clusters (the rest of each region is
+    // block maps of the integrator and the force groups that cover only the members' current clusters (the rest of each region is
     // unused entries); refreshed from the counters after every rebuild.
     // Energy evaluations use the capacity maps, so that every energy partial
     // of a member is written.
-    size_t off_integ_dyn = 0, off_ghost_dyn = 0, dyn_begin = 0, dyn_end = 0;
+    size_t off_integ_dyn = 0, dyn_begin = 0, dyn_end = 0;
     int2* h_dyn = nullptr;
     std::vector<int> gid;
     std::vector<Group> groups;
@@ -2057,7 +2039,6 @@ enum {
     EG_CK_FI,     // FI with the check, flags to the host
     EG_CK_I,      // I with the check, flags to the host
     EG_REB_NOINT, // the rebuild of EG_REB_* without the integration
-    EG_GHOST,     // ghost update
     EG_CHK,       // a whole checked step, the rebuild decided on the device
     EG_COUNT
 };
@@ -2088,22 +2069,15 @@ static void ens_body(MdbCp* c, int kind)
     switch (kind) {
     case EG_PLAIN_FI: enq_plain_step(c); break;
     case EG_PLAIN_I:
-        enq_initial(c);
-        enq_ghost_update(c);
+        enq_initial(c, true);
         enq_force(c, false);
         break;
-    case EG_FRONT_FI:
-        enq_final_initial(c);
-        enq_ghost_update(c);
-        break;
-    case EG_FRONT_I:
-        enq_initial(c);
-        enq_ghost_update(c);
-        break;
+    case EG_FRONT_FI: enq_final_initial(c, initial_args(c, true, false)); break;
+    case EG_FRONT_I: enq_initial(c, true); break;
     case EG_REB_FI:
     case EG_REB_I:
-        if (kind == EG_REB_FI) enq_final_initial(c);
-        else enq_initial(c);
+        if (kind == EG_REB_FI) enq_final_initial(c, initial_args(c, false, false));
+        else enq_initial(c, false);
         enq_gather(c, 1);
         enq_build(c);
         cudaMemcpyAsync(c->h_cnt, c->cnt, CP_SLOTS * sizeof(int), cudaMemcpyDeviceToHost, c->s);
@@ -2150,9 +2124,6 @@ static int ens_dyn_maps(MdbCpEnsemble* e)
     fill(e->nb_integ, [](const MdbCp* c) {
         return mdb_blocks((long long)c->h_cnt[CP_NCL] * c->M, MDB_NTHREADS);
     });
-    fill(e->nb_ghost, [](const MdbCp* c) {
-        return mdb_blocks((long long)c->h_cnt[CP_NGC] * c->N, MDB_NTHREADS);
-    });
     for (size_t q = 0; q < e->groups.size(); q++) {
         const size_t end = w + e->groups[q].nblocks;
         for (int k = 0; k < n; k++) {
@@ -2188,8 +2159,8 @@ static int ens_tables(MdbCpEnsemble* e)
         const MdbCp* c = e->m[k];
         CpStepMember& a = st[k];
         a.cnt = c->cnt, a.cx = c->cx, a.cv = c->cv, a.cf = c->cf, a.cf32 = c->cf32;
-        a.anchor = c->anchor, a.xr = c->xr, a.border = c->border, a.pbc = c->pbc;
-        a.jnat = c->jnat, a.dtf = c->p.dtforce, a.dt = c->p.dt, a.xprd = c->g.xprd;
+        a.anchor = c->anchor, a.xr = c->xr, a.gstart = c->gstart, a.pbc = c->pbc;
+        a.dtf = c->p.dtforce, a.dt = c->p.dt, a.xprd = c->g.xprd;
         a.yprd = c->g.yprd, a.zprd = c->g.zprd, a.M = c->M, a.N = c->N, a.mixed = xr_mode(c);
         a.zero_f = c->p.half_neigh;
         a.xb     = c->disp_max > 0.0 ? c->xbuild : nullptr;
@@ -2234,10 +2205,6 @@ static int ens_tables(MdbCpEnsemble* e)
     for (int k = 0; k < n; k++)
         add(k, mdb_blocks((long long)e->m[k]->ncl_cap * e->m[k]->M, MDB_NTHREADS));
     e->nb_integ  = (int)(maps.size() - e->off_integ);
-    e->off_ghost = maps.size();
-    for (int k = 0; k < n; k++)
-        add(k, mdb_blocks((long long)e->m[k]->ngc_cap * e->m[k]->N, MDB_NTHREADS));
-    e->nb_ghost = (int)(maps.size() - e->off_ghost);
     e->groups.clear();
     std::vector<int> gid(n, -1);
     for (int k = 0; k < n; k++) {
@@ -2271,8 +2238,6 @@ static int ens_tables(MdbCpEnsemble* e)
     e->dyn_begin     = maps.size();
     e->off_integ_dyn = maps.size();
     maps.resize(maps.size() + e->nb_integ, make_int2(-1, 0));
-    e->off_ghost_dyn = maps.size();
-    maps.resize(maps.size() + e->nb_ghost, make_int2(-1, 0));
     for (auto& gr : e->groups) {
         gr.off_dyn = maps.size();
         maps.resize(maps.size() + gr.nblocks, make_int2(-1, 0));
@@ -2322,15 +2287,28 @@ static int ens_tables(MdbCpEnsemble* e)
     return ens_dyn_maps(e);
 }
 
-static void ens_integ(MdbCpEnsemble* e, bool final_, bool initial)
+// every member's slots together as one system's (zero_in_integrator)
+static bool ens_zero_in_integrator(const MdbCpEnsemble* e)
 {
-    launch_cp_integrate_batch(e->s, final_, initial, e->nb_integ, e->d_step,
-        e->d_bmap + e->off_integ_dyn);
+    long long slots = 0;
+    for (const MdbCp* c : e->m) slots += (long long)c->ncl_cap * c->M;
+    return slots <= CP_ZERO_SLOTS;
 }
 
-static void ens_forces(MdbCpEnsemble* e, bool energy)
+// an initial integration updates the members' ghosts too; zero: it clears the
+// half-list force slots for the force evaluation that follows
+static void ens_integ(MdbCpEnsemble* e, bool final_, bool initial, bool zero = false)
 {
-    launch_zero_forces_batch(e->s, e->nb_integ, e->d_step, e->d_bmap + e->off_integ_dyn);
+    bool check = false;
+    for (const MdbCp* c : e->m) check = check || c->disp_max > 0.0;
+    launch_cp_integrate_batch(e->s, final_, initial, e->nb_integ, e->d_step,
+        e->d_bmap + e->off_integ_dyn, zero, check);
+}
+
+static void ens_forces(MdbCpEnsemble* e, bool energy, bool zeroed = false)
+{
+    if (!zeroed)
+        launch_zero_forces_batch(e->s, e->nb_integ, e->d_step, e->d_bmap + e->off_integ_dyn);
     for (const auto& gr : e->groups)
         launch_force_mixed_batch(e->s, gr.N, gr.half, energy, gr.ty, gr.cutsq, gr.nblocks,
             e->d_force, e->d_bmap + (energy ? gr.off : gr.off_dyn));
@@ -2398,23 +2376,23 @@ static void ens_body_batched(MdbCpEnsemble* e, int kind)
     case EG_PLAIN_I:
     case EG_FRONT_FI:
     case EG_FRONT_I:
-        ens_integ(e, fi, true);
-        launch_ghost_update_batch(e->s, e->nb_ghost, e->d_step, e->d_bmap + e->off_ghost_dyn,
-            nullptr);
-        if (kind == EG_PLAIN_FI || kind == EG_PLAIN_I) ens_forces(e, false);
+    {
+        const bool force = kind == EG_PLAIN_FI || kind == EG_PLAIN_I;
+        const bool zero  = force && ens_zero_in_integrator(e);
+        ens_integ(e, fi, true, zero);
+        if (force) ens_forces(e, false, zero);
         break;
+    }
     case EG_REB_FI:
     case EG_REB_I:
     case EG_REB_NOINT: {
         // updateAtoms + the whole rebuild, stage by stage: of every member on
         // the schedule; of the members whose displacement flag is up in a
-        // checked step (EG_REB_NOINT), the others' ghosts updated instead
+        // checked step (EG_REB_NOINT)
         if (kind != EG_REB_NOINT) {
             ens_integ(e, fi, true);
             ens_rebuild_stages(e, nullptr);
         } else {
-            launch_ghost_update_batch(e->s, e->nb_ghost, e->d_step,
-                e->d_bmap + e->off_ghost_dyn, e->d_flags);
             ens_rebuild_stages(e, e->d_flags);
         }
         cudaMemcpyAsync(e->h_cnt_all, e->d_cnt_all, sizeof(int) * CP_SLOTS * e->m.size(),
@@ -2432,10 +2410,6 @@ static void ens_body_batched(MdbCpEnsemble* e, int kind)
         ens_integ(e, kind == EG_CK_FI, true);
         cudaMemcpyAsync(e->h_flags, e->d_flags, sizeof(int) * e->m.size(),
             cudaMemcpyDeviceToHost, e->s);
-        break;
-    case EG_GHOST:
-        launch_ghost_update_batch(e->s, e->nb_ghost, e->d_step, e->d_bmap + e->off_ghost_dyn,
-            nullptr);
         break;
     case EG_FORCE: ens_forces(e, false); break;
     case EG_SAMPLE:
@@ -2516,22 +2490,17 @@ __device__ void fill_map_region(int2* out, int cap, int n, F blocks_of)
 
 __global__ void __launch_bounds__(256) k_ens_dyn_maps(const CpBuildMember* __restrict__ tab,
     const int* __restrict__ info, int n, int2* bmap, size_t off_integ, int nb_integ,
-    size_t off_ghost, int nb_ghost, const size_t* __restrict__ goff,
-    const int* __restrict__ gnb, int ngroups)
+    const size_t* __restrict__ goff, const int* __restrict__ gnb, int ngroups)
 {
     fill_map_region(bmap + off_integ, nb_integ, n, [&](int k) {
-        return (int)(((long long)tab[k].cnt[CP_NCL] * info[5 * k] + MDB_NTHREADS - 1) /
-                     MDB_NTHREADS);
-    });
-    fill_map_region(bmap + off_ghost, nb_ghost, n, [&](int k) {
-        return (int)(((long long)tab[k].cnt[CP_NGC] * info[5 * k + 1] + MDB_NTHREADS - 1) /
+        return (int)(((long long)tab[k].cnt[CP_NCL] * info[4 * k] + MDB_NTHREADS - 1) /
                      MDB_NTHREADS);
     });
     for (int q = 0; q < ngroups; q++)
         fill_map_region(bmap + goff[q], gnb[q], n, [&](int k) {
-            if (info[5 * k + 2] != q) return 0;
-            const int nt = info[5 * k + 4];
-            return (int)(((long long)tab[k].cnt[CP_NCL] * 32 / info[5 * k + 3] + nt - 1) / nt);
+            if (info[4 * k + 1] != q) return 0;
+            const int nt = info[4 * k + 3];
+            return (int)(((long long)tab[k].cnt[CP_NCL] * 32 / info[4 * k + 2] + nt - 1) / nt);
         });
 }
 
@@ -2539,14 +2508,13 @@ __global__ void __launch_bounds__(256) k_ens_dyn_maps(const CpBuildMember* __res
 static int ens_map_info(MdbCpEnsemble* e)
 {
     const int n = (int)e->m.size(), ng = (int)e->groups.size();
-    std::vector<int> info(5 * (size_t)n);
+    std::vector<int> info(4 * (size_t)n);
     for (int k = 0; k < n; k++) {
         const MdbCp* c = e->m[k];
-        info[5 * k]     = c->M;
-        info[5 * k + 1] = c->N;
-        info[5 * k + 2] = e->gid[k];
-        info[5 * k + 3] = c->ty.force_cpw;
-        info[5 * k + 4] = force_mixed_threads(c->ty);
+        info[4 * k]     = c->M;
+        info[4 * k + 1] = e->gid[k];
+        info[4 * k + 2] = c->ty.force_cpw;
+        info[4 * k + 3] = force_mixed_threads(c->ty);
     }
     std::vector<size_t> goff(std::max(ng, 1));
     std::vector<int> gnb(std::max(ng, 1));
@@ -2569,9 +2537,10 @@ static int ens_map_info(MdbCpEnsemble* e)
 }
 
 // One checked step of a batched ensemble as a graph, as capture_chk for a
-// single system: gate; the fused integration with every member's test; if a
-// flag is up, updateAtoms + the rebuild of every member, the overflow test,
-// the snapshots and the flags cleared, else the ghost update; then the force.
+// single system: gate; the fused integration with every member's test and
+// ghost update; if a flag is up, updateAtoms + the rebuild of the members whose
+// flag it is, the overflow test, the snapshots and the flags cleared; then the
+// force.
 // Every launch uses the block maps of the current clusters, which the rebuild
 // refreshes on the device from the members' new counters.
 static int ens_capture_chk(MdbCpEnsemble* e)
@@ -2586,7 +2555,7 @@ static int ens_capture_chk(MdbCpEnsemble* e)
     const cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
     const int n = (int)e->m.size();
     cudaGraphConditionalHandle h_step = 0, h_reb = 0, h_force = 0;
-    cudaGraph_t step[1] = {nullptr}, reb[2] = {nullptr, nullptr}, frc[1] = {nullptr};
+    cudaGraph_t step[1] = {nullptr}, reb[1] = {nullptr}, frc[1] = {nullptr};
     cudaGraph_t graph = nullptr;
     const long long m0 = mark();
     long long* k = e->chk_k;
@@ -2598,26 +2567,18 @@ static int ens_capture_chk(MdbCpEnsemble* e)
         e->s = s2;
         long long m = mark();
         if (what == 0) {
-            // the members whose flag is up rebuild, the others update their
-            // ghosts as in a plain step
-            launch_ghost_update_batch(s2, e->nb_ghost, e->d_step, e->d_bmap + e->off_ghost_dyn,
-                e->d_flags);
+            // the members whose flag is up rebuild
             ens_rebuild_stages(e, e->d_flags);
             k_ens_chk_built<<<1, 128, 0, s2>>>(e->d_build, n, e->dstate);
             k_ens_dyn_maps<<<1, 256, 0, s2>>>(e->d_build, e->d_mapinfo, n, e->d_bmap,
-                e->off_integ_dyn, e->nb_integ, e->off_ghost_dyn, e->nb_ghost, e->d_goff,
-                e->d_gnb, (int)e->groups.size());
+                e->off_integ_dyn, e->nb_integ, e->d_goff, e->d_gnb, (int)e->groups.size());
             launch_snapshot_batch(s2, e->nb_integ, e->d_step, e->d_bmap + e->off_integ,
                 e->d_flags);
             cudaMemsetAsync(e->d_flags, 0, sizeof(int) * n, s2);
-            k[2] = mark() - m + 2;
-        } else if (what == 1) {
-            launch_ghost_update_batch(s2, e->nb_ghost, e->d_step, e->d_bmap + e->off_ghost_dyn,
-                nullptr);
-            k[1] = mark() - m;
+            k[1] = mark() - m + 2;
         } else {
             ens_forces(e, false);
-            k[3] = mark() - m;
+            k[2] = mark() - m;
         }
         e->s = s1;
         r = cudaGetLastError();
@@ -2646,16 +2607,15 @@ static int ens_capture_chk(MdbCpEnsemble* e)
         k_ens_chk_reb<<<1, 128, 0, s1>>>(h_reb, e->d_flags, n, e->dstate, e->d_rebcnt);
         ce = cudaGetLastError();
     }
-    if (ce == cudaSuccess) ce = cap_conditional(s1, h_reb, 2, reb);
+    if (ce == cudaSuccess) ce = cap_conditional(s1, h_reb, 1, reb);
     if (ce == cudaSuccess) ce = body2(reb[0], 0);
-    if (ce == cudaSuccess) ce = body2(reb[1], 1);
     if (ce == cudaSuccess) ce = cap_handle(s1, &h_force);
     if (ce == cudaSuccess) {
         k_chk_force<<<1, 1, 0, s1>>>(h_force, e->dstate);
         ce = cudaGetLastError();
     }
     if (ce == cudaSuccess) ce = cap_conditional(s1, h_force, 1, frc);
-    if (ce == cudaSuccess) ce = body2(frc[0], 2);
+    if (ce == cudaSuccess) ce = body2(frc[0], 1);
     e->s            = s0;
     mdb::g_launches = m0;
     if (cap2) {
@@ -2866,8 +2826,8 @@ static int ens_chk_resolve(MdbCpEnsemble* e, std::vector<int>& launched, int* re
     if (ce != cudaSuccess) return ens_fail(e, MDB_ERR_CUDA, "checked steps", ce);
     const int stopped = e->h_dstate[0], ran = e->h_dstate[1], reb = e->h_dstate[2];
     const long long* k = e->chk_k;
-    e->launches += (long long)launched.size() + ran * k[0] + (ran - reb) * k[1] + reb * k[2] +
-                   (ran - stopped) * k[3];
+    e->launches += (long long)launched.size() + ran * k[0] + reb * k[1] +
+                   (ran - stopped) * k[2];
     e->chk_steps += ran;
     e->chk_replays += stopped ? 1 : 0;
     if (reb > 0) {
@@ -2988,12 +2948,10 @@ extern "C" int mdb_cp_ensemble_run(MdbCpEnsemble* e, int first_step, int nsteps,
             bool any = false;
             for (int k = 0; k < n; k++) any = any || e->h_flags[k] != 0;
             if (any) {
-                // the members whose flag is up rebuild, the others update ghosts
+                // the members whose flag is up rebuild
                 if ((rc = ens_rebuild(e, EG_REB_NOINT))) return rc;
                 for (int k = 0; k < n; k++)
                     if (e->h_flags[k]) e->m[k]->rebuilds_check++;
-            } else if ((rc = ens_launch(e, EG_GHOST))) {
-                return rc;
             }
             if ((rc = ens_launch(e, sample ? EG_SAMPLE : EG_FORCE))) return rc;
             pending_final = !sample;
@@ -3009,8 +2967,8 @@ extern "C" int mdb_cp_ensemble_run(MdbCpEnsemble* e, int first_step, int nsteps,
             cudaStreamSynchronize(e->s);
             const long long m0 = mark();
             for (MdbCp* c : e->m) {
-                if (pending_final) enq_final_initial(c);
-                else enq_initial(c);
+                if (pending_final) enq_final_initial(c, initial_args(c, false, false));
+                else enq_initial(c, false);
                 enq_prune(c);
                 enq_ghost_update(c);
                 enq_force(c, false);

@@ -631,25 +631,6 @@ __global__ void k_ghost_update(int N, int mixed, const int* __restrict__ cnt,
         g.xprd, g.yprd, g.zprd, cx, anchor, xr);
 }
 
-// skip: null, or a flag per member (the members whose flag is set skip it)
-__global__ void k_ghost_update_batch(const CpStepMember* __restrict__ tab,
-    const int2* __restrict__ bmap, const int* __restrict__ skip)
-{
-    const int2 bm = __ldg(&bmap[blockIdx.x]);
-    if (bm.x < 0 || (skip && skip[bm.x])) return;
-    const CpStepMember& m = tab[bm.x];
-    ghost_update_slot(bm.y * blockDim.x + threadIdx.x, m.N, m.mixed, m.cnt, m.border, m.pbc,
-        m.jnat, m.xprd, m.yprd, m.zprd, m.cx, m.anchor, m.xr);
-}
-
-void launch_ghost_update_batch(cudaStream_t s, int nblocks, const CpStepMember* tab,
-    const int2* bmap, const int* skip)
-{
-    if (nblocks <= 0) return;
-    k_ghost_update_batch<<<nblocks, MDB_NTHREADS, 0, s>>>(tab, bmap, skip);
-    g_launches++;
-}
-
 void launch_ghost_update(cudaStream_t s, int N, int ngc_cap, int mixed, const int* cnt,
     const int* border, const int* pbc, const int* jnat, const Geom& g, double4* cx,
     const float4* anchor, float4* xr)

@@ -781,24 +781,50 @@ __device__ __forceinline__ double3 slot_force(int s, const double4* cf, const fl
     return make_double3(f.x, f.y, f.z);
 }
 
-// zero_f: clear the force slot after its use (half lists accumulate into it;
-// only when a force evaluation follows before anything reads the forces)
-// xb (displacement check, null: off): positions at the last build; a slot
-// that moved farther than sqrt(lim2) since then sets *flag.
-template <bool FINAL, bool INITIAL>
+// Optional work of an initial integration.
+// ghosts: the slot's periodic images follow at once (updatePbcCPU, first = 0,
+// clusterpair/pbc.c:43-113): the ghosts of j-cluster cj are gstart[cj] ..
+// gstart[cj + 1], as setupPbc numbered them. Separate from the integrator this
+// was a kernel of its own per step: 25.3 + 5.6 -> 30.7 us at 1M atoms (the time
+// between two kernels saved), 10.8 + 9.1 -> 16.9 over 32 ensemble members, 2.4 +
+// 2.2 -> 3.6 at 840.
+// zero: clear the force slot after its use (half lists accumulate into it; a
+// force evaluation follows before anything reads the forces).
+// xb (null: no displacement check): positions at the last build; a slot that
+// moved farther than sqrt(lim2) since then sets *flag and, in a step graph that
+// decides on the device, the condition of its rebuild (cond: one thread).
+// stop (null: none): a step graph after one whose rebuild overflowed does
+// nothing; ran counts the steps that ran.
+// xq: as xb for the pair codes of the pair-list path.
+// CHECK: with the displacement tests (xb, xq); they take registers that the
+// plain integrator needs for its memory parallelism.
+template <bool FINAL, bool INITIAL, bool CHECK>
 __device__ __forceinline__ void cp_integrate_slot(int s, int M, int N,
     const int* __restrict__ cnt, double dtf, double dt, double4* cx, double4* cv,
     const double4* __restrict__ cf, float4* cf32, const float4* __restrict__ anchor, float4* xr,
-    bool zero_f, int xmode, const double4* __restrict__ xb = nullptr, double lim2 = 0.0,
-    int* flag = nullptr, const float4* __restrict__ xq = nullptr, float qlim2 = 0.f,
-    int* qflag = nullptr)
+    int xmode, const CpInitial& in)
 {
     if (s >= cnt[CP_NCL] * M) return;
+    const int cj = N == 8 ? s >> 3 : s >> 2, b = s & (N - 1);
+    // everything the images need is loaded with the slot's own state, before
+    // the first store holds loads back
+    int g = 0, gend = 0, code = 0, gslot = 0;
+    float4 a = {}, ag = {};
+    if (INITIAL && in.gstart) {
+        g     = __ldg(&in.gstart[cj]);
+        gend  = min(__ldg(&in.gstart[cj + 1]), cnt[CP_NGC]);
+        gslot = cnt[CP_NCJ];
+    }
+    if (INITIAL && xr) a = __ldg(&anchor[cj]);
     double4 p = cx[s];
     if (slot_type(p) < 0) return;
     double4 v       = cv[s];
     const double3 f = slot_force(s, cf, cf32);
-    if (INITIAL && zero_f) {
+    if (INITIAL && g < gend) {
+        code = __ldg(&in.pbc[g]);
+        if (xr) ag = __ldg(&anchor[gslot + g]);
+    }
+    if (INITIAL && in.zero) {
         if (cf32) cf32[s] = make_float4(0.f, 0.f, 0.f, 0.f);
         else const_cast<double4*>(cf)[s] = make_double4(0.0, 0.0, 0.0, 0.0);
     }
@@ -815,41 +841,65 @@ __device__ __forceinline__ void cp_integrate_slot(int s, int M, int N,
         p.y += dt * v.y;
         p.z += dt * v.z;
         cx[s] = p;
-        if (xr) put_rel(xr, s, p, anchor[s / N], xmode, s % N);
-        if (xq) {
-            const float4 r = xr[s], q = xq[s];
-            const float dx = r.x - q.x, dy = r.y - q.y, dz = r.z - q.z;
-            if (dx * dx + dy * dy + dz * dz > qlim2) *qflag = 1;
+        if (xr) put_rel(xr, s, p, a, xmode, b);
+        while (g < gend) {
+            double4 q = p;
+            q.x += (double)((code & 3) - 1) * in.xprd;
+            q.y += (double)(((code >> 2) & 3) - 1) * in.yprd;
+            q.z += (double)(((code >> 4) & 3) - 1) * in.zprd;
+            const int cg    = gslot + g;
+            const float4 ac = ag;
+            if (++g < gend) {
+                code = __ldg(&in.pbc[g]);
+                if (xr) ag = __ldg(&anchor[gslot + g]);
+            }
+            cx[cg * N + b] = q;
+            if (xr) put_rel(xr, cg * N + b, q, ac, xmode, b);
         }
-        if (xb) {
-            const double4 q = xb[s];
+        if (CHECK && in.xq) {
+            const float4 r = xr[s], q = in.xq[s];
+            const float dx = r.x - q.x, dy = r.y - q.y, dz = r.z - q.z;
+            if (dx * dx + dy * dy + dz * dz > in.qlim2) *in.qflag = 1;
+        }
+        if (CHECK && in.xb) {
+            const double4 q = in.xb[s];
             const double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-            if (dx * dx + dy * dy + dz * dz > lim2) *flag = 1;
+            if (dx * dx + dy * dy + dz * dz > in.lim2) {
+                if (!in.cond) *in.flag = 1;
+                else if (atomicExch(in.flag, 1) == 0) cudaGraphSetConditional(in.cond, 1u);
+            }
         }
     }
     cv[s] = v;
 }
 
-template <bool FINAL, bool INITIAL>
-__global__ void k_cp_integrate(int M, int N, const int* __restrict__ cnt, double dtf, double dt,
+template <bool FINAL, bool INITIAL, bool CHECK>
+__global__ void __launch_bounds__(MDB_NTHREADS, 4) k_cp_integrate(int M, int N, const int* __restrict__ cnt, double dtf, double dt,
     double4* cx, double4* cv, const double4* __restrict__ cf, const float4* __restrict__ cf32,
-    const float4* __restrict__ anchor, float4* xr, int xmode, const double4* __restrict__ xb,
-    double lim2, int* flag, const float4* __restrict__ xq, float qlim2, int* qflag)
+    const float4* __restrict__ anchor, float4* xr, int xmode, CpInitial in)
 {
-    cp_integrate_slot<FINAL, INITIAL>(blockIdx.x * blockDim.x + threadIdx.x, M, N, cnt, dtf, dt,
-        cx, cv, cf, const_cast<float4*>(cf32), anchor, xr, false, xmode, xb, lim2, flag, xq,
-        qlim2, qflag);
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (CHECK && in.stop) {
+        if (*in.stop) return;
+        if (s == 0) atomicAdd(in.ran, 1);
+    }
+    cp_integrate_slot<FINAL, INITIAL, CHECK>(s, M, N, cnt, dtf, dt, cx, cv, cf,
+        const_cast<float4*>(cf32), anchor, xr, xmode, in);
 }
 
-template <bool FINAL, bool INITIAL>
-__global__ void k_cp_integrate_batch(const CpStepMember* __restrict__ tab,
-    const int2* __restrict__ bmap)
+template <bool FINAL, bool INITIAL, bool CHECK>
+__global__ void __launch_bounds__(MDB_NTHREADS, 4) k_cp_integrate_batch(const CpStepMember* __restrict__ tab,
+    const int2* __restrict__ bmap, int zero)
 {
     const int2 bm = __ldg(&bmap[blockIdx.x]);
     if (bm.x < 0) return;
     const CpStepMember& m = tab[bm.x];
-    cp_integrate_slot<FINAL, INITIAL>(bm.y * blockDim.x + threadIdx.x, m.M, m.N, m.cnt, m.dtf,
-        m.dt, m.cx, m.cv, m.cf, m.cf32, m.anchor, m.xr, false, m.mixed, m.xb, m.lim2, m.flag);
+    CpInitial in;
+    in.gstart = m.gstart, in.pbc = m.pbc, in.xprd = m.xprd, in.yprd = m.yprd, in.zprd = m.zprd;
+    in.zero = zero && m.zero_f;
+    if (CHECK) in.xb = m.xb, in.lim2 = m.lim2, in.flag = m.flag;
+    cp_integrate_slot<FINAL, INITIAL, CHECK>(bm.y * blockDim.x + threadIdx.x, m.M, m.N, m.cnt, m.dtf,
+        m.dt, m.cx, m.cv, m.cf, m.cf32, m.anchor, m.xr, m.mixed, in);
 }
 
 // Clearing the half-list force slots right before the force kernel (rather
@@ -876,46 +926,54 @@ void launch_zero_forces_batch(cudaStream_t s, int nblocks, const CpStepMember* t
 }
 
 void launch_cp_integrate_batch(cudaStream_t s, bool final_, bool initial, int nblocks,
-    const CpStepMember* tab, const int2* bmap)
+    const CpStepMember* tab, const int2* bmap, int zero, bool check)
 {
     if (nblocks <= 0) return;
-    if (final_ && initial)
-        k_cp_integrate_batch<true, true><<<nblocks, MDB_NTHREADS, 0, s>>>(tab, bmap);
-    else if (initial) k_cp_integrate_batch<false, true><<<nblocks, MDB_NTHREADS, 0, s>>>(tab, bmap);
-    else k_cp_integrate_batch<true, false><<<nblocks, MDB_NTHREADS, 0, s>>>(tab, bmap);
+#define CP_INT(F, I, C) \
+    k_cp_integrate_batch<F, I, C><<<nblocks, MDB_NTHREADS, 0, s>>>(tab, bmap, zero)
+    if (!initial) CP_INT(true, false, false);
+    else if (final_) check ? CP_INT(true, true, true) : CP_INT(true, true, false);
+    else check ? CP_INT(false, true, true) : CP_INT(false, true, false);
+#undef CP_INT
+    g_launches++;
+}
+
+template <bool FINAL, bool INITIAL>
+static void run_integrate(cudaStream_t s, int M, int N, int ncl_cap, const int* cnt, double dtf,
+    double dt, double4* cx, double4* cv, const double4* cf, const float4* cf32,
+    const float4* anchor, float4* xr, int xmode, const CpInitial& in)
+{
+    const int nb = mdb_blocks((long long)ncl_cap * M, MDB_NTHREADS);
+    if (INITIAL && (in.xb || in.xq || in.stop))
+        k_cp_integrate<FINAL, INITIAL, INITIAL><<<nb, MDB_NTHREADS, 0, s>>>(M, N, cnt, dtf, dt,
+            cx, cv, cf, cf32, anchor, xr, xmode, in);
+    else
+        k_cp_integrate<FINAL, INITIAL, false><<<nb, MDB_NTHREADS, 0, s>>>(M, N, cnt, dtf, dt, cx,
+            cv, cf, cf32, anchor, xr, xmode, in);
     g_launches++;
 }
 
 void launch_cp_initial(cudaStream_t s, int M, int N, int ncl_cap, const int* cnt, double dtf,
     double dt, double4* cx, double4* cv, const double4* cf, const float4* cf32,
-    const float4* anchor, float4* xr, int xmode, const double4* xb, double lim2, int* flag,
-    const float4* xq, float qlim2, int* qflag)
+    const float4* anchor, float4* xr, int xmode, const CpInitial& in)
 {
-    long long n = (long long)ncl_cap * M;
-    k_cp_integrate<false, true><<<mdb_blocks(n, MDB_NTHREADS), MDB_NTHREADS, 0, s>>>(M, N, cnt,
-        dtf, dt, cx, cv, cf, cf32, anchor, xr, xmode, xb, lim2, flag, xq, qlim2, qflag);
-    g_launches++;
+    run_integrate<false, true>(s, M, N, ncl_cap, cnt, dtf, dt, cx, cv, cf, cf32, anchor, xr,
+        xmode, in);
 }
 
 void launch_cp_final(cudaStream_t s, int M, int ncl_cap, const int* cnt, double dtf,
     const double4* cx, double4* cv, const double4* cf, const float4* cf32)
 {
-    long long n = (long long)ncl_cap * M;
-    k_cp_integrate<true, false><<<mdb_blocks(n, MDB_NTHREADS), MDB_NTHREADS, 0, s>>>(M, M, cnt,
-        dtf, 0.0, const_cast<double4*>(cx), cv, cf, cf32, nullptr, nullptr, 0, nullptr, 0.0,
-        nullptr, nullptr, 0.f, nullptr);
-    g_launches++;
+    run_integrate<true, false>(s, M, M, ncl_cap, cnt, dtf, 0.0, const_cast<double4*>(cx), cv, cf,
+        cf32, nullptr, nullptr, 0, CpInitial());
 }
 
 void launch_cp_final_initial(cudaStream_t s, int M, int N, int ncl_cap, const int* cnt,
     double dtf, double dt, double4* cx, double4* cv, const double4* cf, const float4* cf32,
-    const float4* anchor, float4* xr, int xmode, const double4* xb, double lim2, int* flag,
-    const float4* xq, float qlim2, int* qflag)
+    const float4* anchor, float4* xr, int xmode, const CpInitial& in)
 {
-    long long n = (long long)ncl_cap * M;
-    k_cp_integrate<true, true><<<mdb_blocks(n, MDB_NTHREADS), MDB_NTHREADS, 0, s>>>(M, N, cnt,
-        dtf, dt, cx, cv, cf, cf32, anchor, xr, xmode, xb, lim2, flag, xq, qlim2, qflag);
-    g_launches++;
+    run_integrate<true, true>(s, M, N, ncl_cap, cnt, dtf, dt, cx, cv, cf, cf32, anchor, xr, xmode,
+        in);
 }
 
 // ---- thermo: computeThermo (common/thermo.c:60-100) over the atom arrays ------------

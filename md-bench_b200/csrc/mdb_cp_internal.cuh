@@ -188,21 +188,35 @@ int launch_force_mixed(cudaStream_t s, int N, int half, int energy, int ncl_cap,
 // threads per block and block count of a mixed force launch
 int force_mixed_threads(const Types& ty);
 int force_mixed_grid(int ncl_cap, const Types& ty);
+// half-list systems of at most this many i-slots clear the force slots in the
+// integrator: its streams (160 B a slot) and the slots then stay in L2 together
+#define CP_ZERO_SLOTS (1 << 18)
+
+// what an initial integration does besides (cp_integrate_slot)
+struct CpInitial {
+    const int* gstart = nullptr; // ghost update (null: none)
+    const int* pbc    = nullptr;
+    double xprd = 0, yprd = 0, zprd = 0;
+    int zero          = 0;       // clear the force slots
+    const double4* xb = nullptr; // displacement check (null: none)
+    double lim2       = 0;
+    int* flag         = nullptr;
+    cudaGraphConditionalHandle cond = 0;
+    const int* stop   = nullptr; // a step graph's stop flag and step counter
+    int* ran          = nullptr;
+    const float4* xq  = nullptr; // positions of the pair codes (null: none)
+    float qlim2       = 0;
+    int* qflag        = nullptr;
+};
 // xmode: the put_rel mode of xr (ignored when xr is null)
-// xb (null: no check): slot positions at the last build; a slot farther than
-// sqrt(lim2) from it sets *flag (the displacement check of a rebuild policy)
-// xq (null: no check): the mixed positions the pair codes were derived from;
-// a slot farther than sqrt(qlim2) from it sets *qflag (the pair-list path)
 void launch_cp_initial(cudaStream_t s, int M, int N, int ncl_cap, const int* cnt, double dtf,
     double dt, double4* cx, double4* cv, const double4* cf, const float4* cf32,
-    const float4* anchor, float4* xr, int xmode, const double4* xb, double lim2, int* flag,
-    const float4* xq = nullptr, float qlim2 = 0.f, int* qflag = nullptr);
+    const float4* anchor, float4* xr, int xmode, const CpInitial& in);
 void launch_cp_final(cudaStream_t s, int M, int ncl_cap, const int* cnt, double dtf,
     const double4* cx, double4* cv, const double4* cf, const float4* cf32);
 void launch_cp_final_initial(cudaStream_t s, int M, int N, int ncl_cap, const int* cnt,
     double dtf, double dt, double4* cx, double4* cv, const double4* cf, const float4* cf32,
-    const float4* anchor, float4* xr, int xmode, const double4* xb, double lim2, int* flag,
-    const float4* xq = nullptr, float qlim2 = 0.f, int* qflag = nullptr);
+    const float4* anchor, float4* xr, int xmode, const CpInitial& in);
 int ke_blocks(int n);
 
 // ---- pair-list force path (mdb_cp_pairs.cu) ---------------------------------
@@ -247,7 +261,7 @@ int launch_force_pairs(cudaStream_t s, int N, int half, int energy, int uniform,
 // of member bmap[b].x, whose buffers come from a device table. The block maps
 // are built on the host from the members' capacities, so a captured graph
 // stays valid until a member's buffers move.
-struct CpStepMember { // integrator and ghost update
+struct CpStepMember { // integrator with ghost update
     const int* cnt;
     double4* cx;
     double4* cv;
@@ -255,13 +269,12 @@ struct CpStepMember { // integrator and ghost update
     float4* cf32;
     const float4* anchor;
     float4* xr;
-    const int* border;
+    const int* gstart;
     const int* pbc;
-    const int* jnat;
     double dtf, dt, xprd, yprd, zprd;
     int M, N, mixed; // mixed: 0 FP64, else the xr mode of put_rel
     int zero_f; // half lists: the force slots are cleared before each force evaluation
-    const double4* xb; // displacement check (null: off), see launch_cp_initial
+    const double4* xb; // displacement check (null: off), see CpInitial
     double lim2;
     int* flag;
 };
@@ -335,15 +348,14 @@ void launch_snapshot_batch(cudaStream_t s, int nblocks, const CpStepMember* tab,
 // every member's CP_SLOTS counters into out[member * CP_SLOTS + k]
 void launch_counters_batch(cudaStream_t s, int nmem, const CpBuildMember* tab, int* out);
 
+// initial: with the members' ghost updates and checks; zero: half-list members
+// clear their force slots; check: some member has a displacement check
 void launch_cp_integrate_batch(cudaStream_t s, bool final_, bool initial, int nblocks,
-    const CpStepMember* tab, const int2* bmap);
+    const CpStepMember* tab, const int2* bmap, int zero, bool check);
 // half-list members (zero_f): force slots [0, ncl * M) to zero, over the
 // integrator's block map; launched right before the force evaluation
 void launch_zero_forces_batch(cudaStream_t s, int nblocks, const CpStepMember* tab,
     const int2* bmap);
-// skip: null, or a flag per member (set = the member skips the update)
-void launch_ghost_update_batch(cudaStream_t s, int nblocks, const CpStepMember* tab,
-    const int2* bmap, const int* skip);
 void launch_force_mixed_batch(cudaStream_t s, int N, int half, int energy, const Types& ty,
     float cutforcesq, int nblocks, const CpForceMember* tab, const int2* bmap);
 void launch_ke_atoms(cudaStream_t s, int n, const double4* av, double mass, double* partials);
