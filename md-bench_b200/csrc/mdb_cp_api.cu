@@ -40,6 +40,7 @@ struct MdbCp {
     Geom g;
     std::vector<int> stencil;
     Types ty;
+    bool tuned        = false; // the force kernel's launch shape was set by the caller
     double cutforcesq = 0;
     double t_scale = 1, dof_boltz = 1, p_scale = 1;
 
@@ -70,7 +71,10 @@ struct MdbCp {
     int *list = nullptr, *numneigh = nullptr, *nmasked = nullptr;
     // counters, scratch, reductions
     int* cnt                 = nullptr;
+    // one block of everything a rebuild starts from zero: zext, then col_count,
+    // col_fill, ncl_col, gcol_count and gfill (each of the column grid's size)
     unsigned long long* zext = nullptr;
+    size_t zero_bytes        = 0;
     int* scan_scratch        = nullptr;
     int scan_scratch_n       = 0;
     double* partials         = nullptr; // npart for energy + npart for ke
@@ -270,6 +274,35 @@ static void setup_columns(MdbCp* ctx)
     }
 }
 
+// The mixed force kernel's launch shape for a system of n atoms, as measured on
+// B200 (us per evaluation, half lists with the clearing of their slots).
+// One warp for four i-clusters shares set-up and reduction and pays once its
+// warps fill the chip; below that a warp for one or two shortens the chain of
+// iterations over a row: 840 atoms 12.3 -> 8.2 with one, 16,384 13.3 -> 11.3,
+// 45,356 18.1 -> 17.2, 87,808 26.7 -> 24.5 with two, 256,000 48.5 both (four
+// types: 2,000 18.5 -> 8.2, 87,808 29.0 -> 28.7). Full lists keep four at every
+// size: the shape sets the rounding of a sum, and a member of an ensemble must
+// follow its run alone bit for bit (ensembles of half lists, whose atomics round
+// in any order, take the large shape for all members).
+// Two j atoms per lane (one 256-bit load) except for 4x8 half lists of one type
+// (57.5 against 58.8 at 256,000).
+// The 64-register budget (variant 2) holds eight blocks of 128 threads on an SM:
+// one type, 1M atoms 162 against 240 without (half), 199 against 231 (full), but
+// 16.1 against 14.4 at 45,356 (full). Several types spill under it: 256,000 atoms
+// 67.4 -> 59.7 (half), 78.0 -> 63.3 (full) without; from half a million atoms on
+// latency counts more: full 268 -> 262 with it at 1M, and 4x4 half lists with
+// eight clusters per warp and one j atom per lane 442 -> 412 at 2M.
+static void set_force_shape(Types& t, int N, int half, int n)
+{
+    const bool large = n > (1 << 19);
+    t.force_cpw   = !half ? 4 : n <= 16384 ? 1 : n <= 131072 ? 2 : 4;
+    t.force_jpl   = t.uniform && N == 8 && half ? 1 : 2; // with four per warp
+    t.force_block = t.uniform ? 128 : 64;
+    if (t.uniform) t.force_variant = half ? (t.force_cpw > 1 ? 2 : 0) : (n > 65536 ? 2 : 0);
+    else t.force_variant = large && N == 4 ? 2 : 0;
+    if (!t.uniform && half && large && N == 4) t.force_cpw = 8;
+}
+
 // computePerTypeLJParameters (common/parameter.c:31-45): per-type sqrt(eps)
 // and sigma^3; pairs mix geometrically (clusterpair/force_lj.c:130-132)
 static int setup_types(MdbCp* ctx)
@@ -291,17 +324,8 @@ static int setup_types(MdbCp* ctx)
     }
     t.uniform     = uniform ? 1 : 0;
     t.force_block   = 128;
-    t.force_variant = 2; // measured fastest on B200 at 1M atoms (4x4 and 4x8, full and half)
     t.force_swizzle = 0;
-    // four i-clusters per warp: measured fastest on B200 at 1M atoms (4x4 and
-    // 4x8, full and half; 170 us against 229 us per launch for one per warp)
-    t.force_cpw     = 4;
-    // two j atoms per lane (one 256-bit load), one atom type: at 1M atoms 189
-    // against 200 us per launch for 4x4 full lists, 159 against 164 us for
-    // 4x4 half lists; 4x8 half lists 188 against 182 us; several types (their
-    // per-atom tables take the registers) 2.83e9 against 3.65e9 atom-steps/s
-    // on the 4-type liquid
-    t.force_jpl     = (t.uniform && (ctx->N == 4 || !ctx->p.half_neigh)) ? 2 : 1;
+    set_force_shape(t, ctx->N, ctx->p.half_neigh, ctx->p.natoms);
     t.eps0        = t.sqrt_eps[0] * t.sqrt_eps[0];
     t.sigma6_0 = t.sigma3[0] * t.sigma3[0];
     // the pair-list path's constants (geometric mixing, in FP64 then rounded)
@@ -332,7 +356,7 @@ extern "C" int mdb_cp_tune(MdbCp* ctx, const char* key, int value)
     if (!strcmp(key, "force_block")) {
         if (value < 32 || value > 512 || value % 32) return MDB_ERR_ARG;
         drop_graph(ctx);
-        ctx->ty.force_block = value;
+        ctx->ty.force_block = value, ctx->tuned = true;
         return MDB_OK;
     }
     if (!strcmp(key, "force_swizzle")) {
@@ -346,20 +370,20 @@ extern "C" int mdb_cp_tune(MdbCp* ctx, const char* key, int value)
         if (value != 1 && value != 2 && value != 4 && !(value == 8 && ctx->N == 4))
             return MDB_ERR_ARG;
         drop_graph(ctx);
-        ctx->ty.force_cpw = value;
+        ctx->ty.force_cpw = value, ctx->tuned = true;
         return MDB_OK;
     }
     if (!strcmp(key, "force_jpl")) {
         // 2: single systems with force_cpw 4
         if (value != 1 && value != 2) return MDB_ERR_ARG;
         drop_graph(ctx);
-        ctx->ty.force_jpl = value;
+        ctx->ty.force_jpl = value, ctx->tuned = true;
         return MDB_OK;
     }
     if (!strcmp(key, "force_variant")) {
         if (value < 0 || value > 3) return MDB_ERR_ARG;
         drop_graph(ctx);
-        ctx->ty.force_variant = value;
+        ctx->ty.force_variant = value, ctx->tuned = true;
         return MDB_OK;
     }
     if (!strcmp(key, "pair_variant")) {
@@ -442,14 +466,14 @@ extern "C" int mdb_cp_synchronize(MdbCp* ctx)
 
 static void free_all(MdbCp* ctx)
 {
-    dfree(ctx->ax), dfree(ctx->av), dfree(ctx->atom_col), dfree(ctx->col_count);
-    dfree(ctx->col_start), dfree(ctx->col_fill), dfree(ctx->col_atoms), dfree(ctx->col_sorted);
-    dfree(ctx->gidx), dfree(ctx->gz), dfree(ctx->ncl_col), dfree(ctx->cl_start);
+    dfree(ctx->ax), dfree(ctx->av), dfree(ctx->atom_col);
+    dfree(ctx->col_start), dfree(ctx->col_atoms), dfree(ctx->col_sorted);
+    dfree(ctx->gidx), dfree(ctx->gz), dfree(ctx->cl_start);
     dfree(ctx->cx), dfree(ctx->cv), dfree(ctx->cf), dfree(ctx->xr), dfree(ctx->cf32);
     dfree(ctx->anchor), dfree(ctx->inat), dfree(ctx->cbin), dfree(ctx->cl_first);
     dfree(ctx->jnat), dfree(ctx->ibbmin), dfree(ctx->ibbmax), dfree(ctx->jbbmin);
     dfree(ctx->jbbmax), dfree(ctx->gcount), dfree(ctx->gstart), dfree(ctx->border);
-    dfree(ctx->pbc), dfree(ctx->gcolumn), dfree(ctx->gcol_count), dfree(ctx->gfill);
+    dfree(ctx->pbc), dfree(ctx->gcolumn);
     dfree(ctx->jcol_n), dfree(ctx->jcol_start), dfree(ctx->gtmp), dfree(ctx->jcol);
     dfree(ctx->ztab);
     dfree(ctx->jcbbmin), dfree(ctx->jcbbmax), dfree(ctx->jcbbf), dfree(ctx->cxf);
@@ -489,21 +513,23 @@ static int alloc_columns(MdbCp* ctx)
 {
     cudaError_t e;
     const int mb1 = ctx->g.mbins + 1;
-    dfree(ctx->stencil_d), dfree(ctx->col_count), dfree(ctx->col_start), dfree(ctx->col_fill);
-    dfree(ctx->ncl_col), dfree(ctx->cl_start), dfree(ctx->gcol_count), dfree(ctx->gfill);
+    dfree(ctx->stencil_d), dfree(ctx->zext), dfree(ctx->col_start), dfree(ctx->cl_start);
     dfree(ctx->jcol_n), dfree(ctx->jcol_start), dfree(ctx->ztab);
+    ctx->zero_bytes = sizeof(unsigned long long) + 5 * sizeof(int) * (size_t)mb1;
     if ((e = dalloc(&ctx->stencil_d, ctx->g.nstencil)) != cudaSuccess ||
-        (e = dalloc(&ctx->col_count, mb1)) != cudaSuccess ||
+        (e = dalloc(&ctx->zext, (ctx->zero_bytes + 7) / 8)) != cudaSuccess ||
         (e = dalloc(&ctx->col_start, mb1 + 1)) != cudaSuccess ||
-        (e = dalloc(&ctx->col_fill, mb1)) != cudaSuccess ||
-        (e = dalloc(&ctx->ncl_col, mb1)) != cudaSuccess ||
         (e = dalloc(&ctx->cl_start, mb1 + 1)) != cudaSuccess ||
-        (e = dalloc(&ctx->gcol_count, mb1)) != cudaSuccess ||
-        (e = dalloc(&ctx->gfill, mb1)) != cudaSuccess ||
         (e = dalloc(&ctx->jcol_n, mb1)) != cudaSuccess ||
         (e = dalloc(&ctx->jcol_start, mb1 + 1)) != cudaSuccess ||
         (e = dalloc(&ctx->ztab, (size_t)ctx->g.mbins * (ctx->g.zq + 2))) != cudaSuccess)
         return fail(ctx, MDB_ERR_NOMEM, "device allocation (columns)", e);
+    int* z          = reinterpret_cast<int*>(ctx->zext + 1);
+    ctx->col_count  = z;
+    ctx->col_fill   = z + mb1;
+    ctx->ncl_col    = z + 2 * (size_t)mb1;
+    ctx->gcol_count = z + 3 * (size_t)mb1;
+    ctx->gfill      = z + 4 * (size_t)mb1;
     if ((e = cudaMemcpy(ctx->stencil_d, ctx->stencil.data(), sizeof(int) * ctx->g.nstencil,
              cudaMemcpyHostToDevice)) != cudaSuccess)
         return fail(ctx, MDB_ERR_CUDA, "stencil copy", e);
@@ -564,7 +590,6 @@ extern "C" int mdb_cp_create(const MdbParams* params, int cluster_n, int prune_e
             goto bad;
         }
         if ((e = dalloc(&ctx->cnt, CP_SLOTS)) != cudaSuccess ||
-            (e = dalloc(&ctx->zext, 1)) != cudaSuccess ||
             (e = dalloc(&ctx->red, 4 * RED_SLOTS)) != cudaSuccess ||
             (e = cudaMallocHost((void**)&ctx->h_cnt, CP_SLOTS * sizeof(int))) != cudaSuccess ||
             (e = cudaMallocHost((void**)&ctx->h_red, 4 * RED_SLOTS * sizeof(double))) !=
@@ -820,10 +845,9 @@ static void enq_clusters(MdbCp* ctx)
     cudaStream_t s = ctx->s;
     const Geom& g  = ctx->g;
     const int mb1  = g.mbins + 1;
-    cudaMemsetAsync(ctx->col_count, 0, sizeof(int) * mb1, s);
-    cudaMemsetAsync(ctx->col_fill, 0, sizeof(int) * mb1, s);
-    cudaMemsetAsync(ctx->ncl_col, 0, sizeof(int) * mb1, s);
-    cudaMemsetAsync(ctx->zext, 0, sizeof(unsigned long long), s);
+    // with the ghost columns' counts, which enq_bin_j reads (and clears again
+    // when the stages run one by one)
+    cudaMemsetAsync(ctx->zext, 0, ctx->zero_bytes, s);
     launch_bin_atoms(s, ctx->nlocal, ctx->ax, g, ctx->atom_col, ctx->col_count, ctx->cnt);
     scan_exclusive(ctx->col_count, ctx->col_start, g.mbins, ctx->scan_scratch, s);
     launch_scatter_atoms(s, ctx->nlocal, ctx->atom_col, ctx->col_start, ctx->col_fill,
@@ -837,10 +861,10 @@ static void enq_clusters(MdbCp* ctx)
         ctx->cnt, ctx->zext);
 }
 
-static void enq_setup_pbc(MdbCp* ctx)
+static void enq_setup_pbc(MdbCp* ctx, bool cleared = false)
 {
     cudaStream_t s = ctx->s;
-    cudaMemsetAsync(ctx->cnt + CP_NGHOST_ATOMS, 0, sizeof(int), s);
+    if (!cleared) cudaMemsetAsync(ctx->cnt + CP_NGHOST_ATOMS, 0, sizeof(int), s);
     launch_ghost_count(s, ctx->ncj_cap, ctx->cnt, ctx->jnat, ctx->jbbmin, ctx->jbbmax, ctx->g,
         ctx->gcount);
     scan_exclusive(ctx->gcount, ctx->gstart, ctx->ncj_cap, ctx->scan_scratch, s);
@@ -850,12 +874,12 @@ static void enq_setup_pbc(MdbCp* ctx)
         ctx->g, ctx->cx, ctx->jnat, ctx->jbbmin, ctx->jbbmax, ctx->anchor, ctx->xr, ctx->zext);
 }
 
-static void enq_bin_j(MdbCp* ctx)
+// cleared: enq_clusters has just run
+static void enq_bin_j(MdbCp* ctx, bool cleared = false)
 {
     cudaStream_t s = ctx->s;
     const int mb1  = ctx->g.mbins + 1;
-    cudaMemsetAsync(ctx->gcol_count, 0, sizeof(int) * mb1, s);
-    cudaMemsetAsync(ctx->gfill, 0, sizeof(int) * mb1, s);
+    if (!cleared) cudaMemsetAsync(ctx->gcol_count, 0, 2 * sizeof(int) * (size_t)mb1, s);
     launch_ghost_columns(s, ctx->N, ctx->ngc_cap, ctx->cnt, ctx->pbc, ctx->jnat, ctx->cx, ctx->g,
         ctx->gcolumn, ctx->gcol_count);
     launch_column_sizes(s, mb1, ctx->jfac, ctx->ncl_col, ctx->gcol_count, ctx->jcol_n);
@@ -890,10 +914,11 @@ static void clear_build_counters(MdbCp* ctx)
 // buildClusters .. buildNeighbor from the atom arrays (idempotent)
 static void enq_build(MdbCp* ctx)
 {
-    clear_build_counters(ctx);
+    // CP_NGHOST_ATOMS, CP_MAXNEED, CP_BADBIN
+    cudaMemsetAsync(ctx->cnt + CP_NGHOST_ATOMS, 0, 3 * sizeof(int), ctx->s);
     enq_clusters(ctx);
-    enq_setup_pbc(ctx);
-    enq_bin_j(ctx);
+    enq_setup_pbc(ctx, true);
+    enq_bin_j(ctx, true);
     enq_list(ctx);
 }
 
@@ -2093,6 +2118,16 @@ static void ens_body(MdbCp* c, int kind)
     }
 }
 
+// a member's types and launch shape in an ensemble: half lists that the caller
+// has not tuned take the shape of a large system, as the members fill the chip
+// together
+static Types ens_types(const MdbCp* c)
+{
+    Types t = c->ty;
+    if (c->p.half_neigh && !c->tuned) set_force_shape(t, c->N, 1, 1 << 30);
+    return t;
+}
+
 static bool same_types(const Types& a, const Types& b)
 {
     if (a.ntypes != b.ntypes || a.uniform != b.uniform || a.eps0 != b.eps0 ||
@@ -2129,7 +2164,7 @@ static int ens_dyn_maps(MdbCpEnsemble* e)
         for (int k = 0; k < n; k++) {
             if (e->gid[k] != (int)q) continue;
             const MdbCp* c = e->m[k];
-            const int nb   = force_mixed_grid(c->h_cnt[CP_NCL], c->ty);
+            const int nb   = force_mixed_grid(c->h_cnt[CP_NCL], e->groups[q].ty);
             for (int b = 0; b < nb && w < end; b++) h[w++] = make_int2(k, b);
         }
         while (w < end) h[w++] = make_int2(-1, 0);
@@ -2213,12 +2248,12 @@ static int ens_tables(MdbCpEnsemble* e)
         for (size_t q = 0; q < e->groups.size() && gid[k] < 0; q++) {
             const auto& gr = e->groups[q];
             if (gr.N == c->N && gr.half == c->p.half_neigh && gr.cutsq == cutsq &&
-                same_types(gr.ty, c->ty))
+                same_types(gr.ty, ens_types(c)))
                 gid[k] = (int)q;
         }
         if (gid[k] < 0) {
             gid[k] = (int)e->groups.size();
-            e->groups.push_back({c->N, c->p.half_neigh, c->ty, cutsq, 0, 0});
+            e->groups.push_back({c->N, c->p.half_neigh, ens_types(c), cutsq, 0, 0});
         }
     }
     for (size_t q = 0; q < e->groups.size(); q++) {
@@ -2227,7 +2262,7 @@ static int ens_tables(MdbCpEnsemble* e)
         for (int k = 0; k < n; k++)
             if (gid[k] == (int)q) {
                 MdbCp* c         = e->m[k];
-                const int nb     = force_mixed_grid(c->ncl_cap, c->ty);
+                const int nb     = force_mixed_grid(c->ncl_cap, gr.ty);
                 c->energy_blocks = nb; // the partials a batched energy launch writes
                 add(k, nb);
             }
@@ -2513,8 +2548,8 @@ static int ens_map_info(MdbCpEnsemble* e)
         const MdbCp* c = e->m[k];
         info[4 * k]     = c->M;
         info[4 * k + 1] = e->gid[k];
-        info[4 * k + 2] = c->ty.force_cpw;
-        info[4 * k + 3] = force_mixed_threads(c->ty);
+        info[4 * k + 2] = e->groups[e->gid[k]].ty.force_cpw;
+        info[4 * k + 3] = force_mixed_threads(e->groups[e->gid[k]].ty);
     }
     std::vector<size_t> goff(std::max(ng, 1));
     std::vector<int> gnb(std::max(ng, 1));
