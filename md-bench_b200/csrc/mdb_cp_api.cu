@@ -69,6 +69,7 @@ struct MdbCp {
     int* stencil_d = nullptr;
     // list
     int *list = nullptr, *numneigh = nullptr, *nmasked = nullptr;
+    int* row_order = nullptr; // i-clusters by row length (mixed)
     // counters, scratch, reductions
     int* cnt                 = nullptr;
     // one block of everything a rebuild starts from zero: zext, then col_count,
@@ -478,7 +479,7 @@ static void free_all(MdbCp* ctx)
     dfree(ctx->ztab);
     dfree(ctx->jcbbmin), dfree(ctx->jcbbmax), dfree(ctx->jcbbf), dfree(ctx->cxf);
     dfree(ctx->stencil_d), dfree(ctx->list), dfree(ctx->numneigh), dfree(ctx->nmasked);
-    dfree(ctx->xbuild), dfree(ctx->dflag);
+    dfree(ctx->row_order), dfree(ctx->xbuild), dfree(ctx->dflag);
     dfree(ctx->pcode), dfree(ctx->pcnt), dfree(ctx->xq), dfree(ctx->qflag);
     ctx->pair_ncl = ctx->pair_chmax = 0;
     if (ctx->h_dflag) cudaFreeHost(ctx->h_dflag);
@@ -623,6 +624,7 @@ static int alloc_atoms(MdbCp* ctx, int n)
     dfree(ctx->col_sorted), dfree(ctx->gidx), dfree(ctx->gz), dfree(ctx->inat), dfree(ctx->cbin);
     dfree(ctx->cl_first), dfree(ctx->ibbmin), dfree(ctx->ibbmax), dfree(ctx->gcount);
     dfree(ctx->gstart), dfree(ctx->numneigh), dfree(ctx->nmasked), dfree(ctx->list);
+    dfree(ctx->row_order);
     dfree(ctx->scan_scratch), dfree(ctx->partials), dfree(ctx->stage), dfree(ctx->stage_i);
     int scan_n          = std::max(std::max(mb + 2, ctx->ncj_cap + 1), 1);
     ctx->scan_scratch_n = scan_scratch_ints(scan_n);
@@ -644,6 +646,7 @@ static int alloc_atoms(MdbCp* ctx, int n)
         (e = dalloc(&ctx->gstart, ctx->ncj_cap + 1)) != cudaSuccess ||
         (e = dalloc(&ctx->numneigh, ctx->ncl_cap)) != cudaSuccess ||
         (e = dalloc(&ctx->nmasked, ctx->ncl_cap)) != cudaSuccess ||
+        (e = dalloc(&ctx->row_order, ctx->mixed ? ctx->ncl_cap : 0)) != cudaSuccess ||
         (e = dalloc(&ctx->list, (size_t)ctx->maxneighs * ctx->ld)) != cudaSuccess ||
         (e = dalloc(&ctx->scan_scratch, ctx->scan_scratch_n)) != cudaSuccess ||
         (e = dalloc(&ctx->partials, 2 * (size_t)ctx->npart)) != cudaSuccess ||
@@ -903,6 +906,8 @@ static void enq_list(MdbCp* ctx)
         ctx->stencil_d, ctx->cbin, ctx->ibbmin, ctx->ibbmax, ctx->jcbbmin, ctx->jcbbmax, ctx->cx,
         ctx->jcbbf, ctx->cxf, ctx->jcol, ctx->ztab, ctx->zext, ctx->maxneighs, lks(ctx),
         lcs(ctx), ctx->list, ctx->numneigh, ctx->nmasked, ctx->cnt);
+    if (ctx->mixed)
+        launch_order_rows(ctx->s, ctx->ncl_cap, ctx->cnt, ctx->numneigh, ctx->row_order);
 }
 
 static void clear_build_counters(MdbCp* ctx)
@@ -1055,7 +1060,7 @@ static void enq_force(MdbCp* ctx, bool energy, bool zeroed = false)
     } else if (ctx->mixed) {
         const int nb = launch_force_mixed(s, ctx->N, ctx->p.half_neigh, energy, ctx->ncl_cap,
             ctx->cnt, ctx->xr, ctx->anchor, ctx->ty, (float)ctx->cutforcesq, ctx->list, lks(ctx),
-            lcs(ctx), ctx->numneigh, ctx->cf32, ctx->partials);
+            lcs(ctx), ctx->numneigh, ctx->row_order, ctx->cf32, ctx->partials);
         if (energy) ctx->energy_blocks = nb;
     } else {
         launch_force_fp64(s, ctx->M, ctx->N, ctx->p.half_neigh, energy, ctx->ncl_cap, ctx->cnt,
@@ -2203,7 +2208,7 @@ static int ens_tables(MdbCpEnsemble* e)
         a.flag   = nullptr; // set once the flags exist, below
         CpForceMember& f = fo[k];
         f.cnt = c->cnt, f.xr = c->xr, f.anchor = c->anchor, f.list = c->list;
-        f.numneigh = c->numneigh, f.cf32 = c->cf32, f.epart = c->partials, f.cs = lcs(c);
+        f.numneigh = c->numneigh, f.row_order = c->row_order, f.cf32 = c->cf32, f.epart = c->partials, f.cs = lcs(c);
         f.pad = 0;
     }
     std::vector<CpBuildMember> bt(n);
@@ -2226,7 +2231,7 @@ static int ens_tables(MdbCpEnsemble* e)
         b.gtmp = c->gtmp, b.jcol = c->jcol, b.jcbbmin = c->jcbbmin, b.jcbbmax = c->jcbbmax;
         b.jcbbf = c->jcbbf, b.cxf = c->cxf, b.slot_cap = c->slot_cap, b.ztab = c->ztab;
         b.stencil = c->stencil_d, b.list = c->list, b.numneigh = c->numneigh;
-        b.nmasked = c->nmasked;
+        b.nmasked = c->nmasked, b.row_order = c->row_order;
     }
     for (int st = 0; st < CB_COUNT; st++) {
         e->off_stage[st] = maps.size();
@@ -2391,6 +2396,7 @@ static void ens_rebuild_stages(MdbCpEnsemble* e, const int* only)
     stage(CB_MERGE);
     stage(CB_PREP);
     stage(CB_LIST);
+    stage(CB_ORDER);
     launch_counters_batch(e->s, n, e->d_build, e->d_cnt_all);
 }
 

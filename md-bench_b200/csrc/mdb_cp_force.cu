@@ -391,8 +391,8 @@ template <int N, bool HALF, bool ENERGY, bool UNIFORM, int PF, int CPW, int JPL>
 __device__ __forceinline__ void force_mixed_block(int bid, const int* __restrict__ cnt,
     const float4* __restrict__ xr, const float4* __restrict__ anchor, const Types& ty,
     float cutforcesq, const int* __restrict__ list, int ks, int cs,
-    const int* __restrict__ numneigh, float4* cf32, double* epart, const float* s_se,
-    const float* s_s3)
+    const int* __restrict__ numneigh, const int* __restrict__ row_order, float4* cf32,
+    double* epart, const float* s_se, const float* s_s3)
 {
     constexpr int L   = 32 / CPW;  // lanes per i-cluster
     constexpr int LPE = N / JPL;   // lanes per list entry
@@ -400,9 +400,11 @@ __device__ __forceinline__ void force_mixed_block(int bid, const int* __restrict
     static_assert(JPW >= 1, "a segment holds at least one list entry");
     const int lane = threadIdx.x & 31;
     const int l    = lane & (L - 1);
-    const int ci   = ((bid * blockDim.x + threadIdx.x) >> 5) * CPW + lane / L;
+    // the segment's i-cluster: rows of one length beside one another (row_order)
+    const int pos  = ((bid * blockDim.x + threadIdx.x) >> 5) * CPW + lane / L;
     const int ncl  = cnt[CP_NCL];
-    const bool act = ci < ncl;
+    const bool act = pos < ncl;
+    const int ci   = CPW > 1 && act ? __ldg(&row_order[pos]) : pos;
     double e       = 0.0;
     if (__any_sync(0xffffffffu, act)) {
         const int cic    = act ? ci : 0; // address arithmetic of inactive segments
@@ -578,14 +580,15 @@ __global__ void __launch_bounds__(MINB ? 128 : 512, MINB ? MINB : 1) k_force_mix
     const int* __restrict__ cnt,
     const float4* __restrict__ xr, const float4* __restrict__ anchor, Types ty,
     float cutforcesq, const int* __restrict__ list, int ks, int cs,
-    const int* __restrict__ numneigh, float4* cf32, double* epart, int slots)
+    const int* __restrict__ numneigh, const int* __restrict__ row_order, float4* cf32,
+    double* epart, int slots)
 {
     __shared__ float s_se[MDB_MAX_TYPES], s_s3[MDB_MAX_TYPES];
     load_type_tables(ty, s_se, s_s3);
     int bid = blockIdx.x;
     if (slots > 0) bid = (blockIdx.x % slots) * (gridDim.x / slots) + blockIdx.x / slots;
     force_mixed_block<N, HALF, ENERGY, UNIFORM, PF, CPW, JPL>(bid, cnt, xr, anchor, ty, cutforcesq,
-        list, ks, cs, numneigh, cf32, epart, s_se, s_s3);
+        list, ks, cs, numneigh, row_order, cf32, epart, s_se, s_s3);
 }
 
 // all members of an ensemble group (same shape, list form, types and launch)
@@ -600,7 +603,7 @@ __global__ void __launch_bounds__(MINB ? 128 : 512, MINB ? MINB : 1) k_force_mix
     load_type_tables(ty, s_se, s_s3);
     const CpForceMember& m = tab[bm.x];
     force_mixed_block<N, HALF, ENERGY, UNIFORM, PF, CPW, JPL>(bm.y, m.cnt, m.xr, m.anchor, ty, cutforcesq,
-        m.list, 1, m.cs, m.numneigh, m.cf32, m.epart, s_se, s_s3);
+        m.list, 1, m.cs, m.numneigh, m.row_order, m.cf32, m.epart, s_se, s_s3);
 }
 
 int force_mixed_threads(const Types& ty)
@@ -684,7 +687,7 @@ void launch_force_mixed_batch(cudaStream_t s, int N, int half, int energy, const
 template <int N, bool HALF, bool ENERGY, bool UNIFORM>
 static void run_mixed(cudaStream_t s, int blocks, const int* cnt, const float4* xr,
     const float4* anchor, const Types& ty, float cutforcesq, const int* list, int ks, int cs,
-    const int* numneigh, float4* cf32, double* epart)
+    const int* numneigh, const int* row_order, float4* cf32, double* epart)
 {
     const int v  = ty.force_variant;
     const int nt = force_mixed_threads(ty);
@@ -707,7 +710,7 @@ static void run_mixed(cudaStream_t s, int blocks, const int* cnt, const float4* 
 #define CP_RUN(PF, MB, C) CP_RUNJ(PF, MB, C, 1)
 #define CP_RUNJ(PF, MB, C, J)                                                            \
     k_force_mixed<N, HALF, ENERGY, UNIFORM, PF, MB, C, J><<<nb, nt, 0, s>>>(cnt, xr, anchor, \
-        ty, cutforcesq, list, ks, cs, numneigh, cf32, epart, slots)
+        ty, cutforcesq, list, ks, cs, numneigh, row_order, cf32, epart, slots)
     // several clusters per warp: prefetch depth 1; bit 0 of the variant
     // lowers the register budget's block count from 8 to 6
     if (ty.force_cpw == 2) {
@@ -743,28 +746,28 @@ static void run_mixed(cudaStream_t s, int blocks, const int* cnt, const float4* 
 template <int N, bool HALF>
 static void run_mixed_e(cudaStream_t s, int blocks, int energy, const int* cnt, const float4* xr,
     const float4* anchor, const Types& ty, float cutforcesq, const int* list, int ks, int cs,
-    const int* numneigh, float4* cf32, double* epart)
+    const int* numneigh, const int* row_order, float4* cf32, double* epart)
 {
     if (ty.uniform) {
-        if (energy) run_mixed<N, HALF, true, true>(s, blocks, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, cf32, epart);
-        else run_mixed<N, HALF, false, true>(s, blocks, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, cf32, epart);
+        if (energy) run_mixed<N, HALF, true, true>(s, blocks, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, row_order, cf32, epart);
+        else run_mixed<N, HALF, false, true>(s, blocks, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, row_order, cf32, epart);
     } else {
-        if (energy) run_mixed<N, HALF, true, false>(s, blocks, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, cf32, epart);
-        else run_mixed<N, HALF, false, false>(s, blocks, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, cf32, epart);
+        if (energy) run_mixed<N, HALF, true, false>(s, blocks, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, row_order, cf32, epart);
+        else run_mixed<N, HALF, false, false>(s, blocks, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, row_order, cf32, epart);
     }
 }
 
 int launch_force_mixed(cudaStream_t s, int N, int half, int energy, int ncl_cap,
     const int* cnt, const float4* xr, const float4* anchor, const Types& ty, float cutforcesq,
-    const int* list, int ks, int cs, const int* numneigh, float4* cf32, double* epart)
+    const int* list, int ks, int cs, const int* numneigh, const int* row_order, float4* cf32, double* epart)
 {
     const int blocks = force_mixed_grid(ncl_cap, ty);
     if (N == 4) {
-        if (half) run_mixed_e<4, true>(s, blocks, energy, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, cf32, epart);
-        else run_mixed_e<4, false>(s, blocks, energy, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, cf32, epart);
+        if (half) run_mixed_e<4, true>(s, blocks, energy, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, row_order, cf32, epart);
+        else run_mixed_e<4, false>(s, blocks, energy, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, row_order, cf32, epart);
     } else {
-        if (half) run_mixed_e<8, true>(s, blocks, energy, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, cf32, epart);
-        else run_mixed_e<8, false>(s, blocks, energy, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, cf32, epart);
+        if (half) run_mixed_e<8, true>(s, blocks, energy, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, row_order, cf32, epart);
+        else run_mixed_e<8, false>(s, blocks, energy, cnt, xr, anchor, ty, cutforcesq, list, ks, cs, numneigh, row_order, cf32, epart);
     }
     g_launches++;
     return blocks;

@@ -171,6 +171,9 @@ void launch_build_list(cudaStream_t s, int M, int N, int half, int ncl_cap, cons
     const float4* jcbbf, const float4* cxf, const int* jcol, const int* ztab,
     const unsigned long long* zext, int maxneighs, int ks, int cs, int* list, int* numneigh,
     int* nmasked, int* cnt_out);
+// order: the i-clusters, every 32 consecutive ones by row length
+void launch_order_rows(cudaStream_t s, int ncl_cap, const int* cnt, const int* numneigh,
+    int* order);
 void launch_prune(cudaStream_t s, int M, int N, int ncl_cap, const int* cnt, const double4* cx,
     double cutneighsq, int maxneighs, int ks, int cs, int* list, int* numneigh, int* nmasked);
 
@@ -184,7 +187,8 @@ void launch_force_fp64(cudaStream_t s, int M, int N, int half, int energy, int n
 // returns the number of blocks launched (= energy partials written)
 int launch_force_mixed(cudaStream_t s, int N, int half, int energy, int ncl_cap,
     const int* cnt, const float4* xr, const float4* anchor, const Types& ty, float cutforcesq,
-    const int* list, int ks, int cs, const int* numneigh, float4* cf32, double* epart);
+    const int* list, int ks, int cs, const int* numneigh, const int* row_order, float4* cf32,
+    double* epart);
 // threads per block and block count of a mixed force launch
 int force_mixed_threads(const Types& ty);
 int force_mixed_grid(int ncl_cap, const Types& ty);
@@ -284,6 +288,7 @@ struct CpForceMember { // mixed force kernel (row-major lists)
     const float4* anchor;
     const int* list;
     const int* numneigh;
+    const int* row_order;
     float4* cf32;
     double* epart;
     int cs, pad;
@@ -309,7 +314,7 @@ struct CpBuildMember {
     int* ztab;
     int slot_cap;
     const int* stencil;
-    int *list, *numneigh, *nmasked;
+    int *list, *numneigh, *nmasked, *row_order;
 };
 // stages of a batched rebuild, in order; the block-map entry of each stage
 // covers every member's grid of the single-member launch
@@ -329,6 +334,7 @@ enum CpBuildStage {
     CB_MERGE,    // binJClusters: merge by bbminz
     CB_PREP,     // buildNeighbor: FP32 copies of boxes and positions, window table
     CB_LIST,     // buildNeighbor
+    CB_ORDER,    // i-clusters by row length, for the mixed force kernel
     CB_COUNT
 };
 // blocks (and threads per block) of a stage for one member
