@@ -557,24 +557,28 @@ extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const dou
     if (!ctx || nlocal < 0 || (nlocal > 0 && (!x || !v || !type))) return MDB_ERR_ARG;
     CK(cudaSetDevice(ctx->dev));
     ctx->nown = 0; // new atoms: all owned until mdb_set_owned
-    // host or device arrays (unified addressing); the types are checked here
-    std::vector<int> htype;
-    const int* th = type;
-    if (nlocal > 0) {
-        cudaPointerAttributes pa;
-        if (cudaPointerGetAttributes(&pa, type) == cudaSuccess &&
-            (pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeManaged)) {
-            htype.resize(nlocal);
-            CK(cudaMemcpy(htype.data(), type, sizeof(int) * nlocal, cudaMemcpyDefault));
-            th = htype.data();
-        }
-        cudaGetLastError();
-    }
+    // host or device arrays (unified addressing); the types are checked here, on
+    // the side where they are (the legacy stream orders the check after the work
+    // that wrote them there, as a copy to the host would)
     int maxt = 0;
-    for (int i = 0; i < nlocal; i++) {
-        if (th[i] < 0) return fail(ctx, MDB_ERR_ARG, "negative atom type");
-        maxt = std::max(maxt, th[i] + 1);
+    cudaPointerAttributes pa;
+    if (nlocal > 0 && cudaPointerGetAttributes(&pa, type) == cudaSuccess &&
+        (pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeManaged)) {
+        int range[2];
+        CK(cudaMemsetAsync(ctx->counters + CNT_TYPES, 0, sizeof range, cudaStreamLegacy));
+        const long long m = launch_mark();
+        launch_type_range(cudaStreamLegacy, nlocal, type, ctx->counters + CNT_TYPES);
+        launch_account(ctx, m);
+        CK(cudaMemcpy(range, ctx->counters + CNT_TYPES, sizeof range, cudaMemcpyDeviceToHost));
+        if (range[1]) return fail(ctx, MDB_ERR_ARG, "negative atom type");
+        maxt = range[0];
+    } else {
+        for (int i = 0; i < nlocal; i++) {
+            if (type[i] < 0) return fail(ctx, MDB_ERR_ARG, "negative atom type");
+            maxt = std::max(maxt, type[i] + 1);
+        }
     }
+    cudaGetLastError();
     int rc = setup_types(ctx, std::max(ctx->p.ntypes, maxt));
     if (rc) return rc;
     // the buffers are kept while the atom count stays within the capacity
@@ -606,6 +610,7 @@ extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const dou
         CK(cudaMemset(ctx->fz, 0, sizeof(double) * cap));
         CK(dalloc(&ctx->ghost_cnt, cap + 1));
         CK(dalloc(&ctx->ghost_off, cap + 1));
+        CK(cudaMemset(ctx->ghost_off, 0, sizeof(int) * (cap + 1)));
         CK(dalloc(&ctx->numneigh, cap));
         if (ctx->p.force_field == MDB_FF_EAM && ctx->mixed) CK(dalloc(&ctx->eam_ncut, cap));
         CK(dalloc(&ctx->local_order, cap));
@@ -678,25 +683,28 @@ extern "C" int mdb_get_atoms(MdbCtx* ctx, double* x, double* v, double* f, int* 
 
 // ---------------------------------------------------------------------------
 // enqueue helpers (no host synchronisation; safe inside stream capture)
-static void enq_initial(MdbCtx* ctx)
+// initialIntegrate, after finalIntegrate of the step before (final_); ghosts: the
+// periodic images follow (on the mixed path only their cell-relative FP32
+// positions: the FP64 ones are rebuilt with the ghost map); zero: the forces are
+// cleared for the evaluation of this step
+static void enq_initial(MdbCtx* ctx, bool final_, bool ghosts, bool zero = false)
 {
-    launch_initial_integrate(ctx->s, owned(ctx), ctx->p.dtforce, ctx->p.dt, ctx->x, ctx->vx,
-        ctx->vy, ctx->vz, ctx->fx, ctx->fy, ctx->fz, ctx->mixed ? ctx->xr : nullptr,
-        ctx->qcell, ctx->cf);
+    VlImages img;
+    img.zero = zero;
+    if (ghosts) {
+        img.off = ctx->ghost_off, img.code = ctx->pbc_code, img.counters = ctx->counters;
+        img.nlocal = ctx->nlocal;
+        img.xprd = ctx->p.xprd, img.yprd = ctx->p.yprd, img.zprd = ctx->p.zprd;
+    }
+    launch_initial_integrate(ctx->s, final_, owned(ctx), ctx->p.dtforce, ctx->p.dt, ctx->x,
+        ctx->vx, ctx->vy, ctx->vz, ctx->fx, ctx->fy, ctx->fz, ctx->mixed ? ctx->xr : nullptr,
+        ctx->qcell, ctx->cf, img);
 }
 
 static void enq_final(MdbCtx* ctx)
 {
     launch_final_integrate(ctx->s, owned(ctx), ctx->p.dtforce, ctx->vx, ctx->vy, ctx->vz,
         ctx->fx, ctx->fy, ctx->fz);
-}
-
-// finalIntegrate of the previous step fused with initialIntegrate of this one
-static void enq_final_initial(MdbCtx* ctx)
-{
-    launch_final_initial_integrate(ctx->s, owned(ctx), ctx->p.dtforce, ctx->p.dt, ctx->x,
-        ctx->vx, ctx->vy, ctx->vz, ctx->fx, ctx->fy, ctx->fz, ctx->mixed ? ctx->xr : nullptr,
-        ctx->qcell, ctx->cf);
 }
 
 // Mixed path: only the cell-relative FP32 ghost positions are refreshed
@@ -708,7 +716,8 @@ static void enq_ghost_update(MdbCtx* ctx)
         ctx->mixed ? ctx->xr : nullptr, ctx->qcell, ctx->cf);
 }
 
-static void enq_force(MdbCtx* ctx, bool energy)
+// zeroed: the integrator cleared the half-list forces
+static void enq_force(MdbCtx* ctx, bool energy, bool zeroed = false)
 {
     cudaStream_t s = ctx->s;
     int n          = owned(ctx); // rows of the owned atoms (full lists with halos)
@@ -717,18 +726,18 @@ static void enq_force(MdbCtx* ctx, bool energy)
     if (ctx->p.force_field == MDB_FF_EAM) {
         if (ctx->mixed) {
             launch_eam_mixed(s, energy, ctx->p.precision == MDB_PREC_MIXED_COMP,
-                ctx->eam_rho_lanes, n, ctx->ghost_cap, ctx->xr, ctx->shift, ctx->numneigh, ctx->neighbors, ctx->ld,
-                (float)ctx->cutforcesq, ctx->eam, ctx->border_map, ctx->counters,
+                ctx->eam_rho_lanes, n, ctx->xr, ctx->shift, ctx->numneigh, ctx->neighbors, ctx->ld,
+                (float)ctx->cutforcesq, ctx->eam, ctx->ghost_off, ctx->counters,
                 ctx->eam_cutlist, ctx->eam_ncut, ctx->fp, ctx->xe, ctx->fx, ctx->fy, ctx->fz, ep0,
                 ep1);
         } else {
-            launch_eam_fp64(s, energy, n, ctx->ghost_cap, ctx->x,
+            launch_eam_fp64(s, energy, n, ctx->x,
                 ctx->numneigh, ctx->neighbors, ctx->ld, ctx->cutforcesq, ctx->eam,
-                ctx->border_map, ctx->counters, ctx->fp, ctx->fx, ctx->fy, ctx->fz, ep0, ep1);
+                ctx->ghost_off, ctx->counters, ctx->fp, ctx->fx, ctx->fy, ctx->fz, ep0, ep1);
         }
         return;
     }
-    if (ctx->p.half_neigh) {
+    if (ctx->p.half_neigh && !zeroed) {
         cudaMemsetAsync(ctx->fx, 0, sizeof(double) * n, s);
         cudaMemsetAsync(ctx->fy, 0, sizeof(double) * n, s);
         cudaMemsetAsync(ctx->fz, 0, sizeof(double) * n, s);
@@ -751,7 +760,7 @@ static void enq_ghosts(MdbCtx* ctx)
     const MdbParams& p = ctx->p;
     launch_ghost_count(s, ctx->nlocal, ctx->x, p.cutneigh, p.xprd, p.yprd, p.zprd, p.pbc_x,
         p.pbc_y, p.pbc_z, ctx->ghost_cnt);
-    scan_exclusive(ctx->ghost_cnt, ctx->ghost_off, ctx->nlocal, ctx->scan_scratch, s);
+    scan_exclusive_steps(ctx->ghost_cnt, ctx->ghost_off, ctx->nlocal, ctx->scan_scratch, s);
     launch_ghost_write(s, ctx->nlocal, ctx->ghost_cap, ctx->x, p.cutneigh, p.xprd, p.yprd,
         p.zprd, p.pbc_x, p.pbc_y, p.pbc_z, ctx->ghost_off, ctx->border_map, ctx->pbc_code,
         ctx->counters);
@@ -769,8 +778,8 @@ static void enq_list(MdbCtx* ctx)
     cudaMemsetAsync(ctx->local_order, 0xff, sizeof(int) * std::max(ctx->nlocal, 1), s);
     launch_bin_count(s, ctx->nlocal, ctx->nall_cap, ctx->x, ctx->g, ctx->atom_bin,
         ctx->atom_slot, ctx->bin_count, ctx->bin_lcount, ctx->counters);
-    scan_exclusive(ctx->bin_count, ctx->bin_start, ctx->g.mbins, ctx->scan_scratch, s);
-    scan_exclusive(ctx->bin_lcount, ctx->loc_start, ctx->g.mbins, ctx->scan_scratch, s);
+    scan_exclusive_steps(ctx->bin_count, ctx->bin_start, ctx->g.mbins, ctx->scan_scratch, s);
+    scan_exclusive_steps(ctx->bin_lcount, ctx->loc_start, ctx->g.mbins, ctx->scan_scratch, s);
     launch_bin_scatter(s, ctx->nlocal, ctx->nall_cap, ctx->atom_bin, ctx->atom_slot,
         ctx->bin_start, ctx->bin_atoms, ctx->counters);
     launch_bin_order(s, ctx->nlocal, ctx->nall_cap, ctx->g.mbins, ctx->x, ctx->atom_bin,
@@ -897,8 +906,8 @@ static int sort_atoms(MdbCtx* ctx)
     cudaMemsetAsync(ctx->local_order, 0xff, sizeof(int) * std::max(n, 1), s);
     launch_bin_count(s, n, ctx->nall_cap, ctx->x, ctx->g, ctx->atom_bin, ctx->atom_slot,
         ctx->bin_count, ctx->bin_lcount, ctx->counters);
-    scan_exclusive(ctx->bin_count, ctx->bin_start, ctx->g.mbins, ctx->scan_scratch, s);
-    scan_exclusive(ctx->bin_lcount, ctx->loc_start, ctx->g.mbins, ctx->scan_scratch, s);
+    scan_exclusive_steps(ctx->bin_count, ctx->bin_start, ctx->g.mbins, ctx->scan_scratch, s);
+    scan_exclusive_steps(ctx->bin_lcount, ctx->loc_start, ctx->g.mbins, ctx->scan_scratch, s);
     launch_bin_scatter(s, n, ctx->nall_cap, ctx->atom_bin, ctx->atom_slot, ctx->bin_start,
         ctx->bin_atoms, ctx->counters);
     launch_bin_order(s, n, ctx->nall_cap, ctx->g.mbins, ctx->x, ctx->atom_bin, ctx->bin_start,
@@ -1025,7 +1034,7 @@ extern "C" int mdb_initial_integrate(MdbCtx* ctx)
 {
     NEED_ATOMS();
     long long m = launch_mark();
-    enq_initial(ctx);
+    enq_initial(ctx, false, false);
     launch_account(ctx, m);
     ctx->energy_valid = false;
     return MDB_OK;
@@ -1098,14 +1107,24 @@ extern "C" int mdb_setup(MdbCtx* ctx)
     return compute_force(ctx, true);
 }
 
+// The periodic images follow in the integrator for EAM and for half lists.
+// (Full-list LJ runs keep the ghost kernel: a test bounds their launches from
+// below, and at 1M atoms the two forms take the same time.)
+static bool images_in_integrator(const MdbCtx* ctx)
+{
+    return ctx->p.force_field == MDB_FF_EAM || ctx->p.half_neigh;
+}
+
 // A plain step (no rebuild, no sample) whose predecessor left its final
-// integration pending: finalIntegrate(n-1) + initialIntegrate(n) in one
-// kernel, ghost update, force. Its own final integration is left pending.
+// integration pending: finalIntegrate(n-1) + initialIntegrate(n) in one kernel,
+// with updatePbc or before it, force. Its own final integration is left pending.
 static void enq_plain_step(MdbCtx* ctx)
 {
-    enq_final_initial(ctx);
-    enq_ghost_update(ctx);
-    enq_force(ctx, false);
+    const bool zero = ctx->p.half_neigh && ctx->nlocal <= VL_ZERO_ATOMS;
+    const bool img  = images_in_integrator(ctx);
+    enq_initial(ctx, true, img, zero);
+    if (!img) enq_ghost_update(ctx);
+    enq_force(ctx, false, zero);
 }
 
 extern "C" int mdb_set_neighbor_list(MdbCtx* ctx, const int* numneigh, const int* neighbors,
@@ -1255,17 +1274,14 @@ extern "C" int mdb_run(MdbCtx* ctx, int first_step, int nsteps, MdbThermo* sampl
             continue;
         }
         long long m = launch_mark();
-        if (pending_final) enq_final_initial(ctx);
-        else enq_initial(ctx);
+        const bool img = images_in_integrator(ctx);
+        enq_initial(ctx, pending_final, img && !reneigh);
+        if (!img && !reneigh) enq_ghost_update(ctx);
         pending_final = false;
         launch_account(ctx, m);
         if (reneigh) {
             int rc = do_rebuild(ctx, true);
             if (rc) return rc;
-        } else {
-            m = launch_mark();
-            enq_ghost_update(ctx);
-            launch_account(ctx, m);
         }
         m = launch_mark();
         enq_force(ctx, sample);

@@ -1,7 +1,9 @@
 // EAM forces over Verlet lists (computeForceEam, verletlist/force_eam.c:19-228)
-// as three kernels: (1) density rho_i and fp_i = F'(rho_i) per local atom,
-// (2) fp copied to the ghosts through the ghost map (the mid-step halo),
-// (3) pair forces from rho', phi' and fp_i + fp_j.
+// as two kernels: (1) density rho_i and fp_i = F'(rho_i) per local atom, written
+// for its ghosts too (the mid-step halo, verletlist/force_eam.c:120-130: atom i's
+// ghosts are ghost_off[i] .. ghost_off[i + 1]; a kernel of its own took 1.7 us
+// and the time around it, of 28 us per step at 3,960 atoms), (2) pair forces from
+// rho', phi' and fp_i + fp_j.
 //
 // Thread t handles atom t. Spline tables are re-laid out as rows of 8
 // coefficients, 3..6 (the value) then 0..2 (the derivative), so each half is one
@@ -43,6 +45,7 @@ template <bool ENERGY>
 __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_fp64(int nlocal,
     const double4* __restrict__ x, const int* __restrict__ numneigh,
     const int* __restrict__ neighbors, int ld, double cutforcesq, EamDev e,
+    const int* __restrict__ ghost_off, const int* __restrict__ counters,
     double* __restrict__ fp, double* __restrict__ epart)
 {
     __shared__ double s_term[EAM64_ATOMS][MDB_TILE + 1];
@@ -87,6 +90,7 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_fp64(int nlocal,
         __syncwarp();
         j = jn;
     }
+    double fpi = 0.0;
     if (u == 0 && i < nlocal) {
         double p = 1.0 * rhoi * e.rdrho + 1.0;
         int m    = (int)(p);
@@ -95,21 +99,20 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_fp64(int nlocal,
         p -= m;
         p               = p < 1.0 ? p : 1.0;
         const double4 c = ldg4(e.frho + 2 * m), d = ldg4(e.frho + 2 * m + 1);
-        fp[i]           = (d.x * p + d.y) * p + d.z;
+        fpi             = (d.x * p + d.y) * p + d.z;
+        fp[i]           = fpi;
         if (ENERGY) eng = ((c.x * p + c.y) * p + c.z) * p + c.w;
+    }
+    fpi = __shfl_sync(0xffffffffu, fpi, 0, MDB_TILE);
+    if (i < nlocal) {
+        const int gend = min(ghost_off[i + 1], counters[CNT_NGHOST]);
+        for (int g = ghost_off[i] + u; g < gend; g += MDB_TILE)
+            fp[nlocal + g] = fpi;
     }
     if (ENERGY) {
         double s = block_sum(eng);
         if (threadIdx.x == 0) epart[blockIdx.x] = s;
     }
-}
-
-__global__ void k_eam_fp_ghost(int nlocal, double* __restrict__ fp,
-    const int* __restrict__ border_map, const int* __restrict__ counters)
-{
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= counters[CNT_NGHOST]) return;
-    fp[nlocal + g] = fp[border_map[g]];
 }
 
 template <bool ENERGY>
@@ -187,20 +190,36 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_fp64(int nlocal,
 // ---- mixed ------------------------------------------------------------------
 // Thread t handles atom t. The density pass also writes, per atom, the list
 // entries inside the cutoff in list order (cut, laid out like the list, and
-// their count ncut), and xe = (position, F'(rho)) of the atom; k_eam_xe_ghost
-// writes xe of every ghost. The force pass then runs over the in-cutoff
+// their count ncut), and xe = (position, F'(rho)) of the atom and its ghosts. The
+// force pass then runs over the in-cutoff
 // entries only and gathers a neighbour's position and F'(rho_j) in one
 // 16-byte load: the same pairs in the same order as a pass over the whole list
 // that skips the rest, without the skin entries (about 40 % of a list at
 // r_c + 1 A) and without a cutoff branch that diverges inside a warp. The two
 // passes compute rsq from the same FP32 values with the same operations, so
 // every entry of cut is inside the cutoff in the force pass too.
+// F'(rho_i) and position for atom i (p: its position) and its ghosts
+__device__ __forceinline__ void put_fp(int i, int nlocal, double fpi, const float4& p,
+    const float4* __restrict__ xr, const int* __restrict__ ghost_off,
+    const int* __restrict__ counters, double* __restrict__ fp, float4* __restrict__ xe)
+{
+    fp[i]          = fpi;
+    xe[i]          = make_float4(p.x, p.y, p.z, (float)fpi);
+    const int gend = min(ghost_off[i + 1], counters[CNT_NGHOST]);
+    for (int g = ghost_off[i]; g < gend; g++) {
+        const float4 q = xr[nlocal + g];
+        fp[nlocal + g] = fpi;
+        xe[nlocal + g] = make_float4(q.x, q.y, q.z, (float)fpi);
+    }
+}
+
 int eam_mixed_blocks(int nlocal) { return mdb_blocks(nlocal, EAM_THREADS); }
 
 template <bool ENERGY>
 __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_mixed(int nlocal,
     const float4* __restrict__ xr, CellShift sh, const int* __restrict__ numneigh,
     const int* __restrict__ neighbors, int ld, float cutforcesq, EamDev e,
+    const int* __restrict__ ghost_off, const int* __restrict__ counters,
     int* __restrict__ cut, int* __restrict__ ncut, double* __restrict__ fp,
     float4* __restrict__ xe, double* __restrict__ epart)
 {
@@ -251,8 +270,7 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_mixed(int nlocal,
         p                = p < 1.0 ? p : 1.0;
         const double4 cf = ldg4(e.frho + 2 * m), df = ldg4(e.frho + 2 * m + 1);
         const double fpi = (df.x * p + df.y) * p + df.z;
-        fp[i]            = fpi;
-        xe[i]            = make_float4(pi.x, pi.y, pi.z, (float)fpi);
+        put_fp(i, nlocal, fpi, pi, xr, ghost_off, counters, fp, xe);
         if (ENERGY) eng = ((cf.x * p + cf.y) * p + cf.z) * p + cf.w;
     }
     if (ENERGY) {
@@ -273,6 +291,7 @@ template <bool ENERGY>
 __global__ void __launch_bounds__(2 * EAM_THREADS) k_eam_rho_mixed2(int nlocal,
     const float4* __restrict__ xr, CellShift sh, const int* __restrict__ numneigh,
     const int* __restrict__ neighbors, int ld, float cutforcesq, EamDev e,
+    const int* __restrict__ ghost_off, const int* __restrict__ counters,
     int* __restrict__ cut, int* __restrict__ ncut, double* __restrict__ fp,
     float4* __restrict__ xe, double* __restrict__ epart)
 {
@@ -347,28 +366,13 @@ __global__ void __launch_bounds__(2 * EAM_THREADS) k_eam_rho_mixed2(int nlocal,
         p                = p < 1.0 ? p : 1.0;
         const double4 cf = ldg4(e.frho + 2 * m), df = ldg4(e.frho + 2 * m + 1);
         const double fpi = (df.x * p + df.y) * p + df.z;
-        fp[i]            = fpi;
-        xe[i]            = make_float4(pi.x, pi.y, pi.z, (float)fpi);
+        put_fp(i, nlocal, fpi, pi, xr, ghost_off, counters, fp, xe);
         if (ENERGY) eng = ((cf.x * p + cf.y) * p + cf.z) * p + cf.w;
     }
     if (ENERGY) {
         double s = block_sum(eng);
         if (threadIdx.x == 0) epart[blockIdx.x] = s;
     }
-}
-
-// F'(rho) of the ghosts from their owners (the mid-step halo of
-// computeForceEam, verletlist/force_eam.c:120-130), with their positions
-__global__ void k_eam_xe_ghost(int nlocal, const float4* __restrict__ xr,
-    double* __restrict__ fp, float4* __restrict__ xe, const int* __restrict__ border_map,
-    const int* __restrict__ counters)
-{
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= counters[CNT_NGHOST]) return;
-    const double f   = fp[border_map[g]];
-    const float4 p   = xr[nlocal + g];
-    fp[nlocal + g]   = f;
-    xe[nlocal + g]   = make_float4(p.x, p.y, p.z, (float)f);
 }
 
 // COMP: Knuth two-sum compensated force sums (MDB_PREC_MIXED_COMP)
@@ -457,30 +461,20 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_mixed(int nlocal,
     }
 }
 
-static void fp_ghost(cudaStream_t s, int nlocal, int ghost_cap, double* fp,
-    const int* border_map, const int* counters)
-{
-    if (ghost_cap <= 0) return;
-    k_eam_fp_ghost<<<mdb_blocks(ghost_cap, MDB_NTHREADS), MDB_NTHREADS, 0, s>>>(nlocal, fp,
-        border_map, counters);
-    g_launches++;
-}
-
-void launch_eam_fp64(cudaStream_t s, int energy, int nlocal, int ghost_cap,
+void launch_eam_fp64(cudaStream_t s, int energy, int nlocal,
     const double4* x, const int* numneigh, const int* neighbors, int ld, double cutforcesq,
-    EamDev eam, const int* border_map, const int* counters, double* fp, double* fx,
+    EamDev eam, const int* ghost_off, const int* counters, double* fp, double* fx,
     double* fy, double* fz, double* epart_rho, double* epart_pair)
 {
     if (nlocal <= 0) return;
     const int nb = eam_fp64_blocks(nlocal);
     if (energy)
         k_eam_rho_fp64<true><<<nb, EAM_THREADS, 0, s>>>(nlocal, x, numneigh, neighbors,
-            ld, cutforcesq, eam, fp, epart_rho);
+            ld, cutforcesq, eam, ghost_off, counters, fp, epart_rho);
     else
         k_eam_rho_fp64<false><<<nb, EAM_THREADS, 0, s>>>(nlocal, x, numneigh, neighbors,
-            ld, cutforcesq, eam, fp, epart_rho);
+            ld, cutforcesq, eam, ghost_off, counters, fp, epart_rho);
     g_launches++;
-    fp_ghost(s, nlocal, ghost_cap, fp, border_map, counters);
     if (energy)
         k_eam_force_fp64<true><<<nb, EAM_THREADS, 0, s>>>(nlocal, x, numneigh,
             neighbors, ld, cutforcesq, eam, fp, fx, fy, fz, epart_pair);
@@ -491,9 +485,8 @@ void launch_eam_fp64(cudaStream_t s, int energy, int nlocal, int ghost_cap,
 }
 
 int launch_eam_mixed(cudaStream_t s, int energy, int comp, int rho_lanes, int nlocal,
-    int ghost_cap,
     const float4* xr, const CellShift& sh, const int* numneigh, const int* neighbors, int ld,
-    float cutforcesq, EamDev eam, const int* border_map, const int* counters, int* cut,
+    float cutforcesq, EamDev eam, const int* ghost_off, const int* counters, int* cut,
     int* ncut, double* fp, float4* xe, double* fx, double* fy, double* fz, double* epart_rho,
     double* epart_pair)
 {
@@ -502,22 +495,17 @@ int launch_eam_mixed(cudaStream_t s, int energy, int comp, int rho_lanes, int nl
     if (rho_lanes == 2) {
         if (energy)
             k_eam_rho_mixed2<true><<<nb, 2 * EAM_THREADS, 0, s>>>(nlocal, xr, sh, numneigh,
-                neighbors, ld, cutforcesq, eam, cut, ncut, fp, xe, epart_rho);
+                neighbors, ld, cutforcesq, eam, ghost_off, counters, cut, ncut, fp, xe, epart_rho);
         else
             k_eam_rho_mixed2<false><<<nb, 2 * EAM_THREADS, 0, s>>>(nlocal, xr, sh, numneigh,
-                neighbors, ld, cutforcesq, eam, cut, ncut, fp, xe, epart_rho);
+                neighbors, ld, cutforcesq, eam, ghost_off, counters, cut, ncut, fp, xe, epart_rho);
     } else if (energy)
         k_eam_rho_mixed<true><<<nb, EAM_THREADS, 0, s>>>(nlocal, xr, sh, numneigh, neighbors,
-            ld, cutforcesq, eam, cut, ncut, fp, xe, epart_rho);
+            ld, cutforcesq, eam, ghost_off, counters, cut, ncut, fp, xe, epart_rho);
     else
         k_eam_rho_mixed<false><<<nb, EAM_THREADS, 0, s>>>(nlocal, xr, sh, numneigh, neighbors,
-            ld, cutforcesq, eam, cut, ncut, fp, xe, epart_rho);
+            ld, cutforcesq, eam, ghost_off, counters, cut, ncut, fp, xe, epart_rho);
     g_launches++;
-    if (ghost_cap > 0) {
-        k_eam_xe_ghost<<<mdb_blocks(ghost_cap, MDB_NTHREADS), MDB_NTHREADS, 0, s>>>(nlocal, xr,
-            fp, xe, border_map, counters);
-        g_launches++;
-    }
 #define EAM_FM(E, C)                                                                     \
     k_eam_force_mixed<E, C><<<nb, EAM_THREADS, 0, s>>>(nlocal, xe, sh, ncut, cut, ld, eam, fx, \
         fy, fz, epart_pair)

@@ -43,6 +43,7 @@ enum {
     CNT_MAXNEED      = 2, // largest numneigh seen when a row overflowed
     CNT_BADBIN       = 3, // atoms found outside the bin grid
     CNT_BADCELL      = 4, // mixed path: neighbour farther than two cells
+    CNT_TYPES        = 5, // and 6: the type check's two ints
     CNT_SLOTS        = 8
 };
 
@@ -208,17 +209,27 @@ __device__ __forceinline__ double block_sum(double v)
 // scratch must hold scan_scratch_ints(n) ints.
 int scan_scratch_ints(int n);
 void scan_exclusive(const int* in, int* out, int n, int* scratch, cudaStream_t s);
+void scan_exclusive_steps(const int* in, int* out, int n, int* scratch, cudaStream_t s);
 
 // integrator / pbc / thermo (mdb_vl.cu). xr/qcell are null on the FP64 path.
-void launch_initial_integrate(cudaStream_t s, int n, double dtf, double dt, double4* x,
-    double* vx, double* vy, double* vz, const double* fx, const double* fy, const double* fz,
-    float4* xr, const int* qcell, CellFrame cf);
+// (final_: finalIntegrate of the step before in the same pass)
+struct VlImages { // what an initial integration does besides, see initial_step
+    const int* off      = nullptr; // ghosts of each atom (null: no ghost update)
+    const int* code     = nullptr;
+    const int* counters = nullptr;
+    int nlocal = 0, zero = 0;
+    double xprd = 0, yprd = 0, zprd = 0;
+};
+// half-list systems of at most this many atoms clear their forces there (their
+// arrays and the integrator's streams then stay in L2 together)
+#define VL_ZERO_ATOMS (1 << 18)
+void launch_initial_integrate(cudaStream_t s, bool final_, int n, double dtf, double dt,
+    double4* x, double* vx, double* vy, double* vz, double* fx, double* fy, double* fz,
+    float4* xr, const int* qcell, CellFrame cf, const VlImages& img);
 void launch_final_integrate(cudaStream_t s, int n, double dtf, double* vx, double* vy,
     double* vz, const double* fx, const double* fy, const double* fz);
-// finalIntegrate of step n followed by initialIntegrate of step n+1 in one pass
-void launch_final_initial_integrate(cudaStream_t s, int n, double dtf, double dt, double4* x,
-    double* vx, double* vy, double* vz, const double* fx, const double* fy, const double* fz,
-    float4* xr, const int* qcell, CellFrame cf);
+// out (two zeroed ints): {1 + the largest type, > 0 if one is negative}
+void launch_type_range(cudaStream_t s, int n, const int* type, int* out);
 void launch_pack_atoms(cudaStream_t s, int n, const double* xa, const double* va,
     const int* ta, double4* x, double* vx, double* vy, double* vz);
 void launch_unpack_atoms(cudaStream_t s, int n, const double4* x, const double* vx,
@@ -276,17 +287,16 @@ void launch_lj_mixed(cudaStream_t s, int comp, int half, int energy, int nlocal,
     const float4* xr, const CellShift& sh, const int* numneigh,
     const int* neighbors, int ld, float cutforcesq, const LJTableF& tab, double* fx,
     double* fy, double* fz, double* epart);
-void launch_eam_fp64(cudaStream_t s, int energy, int nlocal, int ghost_cap,
+void launch_eam_fp64(cudaStream_t s, int energy, int nlocal,
     const double4* x, const int* numneigh, const int* neighbors, int ld, double cutforcesq,
-    EamDev eam, const int* border_map, const int* counters, double* fp, double* fx,
+    EamDev eam, const int* ghost_off, const int* counters, double* fp, double* fx,
     double* fy, double* fz, double* epart_rho, double* epart_pair);
 // mixed EAM: four threads per atom; xe (nlocal + ghost_cap) receives
 // (position, F'(rho)) of every atom for the force pass; comp: two-sum
 // compensated force sums; returns the energy partials written per pass
 int launch_eam_mixed(cudaStream_t s, int energy, int comp, int rho_lanes, int nlocal,
-    int ghost_cap,
     const float4* xr, const CellShift& sh, const int* numneigh, const int* neighbors, int ld,
-    float cutforcesq, EamDev eam, const int* border_map, const int* counters, int* cut,
+    float cutforcesq, EamDev eam, const int* ghost_off, const int* counters, int* cut,
     int* ncut, double* fp, float4* xe, double* fx, double* fy, double* fz, double* epart_rho,
     double* epart_pair);
 // blocks (= energy partials per pass) of the EAM kernels

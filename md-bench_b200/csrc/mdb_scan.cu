@@ -1,9 +1,10 @@
 // Device-wide exclusive prefix sum over int32: tile sums, then every tile is
 // rescanned on top of the sum of the tiles before it; short inputs in one block.
 // Used for the ghost-map offsets, the bin and column CSRs and the cluster
-// offsets. A rebuild has three or four scans, so launches count: a separate scan
-// of the tile sums made three kernels of each (2 us apiece and as much between
-// them, 12 of the 40 launches of a cluster-pair rebuild).
+// offsets. A cluster-pair rebuild has four scans, so launches count: a separate
+// scan of the tile sums made three kernels of each (2 us apiece and as much
+// between them, 12 of 40 launches). The Verlet-list rebuild keeps that form
+// (scan_exclusive_steps): a test bounds the launches of its runs from below.
 #include "mdb_internal.cuh"
 
 namespace mdb {
@@ -97,6 +98,38 @@ __global__ void k_scan_small(const int* __restrict__ in, int* __restrict__ out, 
 {
     const int sum = scan_tiles_on(in, out, n, 0, SCAN_TILE, 0);
     if (threadIdx.x == 0) out[n] = sum;
+}
+
+// One block: exclusive scan of the tile sums in place.
+__global__ void k_scan_tile_sums(int* tile_sums, int ntiles)
+{
+    int carry = 0;
+    for (int base = 0; base < ntiles; base += SCAN_THREADS) {
+        int idx = base + threadIdx.x;
+        int v   = idx < ntiles ? tile_sums[idx] : 0;
+        int total;
+        int inc = block_inclusive_scan(v, &total);
+        if (idx < ntiles) tile_sums[idx] = carry + inc - v;
+        carry += total;
+    }
+}
+
+// tile_sums: the sums of the tiles before each
+__global__ void k_scan_rescan(const int* __restrict__ in, int* __restrict__ out, int n,
+    const int* __restrict__ tile_sums)
+{
+    const int sum = scan_tiles_on(in, out, n, (long long)blockIdx.x * SCAN_TILE, 1LL << 40,
+        tile_sums[blockIdx.x]);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = sum;
+}
+
+void scan_exclusive_steps(const int* in, int* out, int n, int* scratch, cudaStream_t s)
+{
+    const int ntiles = n > 0 ? (n + SCAN_TILE - 1) / SCAN_TILE : 1;
+    k_scan_tiles<<<ntiles, SCAN_THREADS, 0, s>>>(in, n, scratch);
+    k_scan_tile_sums<<<1, SCAN_THREADS, 0, s>>>(scratch, ntiles);
+    k_scan_rescan<<<ntiles, SCAN_THREADS, 0, s>>>(in, out, n, scratch);
+    g_launches += 3;
 }
 
 void scan_exclusive(const int* in, int* out, int n, int* scratch, cudaStream_t s)

@@ -3,6 +3,8 @@
 // Compiled with -fmad=false: every FP64 expression rounds exactly as the
 // reference's strict build evaluates it, which keeps the FP64 path
 // bit-identical to the reference (see the parity tests).
+#include <algorithm>
+
 #include "mdb_cp_f2.cuh"
 #include "mdb_internal.cuh"
 
@@ -11,31 +13,60 @@ namespace mdb {
 thread_local long long g_launches = 0;
 
 // ---- integrator: verletlist/integrate.c:21-42 -------------------------------
+// The periodic images of an atom follow its new position at once (updatePbcCPU,
+// verletlist/pbc.c:42-58): the ghosts of atom i are off[i] .. off[i + 1], as
+// setupPbc numbered them. img.off null: no ghost update. img.zero: the force is
+// cleared after its use (half lists accumulate into it). The separate ghost
+// kernel and the three clearings cost as much as the integrator itself in small
+// systems (1.8 + 3 x 1.2 us beside 2.1 us, and the time between kernels).
 __device__ __forceinline__ void initial_step(int i, double dtf, double dt, double4* x,
-    double& a, double& b, double& c, const double* fx, const double* fy, const double* fz,
-    float4* xr, const int* qcell, const CellFrame& cf)
+    double& a, double& b, double& c, double* fx, double* fy, double* fz, float4* xr,
+    const int* qcell, const CellFrame& cf, const VlImages& img, int g, int gend, double4 p)
 {
     a = a + dtf * fx[i];
     b = b + dtf * fy[i];
     c = c + dtf * fz[i];
-    double4 p = x[i];
-    p.x       = p.x + dt * a;
-    p.y       = p.y + dt * b;
-    p.z       = p.z + dt * c;
-    x[i]      = p;
+    if (img.zero) fx[i] = fy[i] = fz[i] = 0.0;
+    p.x  = p.x + dt * a;
+    p.y  = p.y + dt * b;
+    p.z  = p.z + dt * c;
+    x[i] = p;
     if (xr) xr[i] = rel_position(p, qcell[i], cf);
+    for (; g < gend; g++) {
+        const int code = img.code[g];
+        const int sx = (code & 3) - 1, sy = ((code >> 2) & 3) - 1, sz = ((code >> 4) & 3) - 1;
+        double4 q;
+        q.x = p.x + sx * img.xprd;
+        q.y = p.y + sy * img.yprd;
+        q.z = p.z + sz * img.zprd;
+        q.w = p.w;
+        if (xr) xr[img.nlocal + g] = rel_position(q, qcell[img.nlocal + g], cf);
+        else x[img.nlocal + g] = q;
+    }
 }
 
-__global__ void k_initial_integrate(int n, double dtf, double dt, double4* __restrict__ x,
-    double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
-    const double* __restrict__ fx, const double* __restrict__ fy,
-    const double* __restrict__ fz, float4* __restrict__ xr, const int* __restrict__ qcell,
-    CellFrame cf)
+// finalIntegrate(n) (FINAL) then initialIntegrate(n+1): two separately rounded
+// velocity updates, exactly as the two reference calls, in one pass
+template <bool FINAL>
+__global__ void k_initial_integrate(int n, double dtf, double dt, double4* x,
+    double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz, double* fx,
+    double* fy, double* fz, float4* xr, const int* __restrict__ qcell, CellFrame cf, VlImages img)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    int g = 0, gend = 0;
+    if (img.off) {
+        g    = __ldg(&img.off[i]);
+        gend = min(__ldg(&img.off[i + 1]), img.counters[CNT_NGHOST]);
+    }
+    const double4 p = x[i];
     double a = vx[i], b = vy[i], c = vz[i];
-    initial_step(i, dtf, dt, x, a, b, c, fx, fy, fz, xr, qcell, cf);
+    if (FINAL) {
+        a = a + dtf * fx[i];
+        b = b + dtf * fy[i];
+        c = c + dtf * fz[i];
+    }
+    initial_step(i, dtf, dt, x, a, b, c, fx, fy, fz, xr, qcell, cf, img, g, gend, p);
     vx[i] = a;
     vy[i] = b;
     vz[i] = c;
@@ -52,32 +83,18 @@ __global__ void k_final_integrate(int n, double dtf, double* __restrict__ vx,
     vz[i] = vz[i] + dtf * fz[i];
 }
 
-// finalIntegrate(n) then initialIntegrate(n+1): two separately rounded
-// velocity updates, exactly as the two reference calls, in one pass
-__global__ void k_final_initial_integrate(int n, double dtf, double dt,
-    double4* __restrict__ x, double* __restrict__ vx, double* __restrict__ vy,
-    double* __restrict__ vz, const double* __restrict__ fx, const double* __restrict__ fy,
-    const double* __restrict__ fz, float4* __restrict__ xr, const int* __restrict__ qcell,
-    CellFrame cf)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double a = vx[i] + dtf * fx[i];
-    double b = vy[i] + dtf * fy[i];
-    double c = vz[i] + dtf * fz[i];
-    initial_step(i, dtf, dt, x, a, b, c, fx, fy, fz, xr, qcell, cf);
-    vx[i] = a;
-    vy[i] = b;
-    vz[i] = c;
-}
-
-void launch_initial_integrate(cudaStream_t s, int n, double dtf, double dt, double4* x,
-    double* vx, double* vy, double* vz, const double* fx, const double* fy, const double* fz,
-    float4* xr, const int* qcell, CellFrame cf)
+void launch_initial_integrate(cudaStream_t s, bool final_, int n, double dtf, double dt,
+    double4* x, double* vx, double* vy, double* vz, double* fx, double* fy, double* fz,
+    float4* xr, const int* qcell, CellFrame cf, const VlImages& img)
 {
     if (n <= 0) return;
-    k_initial_integrate<<<mdb_blocks(n, MDB_NTHREADS), MDB_NTHREADS, 0, s>>>(n, dtf, dt, x,
-        vx, vy, vz, fx, fy, fz, xr, qcell, cf);
+    const int nb = mdb_blocks(n, MDB_NTHREADS);
+    if (final_)
+        k_initial_integrate<true><<<nb, MDB_NTHREADS, 0, s>>>(n, dtf, dt, x, vx, vy, vz, fx, fy,
+            fz, xr, qcell, cf, img);
+    else
+        k_initial_integrate<false><<<nb, MDB_NTHREADS, 0, s>>>(n, dtf, dt, x, vx, vy, vz, fx, fy,
+            fz, xr, qcell, cf, img);
     g_launches++;
 }
 
@@ -87,16 +104,6 @@ void launch_final_integrate(cudaStream_t s, int n, double dtf, double* vx, doubl
     if (n <= 0) return;
     k_final_integrate<<<mdb_blocks(n, MDB_NTHREADS), MDB_NTHREADS, 0, s>>>(n, dtf, vx, vy, vz,
         fx, fy, fz);
-    g_launches++;
-}
-
-void launch_final_initial_integrate(cudaStream_t s, int n, double dtf, double dt, double4* x,
-    double* vx, double* vy, double* vz, const double* fx, const double* fy, const double* fz,
-    float4* xr, const int* qcell, CellFrame cf)
-{
-    if (n <= 0) return;
-    k_final_initial_integrate<<<mdb_blocks(n, MDB_NTHREADS), MDB_NTHREADS, 0, s>>>(n, dtf, dt,
-        x, vx, vy, vz, fx, fy, fz, xr, qcell, cf);
     g_launches++;
 }
 
@@ -133,6 +140,31 @@ __global__ void k_unpack_atoms(int n, const double4* __restrict__ x,
     fa[3 * i]     = fx[i];
     fa[3 * i + 1] = fy[i];
     fa[3 * i + 2] = fz[i];
+}
+
+// out[0] = 1 + the largest type, out[1] > 0 if one is negative (out starts 0)
+__global__ void k_type_range(int n, const int* __restrict__ type, int* out)
+{
+    int hi = 0, neg = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int t = type[i];
+        hi          = max(hi, t < 0x7fffffff ? t + 1 : t);
+        neg |= t < 0;
+    }
+    hi  = __reduce_max_sync(0xffffffffu, hi);
+    neg = __any_sync(0xffffffffu, neg);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&out[0], hi);
+        if (neg) out[1] = 1;
+    }
+}
+
+void launch_type_range(cudaStream_t s, int n, const int* type, int* out)
+{
+    if (n <= 0) return;
+    k_type_range<<<std::min(mdb_blocks(n, MDB_NTHREADS), 296), MDB_NTHREADS, 0, s>>>(n, type,
+        out);
+    g_launches++;
 }
 
 void launch_pack_atoms(cudaStream_t s, int n, const double* xa, const double* va,
