@@ -280,28 +280,29 @@ static void setup_columns(MdbCp* ctx)
 // One warp for four i-clusters shares set-up and reduction and pays once its
 // warps fill the chip; below that a warp for one or two shortens the chain of
 // iterations over a row: 840 atoms 12.3 -> 8.2 with one, 16,384 13.3 -> 11.3,
-// 45,356 18.1 -> 17.2, 87,808 26.7 -> 24.5 with two, 256,000 48.5 both (four
-// types: 2,000 18.5 -> 8.2, 87,808 29.0 -> 28.7). Full lists keep four at every
+// 42,592 18.0 -> 16.2 with two, 87,808 24.4 both. Full lists keep four at every
 // size: the shape sets the rounding of a sum, and a member of an ensemble must
 // follow its run alone bit for bit (ensembles of half lists, whose atomics round
 // in any order, take the large shape for all members).
-// Two j atoms per lane (one 256-bit load) except for 4x8 half lists of one type
-// (57.5 against 58.8 at 256,000).
-// The 64-register budget (variant 2) holds eight blocks of 128 threads on an SM:
-// one type, 1M atoms 162 against 240 without (half), 199 against 231 (full), but
-// 16.1 against 14.4 at 45,356 (full). Several types spill under it: 256,000 atoms
-// 67.4 -> 59.7 (half), 78.0 -> 63.3 (full) without; from half a million atoms on
-// latency counts more: full 268 -> 262 with it at 1M, and 4x4 half lists with
-// eight clusters per warp and one j atom per lane 442 -> 412 at 2M.
+// Two j atoms per lane share list handling and loop: 1M atoms 159 -> 152 (half),
+// 207 -> 199 (full).
+// The 64-register budget (variant 2) holds eight blocks of 128 threads on an SM.
+// One type: 1M atoms 152 against 198 without (half), 199 against 231 (full); 4x8
+// half lists 179 against 194 there but 54.7 against 51.3 at 256,000, full lists
+// 16.1 against 14.4 at 45,356. Several types spill under it: 256,000 atoms 65.8 ->
+// 57.4 (half), 78.0 -> 63.3 (full) without. From a million atoms on their latency
+// counts more: 4x4 full lists 268 -> 262 with it, half lists 434 -> 389 at 2M with
+// eight clusters per warp and one j atom per lane (500,000: 108 against 100.5).
 static void set_force_shape(Types& t, int N, int half, int n)
 {
-    const bool large = n > (1 << 19);
-    t.force_cpw   = !half ? 4 : n <= 16384 ? 1 : n <= 131072 ? 2 : 4;
-    t.force_jpl   = t.uniform && N == 8 && half ? 1 : 2; // with four per warp
-    t.force_block = t.uniform ? 128 : 64;
-    if (t.uniform) t.force_variant = half ? (t.force_cpw > 1 ? 2 : 0) : (n > 65536 ? 2 : 0);
-    else t.force_variant = large && N == 4 ? 2 : 0;
-    if (!t.uniform && half && large && N == 4) t.force_cpw = 8;
+    t.force_cpw   = !half ? 4 : n <= 16384 ? 1 : n <= 65536 && N == 4 ? 2 : 4;
+    t.force_jpl   = 2; // with four per warp
+    t.force_block = 128;
+    if (t.uniform && half)
+        t.force_variant = t.force_cpw == 1 || (N == 8 && n <= (1 << 19)) ? 0 : 2;
+    else if (t.uniform) t.force_variant = n > 65536 ? 2 : 0;
+    else t.force_variant = N == 4 && n > (half ? 1 << 20 : 1 << 19) ? 2 : 0;
+    if (!t.uniform && half && N == 4 && n > (1 << 20)) t.force_cpw = 8;
 }
 
 // computePerTypeLJParameters (common/parameter.c:31-45): per-type sqrt(eps)

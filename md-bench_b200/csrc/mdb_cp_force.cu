@@ -320,7 +320,7 @@ __device__ __forceinline__ void mixed_entry(const IPack& ip, const float4& xj, f
 // so no lane branches.
 template <int JPL>
 struct JEntry {
-    float4 x[JPL]; // atoms b0 .. b0 + JPL - 1 of the entry
+    float4 x[JPL]; // atoms b0 + u * BSTEP of the entry
     int cj;
 };
 
@@ -339,19 +339,19 @@ __device__ __forceinline__ void to_i_frame(float4& x, float ax, float ay, float 
 // AW (one atom type): the anchor travels in .w of the entry's slots 0..2 and
 // is applied when the entry is used (after its load has landed); otherwise
 // it is loaded here and applied at once.
-template <int N, bool AW, int JPL>
+template <int N, bool AW, int JPL, int BSTEP>
 __device__ __forceinline__ JEntry<JPL> load_entry(int cj, int b0, const float4* __restrict__ xr,
     const float4* __restrict__ anchor, const float4& ai)
 {
     JEntry<JPL> j;
     j.cj = cj;
-    if (JPL == 2) {
+    if (JPL == 2 && BSTEP == 1) {
         // slots cj * N + b0, b0 even: a 32-byte aligned pair
         ldg_pair4(&xr[cj * N + b0], j.x[0], j.x[JPL - 1]);
     } else {
 #pragma unroll
         for (int u = 0; u < JPL; u++)
-            j.x[u] = __ldg(&xr[cj * N + b0 + u]);
+            j.x[u] = __ldg(&xr[cj * N + b0 + u * BSTEP]);
     }
     if (!AW) {
         const float4 a = __ldg(&anchor[cj]);
@@ -383,8 +383,10 @@ __device__ __forceinline__ JEntry<JPL> load_entry(int cj, int b0, const float4* 
 // of 128 threads per SM asked of the register allocator (0: no request; 8
 // caps a thread at 64 registers, measured best against 6, 7, 9 and 10).
 // Both are launch-shape choices of the autotuner; results do not depend on them.
-// JPL: j atoms per lane (consecutive atoms of one entry; 2 shares a lane's
-// list handling, anchor and loop work between two atoms).
+// JPL: j atoms per lane (2 shares a lane's list handling, anchor and loop work
+// between two atoms of one entry). Full lists take consecutive atoms, in one
+// 256-bit load; half lists atoms bq and bq + N / 2, so that the lanes of an entry
+// add the reactions of neighbouring atoms, whole sectors, in one instruction.
 // The work of block bid (warps x CPW = i-clusters); s_se / s_s3: the type
 // tables in shared memory.
 template <int N, bool HALF, bool ENERGY, bool UNIFORM, int PF, int CPW, int JPL>
@@ -397,6 +399,7 @@ __device__ __forceinline__ void force_mixed_block(int bid, const int* __restrict
     constexpr int L   = 32 / CPW;  // lanes per i-cluster
     constexpr int LPE = N / JPL;   // lanes per list entry
     constexpr int JPW = L / LPE;   // entries per segment iteration
+    constexpr int BSTEP = HALF ? LPE : 1; // between the atoms of a lane
     static_assert(JPW >= 1, "a segment holds at least one list entry");
     const int lane = threadIdx.x & 31;
     const int l    = lane & (L - 1);
@@ -445,7 +448,7 @@ __device__ __forceinline__ void force_mixed_block(int bid, const int* __restrict
         const float sig6u = (float)ty.sigma6_0;
         const f2 A2 = f2_pack(cA, cA), mB2 = f2_pack(-cB, -cB);
         f2 fx[2] = {0, 0}, fy[2] = {0, 0}, fz[2] = {0, 0};
-        const int eidx = l / LPE, bq = l - eidx * LPE, b0 = bq * JPL;
+        const int eidx = l / LPE, bq = l - eidx * LPE, b0 = HALF ? bq : bq * JPL;
         // pairs of the diagonal entry (cj == ci_cj0) excluded as the
         // reference's cond (clusterpair/force_lj.c:108-123): the self pair, and
         // for half lists every pair with the i atom at or after the j atom
@@ -455,19 +458,20 @@ __device__ __forceinline__ void force_mixed_block(int bid, const int* __restrict
             diag_excl[u] = 0;
 #pragma unroll
             for (int a = 0; a < 4; a++)
-                if (HALF ? (ai0 + a >= b0 + u) : (ai0 + a == b0 + u)) diag_excl[u] |= 1u << a;
+                if (HALF ? (ai0 + a >= b0 + u * BSTEP) : (ai0 + a == b0 + u))
+                    diag_excl[u] |= 1u << a;
         }
         const int nn    = act ? numneigh[ci] : 0;
         const int dummy = cnt[CP_NCJ] + cnt[CP_NGC]; // the dummy j-cluster
         const int* row  = list + (size_t)cic * cs;
         int lst_cur = l < nn ? __ldg(&row[(size_t)l * ks]) : dummy;
         int lst_nxt = L + l < nn ? __ldg(&row[(size_t)(L + l) * ks]) : dummy;
-        JEntry<JPL> cur = load_entry<N, UNIFORM, JPL>(
+        JEntry<JPL> cur = load_entry<N, UNIFORM, JPL, BSTEP>(
             __shfl_sync(0xffffffffu, lst_cur, eidx, L), b0, xr, anchor, ai);
         JEntry<JPL> nx1;
         if (PF == 2) {
             const int c1 = __shfl_sync(0xffffffffu, lst_cur, JPW + eidx, L);
-            nx1 = load_entry<N, UNIFORM, JPL>(JPW < nn ? c1 : dummy, b0, xr, anchor, ai);
+            nx1 = load_entry<N, UNIFORM, JPL, BSTEP>(JPW < nn ? c1 : dummy, b0, xr, anchor, ai);
         }
         // one segment iteration: JPW entries, lane (eidx, bq) on atoms b0 ..
         // b0 + JPL - 1 of entry kb + eidx; masked: the iteration may hold the
@@ -481,20 +485,22 @@ __device__ __forceinline__ void force_mixed_block(int bid, const int* __restrict
             }
             const int cjn = __shfl_sync(0xffffffffu, lst_cur, (kn & (L - 1)) + eidx, L);
             const JEntry<JPL> nx =
-                load_entry<N, UNIFORM, JPL>(kn < nn ? cjn : dummy, b0, xr, anchor, ai);
+                load_entry<N, UNIFORM, JPL, BSTEP>(kn < nn ? cjn : dummy, b0, xr, anchor, ai);
             const int cj = cur.cj;
             float ax = 0.f, ay = 0.f, az = 0.f;
             if (UNIFORM) {
                 // the anchor of this entry's j-cluster from .w of its slots
                 // 0..2, held by the entry's lanes JPL slots each
                 const int base = lane - bq;
-                ax = __shfl_sync(0xffffffffu, cur.x[0 % JPL].w, base + 0 / JPL);
-                ay = __shfl_sync(0xffffffffu, cur.x[1 % JPL].w, base + 1 / JPL);
-                az = __shfl_sync(0xffffffffu, cur.x[2 % JPL].w, base + 2 / JPL);
+                constexpr auto reg = [](int b) { return HALF ? b / LPE : b % JPL; };
+                constexpr auto who = [](int b) { return HALF ? b % LPE : b / JPL; };
+                ax = __shfl_sync(0xffffffffu, cur.x[reg(0)].w, base + who(0));
+                ay = __shfl_sync(0xffffffffu, cur.x[reg(1)].w, base + who(1));
+                az = __shfl_sync(0xffffffffu, cur.x[reg(2)].w, base + who(2));
             }
 #pragma unroll
             for (int u = 0; u < JPL; u++) {
-                const int b = b0 + u;
+                const int b = b0 + u * BSTEP;
                 float4 xj   = cur.x[u];
                 if (UNIFORM) to_i_frame(xj, ax, ay, az, ai);
                 float sej = 0.f, s3j = 0.f;
