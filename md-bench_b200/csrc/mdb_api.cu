@@ -528,7 +528,7 @@ static int alloc_ghost_sized(MdbCtx* ctx, int ghost_cap)
     CK(dalloc(&ctx->bin_atoms, nall));
     CK(dalloc(&ctx->bin_jq, nall));
     CK(dalloc(&ctx->binf, 3 * (size_t)bin_stride(nall)));
-    if (ctx->p.force_field == MDB_FF_EAM) CK(dalloc(&ctx->fp, nall));
+    if (ctx->p.force_field == MDB_FF_EAM) CK(dalloc(&ctx->fp, (size_t)nall + 1)); // with the dummy atom
     if (ctx->p.force_field == MDB_FF_EAM && ctx->mixed) CK(dalloc(&ctx->xe, nall));
     ctx->ghost_cap   = ghost_cap;
     ctx->nall_cap    = nall;

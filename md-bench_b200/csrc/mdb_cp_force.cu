@@ -36,8 +36,8 @@ int force_blocks(int ncl_cap)
 // 228 listed pairs each, with few idle threads. FP64_QUEUE entries hold one row
 // of nearly every atom at LJ density; longer rows go in several turns. 97 -> 54
 // us per launch at 73,656 atoms (full lists), 85 -> 41 us at 4,000, 190 -> 173
-// us at 256,000 (half lists), where the broadcast loads of j positions (8 cycles
-// each for 32 threads of 32 bytes) bound the distance loop.
+// us at 256,000 (half lists), where the load path bounds it: 228 broadcast loads
+// of 32 bytes (8 cycles a warp) and 66 scattered ones per 32 slots.
 static constexpr int FP64_THREADS = 64;
 static constexpr int FP64_QUEUE   = 88;
 
@@ -74,18 +74,32 @@ __global__ void __launch_bounds__(FP64_THREADS) k_force_fp64(const int* __restri
     const int nmax  = __reduce_max_sync(0xffffffffu, nn);
     double fx = 0.0, fy = 0.0, fz = 0.0;
     double fix = 0.0, fiy = 0.0, fiz = 0.0; // the entry's sum
-    int cj_next = nn > 0 ? __ldg(row) : 0;
+    // the next entry's j atoms, and the cluster of the one after it, are in
+    // flight while an entry is tested: small systems have few warps per scheduler
+    // (4x4: 41 -> 33 us at 4,000 atoms, 53.5 -> 49.5 at 73,656; the eight atoms of
+    // a 4x8 entry would cost half the warps, 173 -> 196 us at 256,000)
+    constexpr bool AHEAD = N == 4;
+    int cj_cur = nn > 0 ? __ldg(row) : 0, cj_next = nn > 1 ? __ldg(&row[ks]) : cj_cur;
+    double4 pn[N];
+    if (AHEAD) {
+#pragma unroll
+        for (int b = 0; b < N; b++)
+            pn[b] = ldg4(&cx[cj_cur * N + b]);
+    }
     for (int k = 0; k < nmax;) {
         int n = 0;
         // distances of whole entries while every thread's queue has room
         do {
             if (k < nn) {
-                const int cj = cj_next;
-                if (k + 1 < nn) cj_next = __ldg(&row[(size_t)(k + 1) * ks]);
+                const int cj = cj_cur;
                 double4 pj[N];
 #pragma unroll
-                for (int b = 0; b < N; b++)
-                    pj[b] = ldg4(&cx[cj * N + b]);
+                for (int b = 0; b < N; b++) {
+                    pj[b] = AHEAD ? pn[b] : ldg4(&cx[cj * N + b]);
+                    if (AHEAD) pn[b] = ldg4(&cx[cj_next * N + b]);
+                }
+                cj_cur = cj_next;
+                if (k + 2 < nn) cj_next = __ldg(&row[(size_t)(k + 2) * ks]);
                 int first = 0x80000000; // marks an entry's first queued slot
 #pragma unroll
                 for (int b = 0; b < N; b++) {
@@ -106,15 +120,27 @@ __global__ void __launch_bounds__(FP64_THREADS) k_force_fp64(const int* __restri
         } while (k < nmax && !__any_sync(0xffffffffu, n > FP64_QUEUE - N));
         // two queued pairs at a time: their square distances, divisions and
         // products overlap, the sums stay in list order
+        int vn[2]  = {};
+        double4 qn[2];
+        auto fetch = [&](int q) {
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (q + u < n) vn[u] = queue[(q + u) * FP64_THREADS];
+                qn[u] = ldg4(&cx[vn[u] & 0x7fffffff]);
+            }
+        };
+        if (AHEAD) fetch(0);
         for (int q = 0; q < n; q += 2) {
             int v[2];
             double4 pj[2];
             double tx[2], ty[2], tz[2];
-            v[0] = queue[q * FP64_THREADS];
-            v[1] = q + 1 < n ? queue[(q + 1) * FP64_THREADS] : v[0];
+            if (!AHEAD) fetch(q);
 #pragma unroll
-            for (int u = 0; u < 2; u++)
-                pj[u] = ldg4(&cx[v[u] & 0x7fffffff]);
+            for (int u = 0; u < 2; u++) {
+                v[u]  = vn[u];
+                pj[u] = qn[u];
+            }
+            if (AHEAD) fetch(q + 2);
 #pragma unroll
             for (int u = 0; u < 2; u++) {
                 const double delx = pi.x - pj[u].x;

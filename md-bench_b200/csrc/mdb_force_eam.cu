@@ -34,7 +34,7 @@ static constexpr int EUNROLL     = 4;
 // their terms in shared memory, where one thread per sum adds them up in order.
 // (One thread per atom spent its time waiting on its own chain of dependent
 // square roots, divisions and table rows, at 31 blocks for 4,000 atoms.)
-// A pair outside the cutoff adds an exact zero. Both passes: 85 -> 20 us at 3,960
+// A pair outside the cutoff adds an exact zero. Both passes: 85 -> 16 us at 3,960
 // atoms, 302 -> 211 us at 131,072, where the scattered table rows bound them (one
 // 32-byte load per half row; 307 us with eight-byte loads of the coefficients).
 static constexpr int EAM64_ATOMS = EAM_THREADS / MDB_TILE; // atoms per block
@@ -58,14 +58,19 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_fp64(int nlocal,
     const int* nb    = neighbors + list_at(0, ld, ia) + u;
     const int nmax   = __reduce_max_sync(0xffffffffu, n);
     double rhoi      = 0.0;
-    int j            = n > 0 ? __ldcs(nb) : -1;
+    // the next tile's positions and the entries of the one after it are in flight
+    // while a tile is worked on
+    auto entry = [&](int k) {
+        return k < n ? __ldcs(nb + (size_t)(k / MDB_TILE) * ld * MDB_TILE) : -1;
+    };
+    int j      = entry(0), j1 = entry(MDB_TILE);
+    double4 xn = ldg4(x + max(j, 0));
     for (int k = 0; k < nmax; k += MDB_TILE) {
-        double term = 0.0;
-        const int jn = k + MDB_TILE < n
-                           ? __ldcs(nb + (size_t)(k / MDB_TILE + 1) * ld * MDB_TILE)
-                           : -1;
+        double term      = 0.0;
+        const double4 xj = xn;
+        xn               = ldg4(x + max(j1, 0));
+        const int j2     = entry(k + 2 * MDB_TILE);
         if (j >= 0) {
-            const double4 xj = ldg4(x + j);
             double delx = xi.x - xj.x;
             double dely = xi.y - xj.y;
             double delz = xi.z - xj.z;
@@ -88,7 +93,8 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_fp64(int nlocal,
                 rhoi += s_term[g][q];
         }
         __syncwarp();
-        j = jn;
+        j  = j1;
+        j1 = j2;
     }
     double fpi = 0.0;
     if (u == 0 && i < nlocal) {
@@ -133,14 +139,20 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_fp64(int nlocal,
     const int nmax   = __reduce_max_sync(0xffffffffu, n);
     const double fpi = fp[ia];
     double sum       = 0.0; // threads 0, 1, 2: the x, y, z force
-    int j            = n > 0 ? __ldcs(nb) : -1;
+    auto entry       = [&](int k) {
+        return k < n ? __ldcs(nb + (size_t)(k / MDB_TILE) * ld * MDB_TILE) : -1;
+    };
+    int j      = entry(0), j1 = entry(MDB_TILE);
+    double4 xn = ldg4(x + max(j, 0));
+    double fpn = __ldg(fp + max(j, 0));
     for (int k = 0; k < nmax; k += MDB_TILE) {
         double tx = 0.0, ty = 0.0, tz = 0.0;
-        const int jn = k + MDB_TILE < n
-                           ? __ldcs(nb + (size_t)(k / MDB_TILE + 1) * ld * MDB_TILE)
-                           : -1;
+        const double4 xj = xn;
+        const double fpj = fpn;
+        xn               = ldg4(x + max(j1, 0));
+        fpn              = __ldg(fp + max(j1, 0));
+        const int j2     = entry(k + 2 * MDB_TILE);
         if (j >= 0) {
-            const double4 xj = ldg4(x + j);
             double delx = xi.x - xj.x;
             double dely = xi.y - xj.y;
             double delz = xi.z - xj.z;
@@ -160,7 +172,7 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_fp64(int nlocal,
                 double recip = 1.0 / r;
                 double phi   = z2 * recip;
                 double phip  = z2p * recip - phi * recip;
-                double psip  = fpi * rhoip + __ldg(fp + j) * rhoip + phip;
+                double psip  = fpi * rhoip + fpj * rhoip + phip;
                 double fpair = -psip * recip;
                 tx = delx * fpair;
                 ty = dely * fpair;
@@ -178,7 +190,8 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_fp64(int nlocal,
                 sum += s_term[g][u][q];
         }
         __syncwarp();
-        j = jn;
+        j  = j1;
+        j1 = j2;
     }
     if (i < nlocal && u < 3) (u == 0 ? fx : u == 1 ? fy : fz)[i] = sum;
     if (ENERGY) {

@@ -527,21 +527,21 @@ void launch_bin_order(cudaStream_t s, int nlocal, int nall_cap, int mbins, const
 // on every distance to its atoms, with a relative margin: only candidates that
 // would fail the test are left out). Candidates are tested eight at a time, two
 // per packed instruction and without a branch: the signs of rsq - hi collect in
-// a bit mask of up to 32 candidates. hi and lo bound cutneigh^2 by the FP32
-// rounding error `margin`; candidates between them take the reference's exact
-// FP64 test. The accepted ones' places go, in order, to a ring in shared memory;
+// a bit mask of up to 32 candidates. hi lies above cutneigh^2 by the FP32 rounding
+// error `margin`; a mask with a candidate within twice that below hi goes through
+// the reference's exact FP64 test. The accepted ones' places go, in order, to a ring in shared memory;
 // its full tiles are turned into list entries together (the threads of a warp
 // stay converged there) and leave as whole 32-byte sectors, wherever the row
 // lies. On the mixed path each entry also carries the cell offset of the pair
 // (2 bits per axis below the index). Bound by instructions: threads of a warp
 // differ in their runs and accepted candidates (15 of 32 threads active). 1M LJ
-// atoms 1,330 -> 975 us, 47,840 137 -> 99 us (half lists), Cu 131,072 227 -> 174
+// atoms 1,330 -> 913 us, 47,840 137 -> 111 us (half lists), Cu 131,072 227 -> 127
 // us, 3,960 130 -> 62 us against one branching test per candidate.
 static constexpr int BL_THREADS = 128;
-static constexpr int BL_RING    = 64; // > BL_KEEP + 32 accepted of a mask
-static constexpr int BL_KEEP    = 31; // entries that wait before tiles are written
+static constexpr int BL_KEEP    = 15; // entries that wait before tiles are written
+static constexpr int BL_RING    = 48; // > BL_KEEP + 32 accepted of a mask
 
-__global__ void __launch_bounds__(BL_THREADS, 6) k_build_list(int nlocal,
+__global__ void __launch_bounds__(BL_THREADS, 8) k_build_list(int nlocal,
     const int* __restrict__ local_order, const int* __restrict__ loc_start,
     const double4* __restrict__ x, BinGeom g, int nrows, const int4* __restrict__ rows,
     const int* __restrict__ atom_bin, const int* __restrict__ bin_start,
@@ -572,10 +572,11 @@ __global__ void __launch_bounds__(BL_THREADS, 6) k_build_list(int nlocal,
     const float by = (float)g.binsizey, bz = (float)g.binsizez;
     const float bxinv = 1.0f / (float)g.binsizex;
     const float skip2 = (float)cutneighsq * 1.0001f + 1e-4f;
-    const float lo = (float)cutneighsq - margin, hi = (float)cutneighsq + margin;
+    const float hi = (float)cutneighsq + margin;
+    const float near = 2.0f * margin + 1e-6f * hi; // hi - rsq of a candidate left to FP64
     const f2 XI = f2_pack((float)xi.x, (float)xi.x), YI = f2_pack((float)xi.y, (float)xi.y),
              ZI = f2_pack((float)xi.z, (float)xi.z);
-    const f2 HI = f2_pack(hi, hi), LO = f2_pack(lo, lo);
+    const f2 HI = f2_pack(hi, hi);
     // 1 + the difference of two packed cells, field by field
     const int q1 = qcell ? 0x00100401 - qcell[i] : 0;
     int* ring    = &s_ring[0][threadIdx.x];
@@ -635,7 +636,8 @@ __global__ void __launch_bounds__(BL_THREADS, 6) k_build_list(int nlocal,
                 const int ng    = min(4, (end - mb + 7) >> 3);
                 const float4* p = reinterpret_cast<const float4*>(binf + mb);
                 const int s4    = stride >> 2;
-                unsigned in = 0, un = 0; // first candidate in the highest bit
+                unsigned in = 0;     // first candidate in the highest bit
+                float mn    = 1e30f; // smallest |rsq - hi|
                 for (int q = 0; q < ng; q++, p += 2) {
                     float4 X[2], Y[2], Z[2];
 #pragma unroll
@@ -651,22 +653,20 @@ __global__ void __launch_bounds__(BL_THREADS, 6) k_build_list(int nlocal,
                         const f2 dy = f2_sub(YI, w & 1 ? f2_pack(b.z, b.w) : f2_pack(b.x, b.y));
                         const f2 dz = f2_sub(ZI, w & 1 ? f2_pack(c.z, c.w) : f2_pack(c.x, c.y));
                         const f2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
-                        float a0, a1, u0, u1;
+                        float a0, a1;
                         f2_unpack(f2_sub(r2, HI), a0, a1);
-                        f2_unpack(f2_sub(LO, r2), u0, u1);
                         in = __funnelshift_l(__float_as_uint(a0), in, 1);
-                        un = __funnelshift_l(__float_as_uint(u0), un, 1);
                         in = __funnelshift_l(__float_as_uint(a1), in, 1);
-                        un = __funnelshift_l(__float_as_uint(u1), un, 1);
+                        mn = fminf(fminf(fabsf(a0), fabsf(a1)), mn);
                     }
                 }
                 in <<= 32 - 8 * ng;
-                un <<= 32 - 8 * ng;
                 if (beg > mb) in &= 0xffffffffu >> (beg - mb);
                 if (end - mb < 32) in &= ~(0xffffffffu >> (end - mb));
                 if ((unsigned)(self - mb) < 32u) in &= ~(0x80000000u >> (self - mb));
-                un &= in;
-                while (un) { // the reference's test, verletlist/neighbor.c:320-330
+                // near the cutoff (3 atoms in 100 have such a candidate):
+                // the reference's test, verletlist/neighbor.c:320-330
+                for (unsigned un = mn <= near ? in : 0; un;) {
                     const unsigned bit = 0x80000000u >> __clz(un);
                     un ^= bit;
                     const double4 xj = ldg4(&x[bin_jq[mb + __clz(bit)].x]);
@@ -683,7 +683,8 @@ __global__ void __launch_bounds__(BL_THREADS, 6) k_build_list(int nlocal,
                     ring[(n % BL_RING) * BL_THREADS] = mb + u;
                     n++;
                 }
-                if (n - nf > BL_KEEP)
+                // the threads that are here together write together
+                if (__any_sync(__activemask(), n - nf > BL_KEEP))
                     while (n - nf >= MDB_TILE)
                         flush();
             }
