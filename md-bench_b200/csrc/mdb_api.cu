@@ -621,6 +621,9 @@ extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const dou
         CK(dalloc(&ctx->scan_scratch, nscan));
         ctx->npart = std::max(std::max(force_partial_blocks(cap), ke_partial_blocks(cap)),
             ctx->p.force_field == MDB_FF_EAM ? eam_fp64_blocks(cap) : 1);
+        // (FP64 LJ: fewer atoms than the capacity can take more blocks; 16 atoms
+        // a block at the least)
+        if (!ctx->mixed) ctx->npart = std::max(ctx->npart, mdb_blocks(cap, 16));
         CK(dalloc(&ctx->partials, 3 * (size_t)ctx->npart));
         ctx->nred_slots = 64;
         CK(dalloc(&ctx->red, 4 * (size_t)ctx->nred_slots));
@@ -1058,9 +1061,11 @@ static void enq_thermo(MdbCtx* ctx, int slot, bool with_pe)
         ctx->partials + 2 * (size_t)ctx->npart);
     launch_reduce_partials(s, nke, ctx->partials + 2 * (size_t)ctx->npart, r + 0);
     if (with_pe) {
-        const int nf = ctx->p.force_field != MDB_FF_EAM ? force_partial_blocks(owned(ctx))
-                       : ctx->mixed                     ? eam_mixed_blocks(owned(ctx))
-                                                        : eam_fp64_blocks(owned(ctx));
+        const int n  = owned(ctx);
+        const int nf = ctx->p.force_field != MDB_FF_EAM
+                           ? (ctx->mixed ? force_partial_blocks(n)
+                                         : lj_fp64_blocks(ctx->p.half_neigh, n))
+                           : (ctx->mixed ? eam_mixed_blocks(n) : eam_fp64_blocks(n));
         launch_reduce_partials(s, nf, ctx->partials, r + 1);
         if (ctx->p.force_field == MDB_FF_EAM)
             launch_reduce_partials(s, nf, ctx->partials + ctx->npart, r + 2);

@@ -263,10 +263,16 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_rho_mixed(int nlocal,
                 c++;
             }
         };
-        for (int k = 0; k < n; k += MDB_TILE, nb += (size_t)ld * MDB_TILE) {
+        int nx[MDB_TILE]; // the next tile is in flight while one is worked on
+        if (n > 0) ld_tile(nb, nx);
+        for (int k = 0; k < n; k += MDB_TILE) {
             int en[MDB_TILE];
             float4 pj[MDB_TILE];
-            ld_tile(nb, en);
+#pragma unroll
+            for (int v = 0; v < MDB_TILE; v++)
+                en[v] = nx[v];
+            nb += (size_t)ld * MDB_TILE;
+            if (k + MDB_TILE < n) ld_tile(nb, nx);
 #pragma unroll
             for (int v = 0; v < MDB_TILE; v++)
                 pj[v] = __ldg(xr + entry_index(en[v]));
@@ -447,12 +453,19 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_mixed(int nlocal,
             if (ENERGY) eng += 0.5 * (double)phi;
         };
         int k = 0;
+        int nx[EUNROLL]; // the next entries are in flight while four are worked on
+#pragma unroll
+        for (int v = 0; v < EUNROLL; v++)
+            nx[v] = v < n ? __ldcs(nb + (size_t)v * ld) : 0;
         for (; k + EUNROLL <= n; k += EUNROLL) {
             int en[EUNROLL];
             float4 pj[EUNROLL];
 #pragma unroll
-            for (int v = 0; v < EUNROLL; v++)
-                en[v] = __ldcs(nb + (size_t)(k + v) * ld);
+            for (int v = 0; v < EUNROLL; v++) {
+                en[v]      = nx[v];
+                const int q = k + EUNROLL + v;
+                if (q < n) nx[v] = __ldcs(nb + (size_t)q * ld);
+            }
 #pragma unroll
             for (int v = 0; v < EUNROLL; v++)
                 pj[v] = __ldg(xe + entry_index(en[v]));
@@ -460,10 +473,9 @@ __global__ void __launch_bounds__(EAM_THREADS) k_eam_force_mixed(int nlocal,
             for (int v = 0; v < EUNROLL; v++)
                 pair(en[v], pj[v]);
         }
-        for (; k < n; k++) {
-            const int en = __ldcs(nb + (size_t)k * ld);
-            pair(en, __ldg(xe + entry_index(en)));
-        }
+#pragma unroll
+        for (int v = 0; v < EUNROLL; v++)
+            if (k + v < n) pair(nx[v], __ldg(xe + entry_index(nx[v])));
         fx[i] = (double)fix + (double)cx;
         fy[i] = (double)fiy + (double)cy;
         fz[i] = (double)fiz + (double)cz;

@@ -24,7 +24,21 @@ static constexpr int LJ_THREADS = 128;
 
 int force_partial_blocks(int n) { return mdb_blocks(n > 0 ? n : 1, LJ_THREADS); }
 
-template <bool HALF, bool UNIFORM, bool ENERGY>
+// Whether an FP64 system of n atoms shares an atom among 8 threads
+// (k_lj_fp64_shared): half lists at every size (29.5 -> 19.7 us per launch at
+// 47,840 atoms, 311 -> 235 at 702,464: more of their atomics are in flight), full
+// lists while a thread per atom leaves the chip idle (15.8 -> 5.6 us at 4,000, 20.5
+// -> 11.2 at 15,360, but 17.0 against 20.4 at 32,000, and 66 at 119,164 where a
+// thread per atom takes 41 at 143,748).
+static bool lj_fp64_shared(int half, int n) { return half || n <= 16384; }
+
+int lj_fp64_blocks(int half, int n)
+{
+    return lj_fp64_shared(half, n) ? mdb_blocks(n > 0 ? n : 1, LJ_THREADS / MDB_TILE)
+                                   : force_partial_blocks(n);
+}
+
+template <bool UNIFORM, bool ENERGY>
 __global__ void __launch_bounds__(LJ_THREADS) k_lj_fp64(int nlocal, const double4* __restrict__ x,
     const int* __restrict__ numneigh, const int* __restrict__ neighbors, int ld,
     double cutforcesq, LJTable tab, double* __restrict__ fx, double* __restrict__ fy,
@@ -51,7 +65,7 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_fp64(int nlocal, const double
         double fix = 0.0, fiy = 0.0, fiz = 0.0;
         const double eps0 = tab.eps[0], sig0 = tab.sig6[0];
 
-        auto pair = [&](int j, const double4& xj) {
+        auto pair = [&](const double4& xj) {
             double delx = xi.x - xj.x;
             double dely = xi.y - xj.y;
             double delz = xi.z - xj.z;
@@ -69,38 +83,140 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_fp64(int nlocal, const double
                 fix += delx * force;
                 fiy += dely * force;
                 fiz += delz * force;
+                if (ENERGY) epot += 0.5 * (4.0 * epsilon * sr6 * (sr6 - 1.0));
+            }
+        };
+
+        // the next tile is in flight while one is worked on
+        int jn[MDB_TILE];
+        if (n > 0) ld_tile(nb, jn);
+        for (int k = 0; k < n; k += MDB_TILE) {
+            int j[MDB_TILE];
+            double4 xj[MDB_TILE];
+#pragma unroll
+            for (int u = 0; u < MDB_TILE; u++)
+                j[u] = jn[u];
+            nb += (size_t)ld * MDB_TILE;
+            if (k + MDB_TILE < n) ld_tile(nb, jn);
+#pragma unroll
+            for (int u = 0; u < MDB_TILE; u++)
+                xj[u] = ldg4(x + j[u]);
+#pragma unroll
+            for (int u = 0; u < MDB_TILE; u++)
+                pair(xj[u]);
+        }
+        fx[i] = fix;
+        fy[i] = fiy;
+        fz[i] = fiz;
+    }
+    if (ENERGY) {
+        double e = block_sum(epot);
+        if (threadIdx.x == 0) epart[blockIdx.x] = e;
+    }
+}
+
+// The same with 8 threads per atom, one entry of a tile each: a thread per atom
+// leaves small systems with a few warps per scheduler, each on a chain of gathers
+// and divisions. Full lists leave their terms in shared memory, where one thread
+// per component adds them in list order (a pair outside the cutoff adds an exact
+// zero), so forces stay bit-identical; half lists sum per thread and then across
+// the 8.
+template <bool HALF, bool UNIFORM, bool ENERGY>
+__global__ void __launch_bounds__(LJ_THREADS) k_lj_fp64_shared(int nlocal,
+    const double4* __restrict__ x, const int* __restrict__ numneigh,
+    const int* __restrict__ neighbors, int ld, double cutforcesq, LJTable tab,
+    double* __restrict__ fx, double* __restrict__ fy, double* __restrict__ fz,
+    double* __restrict__ epart)
+{
+    constexpr int ATOMS = LJ_THREADS / MDB_TILE;
+    __shared__ double s_eps[MDB_MAX_TYPES * MDB_MAX_TYPES];
+    __shared__ double s_sig6[MDB_MAX_TYPES * MDB_MAX_TYPES];
+    __shared__ double s_term[HALF ? 1 : ATOMS][3][MDB_TILE + 1];
+    const int nt = tab.ntypes;
+    if (!UNIFORM) {
+        for (int k = threadIdx.x; k < nt * nt; k += blockDim.x) {
+            s_eps[k]  = tab.eps[k];
+            s_sig6[k] = tab.sig6[k];
+        }
+        __syncthreads();
+    }
+    const int g = threadIdx.x / MDB_TILE, u = threadIdx.x % MDB_TILE;
+    const int i = blockIdx.x * ATOMS + g;
+    const int ia     = i < nlocal ? i : 0;
+    const double4 xi = x[ia];
+    const int ti     = type_of(xi);
+    const int n      = i < nlocal ? numneigh[ia] : 0;
+    const int* nb    = neighbors + list_at(0, ld, ia) + u;
+    const int nmax   = __reduce_max_sync(0xffffffffu, n);
+    double epot      = 0.0;
+    double sx = 0.0, sy = 0.0, sz = 0.0; // full lists: sx of threads 0, 1, 2 = x, y, z
+    // positions of the next tile and entries of the one after it are in flight
+    auto entry = [&](int k) {
+        return k < n ? __ldcs(nb + (size_t)(k / MDB_TILE) * ld * MDB_TILE) : -1;
+    };
+    int j      = entry(0), j1 = entry(MDB_TILE);
+    double4 xn = ldg4(x + max(j, 0));
+    for (int k = 0; k < nmax; k += MDB_TILE) {
+        double tx = 0.0, ty = 0.0, tz = 0.0;
+        const double4 xj = xn;
+        xn               = ldg4(x + max(j1, 0));
+        const int j2     = entry(k + 2 * MDB_TILE);
+        if (j >= 0) {
+            double delx = xi.x - xj.x;
+            double dely = xi.y - xj.y;
+            double delz = xi.z - xj.z;
+            double rsq  = delx * delx + dely * dely + delz * delz;
+            if (rsq < cutforcesq) {
+                const int tij        = UNIFORM ? 0 : ti * nt + type_of(xj);
+                const double sigma6  = UNIFORM ? tab.sig6[0] : s_sig6[tij];
+                const double epsilon = UNIFORM ? tab.eps[0] : s_eps[tij];
+                double sr2   = 1.0 / rsq;
+                double sr6   = sr2 * sr2 * sr2 * sigma6;
+                double force = 48.0 * sr6 * (sr6 - 0.5) * sr2 * epsilon;
+                tx = delx * force;
+                ty = dely * force;
+                tz = delz * force;
                 if (HALF && j < nlocal) {
-                    atomicAdd(&fx[j], -(delx * force));
-                    atomicAdd(&fy[j], -(dely * force));
-                    atomicAdd(&fz[j], -(delz * force));
+                    atomicAdd(&fx[j], -tx);
+                    atomicAdd(&fy[j], -ty);
+                    atomicAdd(&fz[j], -tz);
                 }
                 if (ENERGY) {
                     double e = 4.0 * epsilon * sr6 * (sr6 - 1.0);
                     epot += (HALF && j < nlocal) ? e : 0.5 * e;
                 }
             }
-        };
-
-        for (int k = 0; k < n; k += MDB_TILE, nb += (size_t)ld * MDB_TILE) {
-            int j[MDB_TILE];
-            double4 xj[MDB_TILE];
-            ld_tile(nb, j);
-#pragma unroll
-            for (int u = 0; u < MDB_TILE; u++)
-                xj[u] = ldg4(x + j[u]);
-#pragma unroll
-            for (int u = 0; u < MDB_TILE; u++)
-                pair(j[u], xj[u]);
         }
         if (HALF) {
-            atomicAdd(&fx[i], fix);
-            atomicAdd(&fy[i], fiy);
-            atomicAdd(&fz[i], fiz);
+            sx += tx;
+            sy += ty;
+            sz += tz;
         } else {
-            fx[i] = fix;
-            fy[i] = fiy;
-            fz[i] = fiz;
+            s_term[g][0][u] = tx;
+            s_term[g][1][u] = ty;
+            s_term[g][2][u] = tz;
+            __syncwarp();
+            if (u < 3) {
+#pragma unroll
+                for (int q = 0; q < MDB_TILE; q++)
+                    sx += s_term[g][u][q];
+            }
+            __syncwarp();
         }
+        j  = j1;
+        j1 = j2;
+    }
+    if (HALF) {
+#pragma unroll
+        for (int o = MDB_TILE / 2; o > 0; o >>= 1) {
+            sx += __shfl_xor_sync(0xffffffffu, sx, o);
+            sy += __shfl_xor_sync(0xffffffffu, sy, o);
+            sz += __shfl_xor_sync(0xffffffffu, sz, o);
+        }
+        if (i < nlocal && u < 3)
+            atomicAdd(u == 0 ? &fx[i] : u == 1 ? &fy[i] : &fz[i], u == 0 ? sx : u == 1 ? sy : sz);
+    } else if (i < nlocal && u < 3) {
+        (u == 0 ? fx : u == 1 ? fy : fz)[i] = sx;
     }
     if (ENERGY) {
         double e = block_sum(epot);
@@ -191,14 +307,17 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal, const float
         };
 
         double rx = 0.0, ry = 0.0, rz = 0.0;
+        int en[MDB_TILE]; // the next tile is in flight while one is worked on
+        if (n > 0) ld_tile(nb, en);
         if (UNIFORM && !HALF && !COMP) {
             // One type, full lists: two entries per packed instruction and no
             // branch; a pair outside the cutoff adds an exact zero (the same
             // forces with and without the energy). Even and odd
             // entries of a tile sum apart in FP32, the tiles in FP64 (6 instructions
             // in 8 pairs; a row's sum then rounds less than pair by pair in FP32).
-            // 168 -> 132 us per launch at 1M atoms (155 with tiles alone): half
-            // the instructions per pair, the gathers' latency and L1 bound it.
+            // 168 -> 126 us per launch at 1M atoms (155 with tiles alone, 132 with
+            // the next tile not loaded ahead): half the instructions per pair,
+            // the gathers' latency and L1 bound it.
             using namespace cp;
             const f2 G0 = f2_pack(-cg, -cg), G1 = f2_pack(-0.25f * cg, -0.25f * cg),
                      G2 = f2_pack(-0.0625f * cg, -0.0625f * cg);
@@ -206,10 +325,14 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal, const float
                      B1 = f2_pack(CELL_BIAS(1), CELL_BIAS(1)),
                      B2 = f2_pack(CELL_BIAS(2), CELL_BIAS(2));
             const f2 A2 = f2_pack(cA, cA), mB2 = f2_pack(-cB, -cB);
-            for (int k = 0; k < n; k += MDB_TILE, nb += (size_t)ld * MDB_TILE) {
+            for (int k = 0; k < n; k += MDB_TILE) {
                 int e[MDB_TILE];
                 float4 pj[MDB_TILE];
-                ld_tile(nb, e);
+#pragma unroll
+                for (int u = 0; u < MDB_TILE; u++)
+                    e[u] = en[u];
+                nb += (size_t)ld * MDB_TILE;
+                if (k + MDB_TILE < n) ld_tile(nb, en);
 #pragma unroll
                 for (int u = 0; u < MDB_TILE; u++)
                     pj[u] = __ldg(xr + entry_index(e[u]));
@@ -253,10 +376,14 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal, const float
                 rz += (double)(t0 + t1);
             }
         } else {
-            for (int k = 0; k < n; k += MDB_TILE, nb += (size_t)ld * MDB_TILE) {
+            for (int k = 0; k < n; k += MDB_TILE) {
                 int e[MDB_TILE];
                 float4 pj[MDB_TILE];
-                ld_tile(nb, e);
+#pragma unroll
+                for (int u = 0; u < MDB_TILE; u++)
+                    e[u] = en[u];
+                nb += (size_t)ld * MDB_TILE;
+                if (k + MDB_TILE < n) ld_tile(nb, en);
 #pragma unroll
                 for (int u = 0; u < MDB_TILE; u++)
                     pj[u] = __ldg(xr + entry_index(e[u]));
@@ -284,17 +411,31 @@ __global__ void __launch_bounds__(LJ_THREADS) k_lj_mixed(int nlocal, const float
     }
 }
 
-template <bool HALF, bool UNIFORM>
-static void lj64(cudaStream_t s, int energy, int nb, int nlocal,
-    const double4* x, const int* numneigh, const int* neighbors, int ld, double cut,
-    const LJTable& tab, double* fx, double* fy, double* fz, double* epart)
+template <bool HALF, bool UNIFORM, bool ENERGY>
+static void lj64(cudaStream_t s, int nlocal, const double4* x, const int* numneigh,
+    const int* neighbors, int ld, double cut, const LJTable& tab, double* fx, double* fy,
+    double* fz, double* epart)
 {
-    if (energy)
-        k_lj_fp64<HALF, UNIFORM, true><<<nb, LJ_THREADS, 0, s>>>(nlocal, x, numneigh,
+    const int nb = lj_fp64_blocks(HALF, nlocal);
+    if (lj_fp64_shared(HALF, nlocal))
+        k_lj_fp64_shared<HALF, UNIFORM, ENERGY><<<nb, LJ_THREADS, 0, s>>>(nlocal, x, numneigh,
             neighbors, ld, cut, tab, fx, fy, fz, epart);
     else
-        k_lj_fp64<HALF, UNIFORM, false><<<nb, LJ_THREADS, 0, s>>>(nlocal, x, numneigh,
-            neighbors, ld, cut, tab, fx, fy, fz, epart);
+        k_lj_fp64<UNIFORM, ENERGY><<<nb, LJ_THREADS, 0, s>>>(nlocal, x, numneigh, neighbors, ld,
+            cut, tab, fx, fy, fz, epart);
+}
+
+template <bool HALF, bool UNIFORM>
+static void lj64_e(cudaStream_t s, int energy, int nlocal, const double4* x, const int* numneigh,
+    const int* neighbors, int ld, double cut, const LJTable& tab, double* fx, double* fy,
+    double* fz, double* epart)
+{
+    if (energy)
+        lj64<HALF, UNIFORM, true>(s, nlocal, x, numneigh, neighbors, ld, cut, tab, fx, fy, fz,
+            epart);
+    else
+        lj64<HALF, UNIFORM, false>(s, nlocal, x, numneigh, neighbors, ld, cut, tab, fx, fy, fz,
+            epart);
 }
 
 void launch_lj_fp64(cudaStream_t s, int half, int energy, int nlocal,
@@ -302,22 +443,11 @@ void launch_lj_fp64(cudaStream_t s, int half, int energy, int nlocal,
     const LJTable& tab, double* fx, double* fy, double* fz, double* epart)
 {
     if (nlocal <= 0) return;
-    int nb = force_partial_blocks(nlocal);
-    if (half) {
-        if (tab.uniform)
-            lj64<true, true>(s, energy, nb, nlocal, x, numneigh, neighbors, ld,
-                cutforcesq, tab, fx, fy, fz, epart);
-        else
-            lj64<true, false>(s, energy, nb, nlocal, x, numneigh, neighbors, ld,
-                cutforcesq, tab, fx, fy, fz, epart);
-    } else {
-        if (tab.uniform)
-            lj64<false, true>(s, energy, nb, nlocal, x, numneigh, neighbors, ld,
-                cutforcesq, tab, fx, fy, fz, epart);
-        else
-            lj64<false, false>(s, energy, nb, nlocal, x, numneigh, neighbors, ld,
-                cutforcesq, tab, fx, fy, fz, epart);
-    }
+#define LJ64(H, U)                                                                       \
+    lj64_e<H, U>(s, energy, nlocal, x, numneigh, neighbors, ld, cutforcesq, tab, fx, fy, fz, epart)
+    if (half) tab.uniform ? LJ64(true, true) : LJ64(true, false);
+    else tab.uniform ? LJ64(false, true) : LJ64(false, false);
+#undef LJ64
     g_launches++;
 }
 

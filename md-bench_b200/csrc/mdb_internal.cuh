@@ -279,7 +279,9 @@ void launch_ke_partial(cudaStream_t s, int n, const double* vx, const double* vy
 void launch_reduce_partials(cudaStream_t s, int nparts, const double* partials, double* out);
 
 // forces (mdb_force_lj.cu, mdb_force_eam.cu)
+// blocks (= energy partials) of the mixed and the FP64 LJ kernels
 int force_partial_blocks(int n);
+int lj_fp64_blocks(int half, int n);
 void launch_lj_fp64(cudaStream_t s, int half, int energy, int nlocal,
     const double4* x, const int* numneigh, const int* neighbors, int ld, double cutforcesq,
     const LJTable& tab, double* fx, double* fy, double* fz, double* epart);
