@@ -46,20 +46,23 @@ int mdb_cp_synchronize(MdbCp* ctx);
 /* Launch tuning (no counterpart in the reference; results are unchanged
  * except where noted):
  * "force_cpw" = i-clusters per warp of the mixed cluster-pair kernel: 1, 2, 4,
- * or 8 with 4x4 clusters (default 4). Each i-cluster gets 32 / force_cpw
+ * or 8 with 4x4 clusters (default by size: half lists of up to 16,384 atoms 1,
+ * 4x4 ones up to 65,536 atoms 2, 4x4 ones of several types from 1,048,577 on 8,
+ * else 4). Each i-cluster gets 32 / force_cpw
  * lanes; the rows of a warp's clusters run side by side. The same pairs are
  * evaluated, but a row's split among the lanes, and so the FP32 rounding of
- * the i sums, depends on the setting. Ensemble members keep theirs;
+ * the i sums, depends on the setting. Ensemble members keep theirs, except
+ * half-list members with no launch setting of their own, which take the
+ * default of a large system;
  * "force_jpl" = j atoms per lane of the mixed cluster-pair kernel: 1, or 2
- * with force_cpw 4 (two consecutive atoms of an entry share a lane's list,
- * anchor and loop work; FP32 rounding changes as for force_cpw; default 2
- * for one atom type, 1 for several types and for 4x8 half lists; ensemble
- * members keep theirs);
+ * with force_cpw 4 (two atoms of an entry share a lane's list, anchor and loop
+ * work; FP32 rounding changes as for force_cpw; default 2; ensemble members
+ * keep theirs);
  * "force_block" = threads per block of the mixed force kernel (32..512, a
  * multiple of 32; default 128); "force_variant" = 0..3: 0 and 1 prefetch the
  * j data one or two list blocks ahead with no register budget, 2 and 3 the same
  * with a budget for 8 resident blocks of 128 threads per SM (these run blocks
- * of 128 threads; default 2; with force_cpw > 1 the prefetch is one block,
+ * of 128 threads; default 0 or 2 by size, list form and types; with force_cpw > 1 the prefetch is one block,
  * 1 runs as 0 and 3 asks a budget for 6 blocks instead of 8);
  * "force_swizzle" = 1: the blocks one resident
  * slot runs in turn take neighbouring i-clusters (L1 reuse of j data; default
