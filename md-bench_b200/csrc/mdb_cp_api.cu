@@ -1128,8 +1128,9 @@ static void enq_prune(MdbCp* ctx)
 }
 
 // T and P from the atom arrays (as computeThermo reads them), KE of the
-// cluster state, PE from the last energy evaluation
-static void enq_thermo(MdbCp* ctx, int slot, bool with_pe)
+// cluster state, PE from the eblocks partials of the last energy evaluation
+// (0: no PE)
+static void enq_thermo(MdbCp* ctx, int slot, int eblocks)
 {
     cudaStream_t s = ctx->s;
     double* r      = ctx->red + 4 * slot;
@@ -1138,7 +1139,7 @@ static void enq_thermo(MdbCp* ctx, int slot, bool with_pe)
     launch_reduce_partials(s, ke_blocks(ctx->nlocal), pk, r + 0);
     launch_ke_slots(s, ctx->M, ctx->ncl_cap, ctx->cnt, ctx->cx, ctx->cv, ctx->p.mass, pk);
     launch_reduce_partials(s, ke_blocks(ctx->ncl_cap * ctx->M), pk, r + 2);
-    if (with_pe) launch_reduce_partials(s, ctx->energy_blocks, ctx->partials, r + 1);
+    if (eblocks > 0) launch_reduce_partials(s, eblocks, ctx->partials, r + 1);
     else cudaMemsetAsync(r + 1, 0, sizeof(double), s);
 }
 
@@ -1367,7 +1368,7 @@ extern "C" int mdb_cp_thermo(MdbCp* ctx, MdbThermo* out)
     }
     bool pe     = ctx->energy_valid && ctx->have_clusters;
     if (ctx->have_clusters) {
-        enq_thermo(ctx, 0, pe);
+        enq_thermo(ctx, 0, pe ? ctx->energy_blocks : 0);
     } else {
         double* pk = ctx->partials + ctx->npart;
         launch_ke_atoms(ctx->s, ctx->nlocal, ctx->av, ctx->p.mass, pk);
@@ -1669,7 +1670,7 @@ static int run_checked(MdbCp* ctx, int first_step, int nsteps, MdbThermo* sample
         if (sample || n == last) enq_final(ctx);
         else pending_final = true;
         if (sample && nslot < RED_SLOTS && nslot < max_samples) {
-            enq_thermo(ctx, nslot, true);
+            enq_thermo(ctx, nslot, ctx->energy_blocks);
             slot_step.push_back(n + 1);
             nslot++;
         }
@@ -1769,7 +1770,7 @@ extern "C" int mdb_cp_run(MdbCp* ctx, int first_step, int nsteps, MdbThermo* sam
         if (sample || n == last) enq_final(ctx);
         else pending_final = true;
         if (sample && nslot < RED_SLOTS && nslot < max_samples) {
-            enq_thermo(ctx, nslot, true);
+            enq_thermo(ctx, nslot, ctx->energy_blocks);
             slot_step.push_back(n + 1);
             nslot++;
         }
@@ -2052,6 +2053,10 @@ struct MdbCpEnsemble {
     int2* h_dyn = nullptr;
     std::vector<int> gid;
     std::vector<Group> groups;
+    // energy partials a batched energy launch writes per member. A member alone
+    // may write another number (MdbCp::energy_blocks): its launch shape goes by
+    // its own size (ens_types)
+    std::vector<int> epart;
 };
 
 // step parts captured per ensemble: FI = final integration of the previous
@@ -2117,7 +2122,7 @@ static void ens_body(MdbCp* c, int kind)
     case EG_SAMPLE:
         enq_force(c, true);
         enq_final(c);
-        enq_thermo(c, 0, true);
+        enq_thermo(c, 0, c->energy_blocks);
         cudaMemcpyAsync(c->h_red, c->red, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->s);
         break;
     case EG_FINAL: enq_final(c); break;
@@ -2262,15 +2267,14 @@ static int ens_tables(MdbCpEnsemble* e)
             e->groups.push_back({c->N, c->p.half_neigh, ens_types(c), cutsq, 0, 0});
         }
     }
+    e->epart.assign(n, 0);
     for (size_t q = 0; q < e->groups.size(); q++) {
         auto& gr = e->groups[q];
         gr.off   = maps.size();
         for (int k = 0; k < n; k++)
             if (gid[k] == (int)q) {
-                MdbCp* c         = e->m[k];
-                const int nb     = force_mixed_grid(c->ncl_cap, gr.ty);
-                c->energy_blocks = nb; // the partials a batched energy launch writes
-                add(k, nb);
+                e->epart[k] = force_mixed_grid(e->m[k]->ncl_cap, gr.ty);
+                add(k, e->epart[k]);
             }
         gr.nblocks = (int)(maps.size() - gr.off);
     }
@@ -2362,7 +2366,7 @@ template <class F> static void ens_fork(MdbCpEnsemble* e, F&& body)
     for (size_t k = 0; k < e->m.size(); k++) {
         MdbCp* c = e->m[k];
         cudaStreamWaitEvent(c->s, e->fork, 0);
-        body(c);
+        body(c, k);
         cudaEventRecord(e->join[k], c->s);
         cudaStreamWaitEvent(e->s, e->join[k], 0);
     }
@@ -2457,8 +2461,8 @@ static void ens_body_batched(MdbCpEnsemble* e, int kind)
     case EG_SAMPLE:
         ens_forces(e, true);
         ens_integ(e, true, false);
-        ens_fork(e, [](MdbCp* c) {
-            enq_thermo(c, 0, true);
+        ens_fork(e, [e](MdbCp* c, size_t k) {
+            enq_thermo(c, 0, e->epart[k]);
             cudaMemcpyAsync(c->h_red, c->red, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->s);
         });
         break;
@@ -2695,7 +2699,7 @@ static int ens_capture(MdbCpEnsemble* e, int kind)
     cudaError_t ce = cudaStreamBeginCapture(e->s, cudaStreamCaptureModeThreadLocal);
     if (ce != cudaSuccess) return ens_fail(e, MDB_ERR_CUDA, "ensemble capture", ce);
     if (e->batched) ens_body_batched(e, kind);
-    else ens_fork(e, [kind](MdbCp* c) { ens_body(c, kind); });
+    else ens_fork(e, [kind](MdbCp* c, size_t) { ens_body(c, kind); });
     ce        = cudaStreamEndCapture(e->s, &graph);
     g.kernels = mdb::g_launches - m0;
     mdb::g_launches = m0;
@@ -2960,6 +2964,8 @@ extern "C" int mdb_cp_ensemble_run(MdbCpEnsemble* e, int first_step, int nsteps,
         if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_rebcnt, 0, n * sizeof(int), e->s);
         if (ce != cudaSuccess) return ens_fail(e, MDB_ERR_NOMEM, "checked steps", ce);
     }
+    if (nsteps > 0) // until a sample of the last step, or the end of the run
+        for (MdbCp* c : e->m) c->energy_valid = c->force_current = false;
     std::vector<int> launched;
     const int last     = first_step + nsteps - 1;
     bool pending_final = false;
@@ -3038,6 +3044,9 @@ extern "C" int mdb_cp_ensemble_run(MdbCpEnsemble* e, int first_step, int nsteps,
             for (int k = 0; k < n; k++) {
                 MdbCp* c = e->m[k];
                 finish_thermo(c, c->h_red, step + 1, &samples[(size_t)k * max_samples + nslot]);
+                if (step != last) continue;
+                // the member's own reductions read this evaluation's partials
+                if (e->batched) c->energy_blocks = e->epart[k];
                 c->energy_valid = true;
             }
             nslot++;
@@ -3046,6 +3055,8 @@ extern "C" int mdb_cp_ensemble_run(MdbCpEnsemble* e, int first_step, int nsteps,
     if (pending_final && (rc = ens_launch(e, EG_FINAL))) return rc;
     cudaError_t ce = cudaStreamSynchronize(e->s);
     if (ce != cudaSuccess) return ens_fail(e, MDB_ERR_CUDA, "ensemble run", ce);
+    if (nsteps > 0)
+        for (MdbCp* c : e->m) c->force_current = true;
     if (nsamples) *nsamples = nslot;
     return MDB_OK;
 }
