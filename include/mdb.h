@@ -118,8 +118,7 @@ void mdb_eam_free(MdbEamTables* t);
 /* Local atoms, AoS arrays. Replaces copyDataToCUDADevice /
  * copyDataFromCUDADevice (verletlist/forceCuda.cu:331-343). The arrays may be
  * host or device memory of the context's device (unified addressing), so a
- * caller that keeps its atoms on the GPU moves them without a host copy (the
- * types of device arrays are copied to the host once, to be checked). */
+ * caller that keeps its atoms on the GPU moves them without a host copy. */
 int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const double* v, const int* type);
 int mdb_get_atoms(MdbCtx* ctx, double* x, double* v, double* f, int* type);
 

@@ -79,7 +79,8 @@ struct MdbCtx {
     // and their count per atom, written by the density pass
     int *eam_cutlist = nullptr, *eam_ncut = nullptr;
     double* stage  = nullptr; // 9 * nlocal doubles: AoS x, v, f for host transfers
-    int* stage_t   = nullptr; // nlocal types
+    int* stage_t   = nullptr; // the atoms' types
+    int stage_t_n  = 0;       // ints in it
     double4 *eam_frho = nullptr, *eam_rhor = nullptr, *eam_z2r = nullptr; // see EamDev
     float4 *eam_dens32 = nullptr, *eam_pair32 = nullptr;
     EamDev eam;
@@ -448,7 +449,6 @@ static void free_atom_buffers(MdbCtx* ctx)
     dfree(ctx->fp);
     dfree(ctx->xe);
     dfree(ctx->stage);
-    dfree(ctx->stage_t);
     if (ctx->h_red) cudaFreeHost(ctx->h_red);
     ctx->h_red = nullptr;
 }
@@ -459,6 +459,7 @@ extern "C" int mdb_destroy(MdbCtx* ctx)
     if (ctx->s) cudaStreamSynchronize(ctx->s);
     drop_graphs(ctx);
     free_atom_buffers(ctx);
+    dfree(ctx->stage_t);
     dfree(ctx->counters);
     dfree(ctx->rows_d);
     dfree(ctx->bin_count);
@@ -551,6 +552,18 @@ static int alloc_list(MdbCtx* ctx, int maxneighs)
     return MDB_OK;
 }
 
+// room for n types, with the atom buffers' reserve; scratch only, so it may grow
+// before a call is known to be accepted
+static int grow_stage_t(MdbCtx* ctx, int n)
+{
+    if (ctx->stage_t && n <= ctx->stage_t_n) return MDB_OK;
+    dfree(ctx->stage_t);
+    ctx->stage_t_n = 0;
+    CK(dalloc(&ctx->stage_t, n + n / 32 + 64));
+    ctx->stage_t_n = n + n / 32 + 64;
+    return MDB_OK;
+}
+
 extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const double* v,
     const int* type)
 {
@@ -559,15 +572,23 @@ extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const dou
     ctx->nown = 0; // new atoms: all owned until mdb_set_owned
     // host or device arrays (unified addressing); the types are checked here, on
     // the side where they are (the legacy stream orders the check after the work
-    // that wrote them there, as a copy to the host would)
+    // that wrote them there, as a copy to the host would). The kernel reads a copy
+    // of device types: a copy takes any address (not aligned, another GPU's) and
+    // is refused where the array is too short.
+    int rc = grow_stage_t(ctx, nlocal);
+    if (rc) return rc;
     int maxt = 0;
     cudaPointerAttributes pa;
-    if (nlocal > 0 && cudaPointerGetAttributes(&pa, type) == cudaSuccess &&
-        (pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeManaged)) {
+    const bool dev_types =
+        nlocal > 0 && cudaPointerGetAttributes(&pa, type) == cudaSuccess &&
+        (pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeManaged);
+    if (dev_types) {
         int range[2];
+        CK(cudaMemcpyAsync(ctx->stage_t, type, sizeof(int) * nlocal, cudaMemcpyDefault,
+            cudaStreamLegacy));
         CK(cudaMemsetAsync(ctx->counters + CNT_TYPES, 0, sizeof range, cudaStreamLegacy));
         const long long m = launch_mark();
-        launch_type_range(cudaStreamLegacy, nlocal, type, ctx->counters + CNT_TYPES);
+        launch_type_range(cudaStreamLegacy, nlocal, ctx->stage_t, ctx->counters + CNT_TYPES);
         launch_account(ctx, m);
         CK(cudaMemcpy(range, ctx->counters + CNT_TYPES, sizeof range, cudaMemcpyDeviceToHost));
         if (range[1]) return fail(ctx, MDB_ERR_ARG, "negative atom type");
@@ -579,7 +600,7 @@ extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const dou
         }
     }
     cudaGetLastError();
-    int rc = setup_types(ctx, std::max(ctx->p.ntypes, maxt));
+    rc = setup_types(ctx, std::max(ctx->p.ntypes, maxt));
     if (rc) return rc;
     // the buffers are kept while the atom count stays within the capacity
     // (a domain's atom count changes a little at every rebuild)
@@ -615,7 +636,6 @@ extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const dou
         if (ctx->p.force_field == MDB_FF_EAM && ctx->mixed) CK(dalloc(&ctx->eam_ncut, cap));
         CK(dalloc(&ctx->local_order, cap));
         CK(dalloc(&ctx->stage, 9 * (size_t)cap));
-        CK(dalloc(&ctx->stage_t, cap));
         int nscan         = std::max(scan_scratch_ints(cap), scan_scratch_ints(ctx->g.mbins));
         ctx->scan_scratch_n = nscan;
         CK(dalloc(&ctx->scan_scratch, nscan));
@@ -645,7 +665,8 @@ extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const dou
     size_t n3      = 3 * (size_t)nlocal;
     CK(cudaMemcpyAsync(ctx->stage, x, sizeof(double) * n3, cudaMemcpyDefault, s));
     CK(cudaMemcpyAsync(ctx->stage + n3, v, sizeof(double) * n3, cudaMemcpyDefault, s));
-    CK(cudaMemcpyAsync(ctx->stage_t, type, sizeof(int) * nlocal, cudaMemcpyDefault, s));
+    if (!dev_types)
+        CK(cudaMemcpyAsync(ctx->stage_t, type, sizeof(int) * nlocal, cudaMemcpyDefault, s));
     {
         long long m = launch_mark();
         launch_pack_atoms(s, nlocal, ctx->stage, ctx->stage + n3, ctx->stage_t, ctx->x, ctx->vx,
