@@ -2129,13 +2129,30 @@ static void ens_body(MdbCp* c, int kind)
     }
 }
 
-// a member's types and launch shape in an ensemble: half lists that the caller
-// has not tuned take the shape of a large system, as the members fill the chip
-// together
-static Types ens_types(const MdbCp* c)
+// A member's types and launch shape in an ensemble, whose members fill the chip
+// together. Members that the caller has not tuned take, with half lists, the shape
+// of a large system. With full lists they follow their run alone bit for bit, so
+// only what leaves the sums alone changes: the register budget (variant 2) goes by
+// the atoms n of all such members. us per batched launch without / with it, one type:
+//   atoms     96,000       228,592      389,208      1,224,764
+//   4x4    23.2 / 23.6   48.8 / 45.5  91.0 / 75.8    304 / 232
+//   4x8    24.0 / 26.3   50.8 / 51.8  88.8 / 83.1    292 / 250
+// Four types, 4x4: 58.2 / 63.8 at 229,972 atoms, 103.2 / 103.9 at 391,460, 182.7 /
+// 172.0 at 662,648; 4x8: 356 / 372 at 1,233,840.
+static Types ens_types(const MdbCpEnsemble* e, const MdbCp* c)
 {
     Types t = c->ty;
-    if (c->p.half_neigh && !c->tuned) set_force_shape(t, c->N, 1, 1 << 30);
+    if (c->tuned) return t;
+    if (c->p.half_neigh) {
+        set_force_shape(t, c->N, 1, 1 << 30);
+        return t;
+    }
+    long long n = 0;
+    for (const MdbCp* m : e->m)
+        if (!m->tuned && !m->p.half_neigh && m->N == c->N) n += m->nlocal;
+    const bool budget = t.uniform ? n > (c->N == 4 ? 1 << 17 : 1 << 18)
+                                  : c->N == 4 && n > 1 << 19;
+    t.force_variant = budget ? 2 : 0;
     return t;
 }
 
@@ -2255,16 +2272,17 @@ static int ens_tables(MdbCpEnsemble* e)
     std::vector<int> gid(n, -1);
     for (int k = 0; k < n; k++) {
         const MdbCp* c    = e->m[k];
+        const Types ty    = ens_types(e, c);
         const float cutsq = (float)c->cutforcesq;
         for (size_t q = 0; q < e->groups.size() && gid[k] < 0; q++) {
             const auto& gr = e->groups[q];
             if (gr.N == c->N && gr.half == c->p.half_neigh && gr.cutsq == cutsq &&
-                same_types(gr.ty, ens_types(c)))
+                same_types(gr.ty, ty))
                 gid[k] = (int)q;
         }
         if (gid[k] < 0) {
             gid[k] = (int)e->groups.size();
-            e->groups.push_back({c->N, c->p.half_neigh, ens_types(c), cutsq, 0, 0});
+            e->groups.push_back({c->N, c->p.half_neigh, ty, cutsq, 0, 0});
         }
     }
     e->epart.assign(n, 0);
