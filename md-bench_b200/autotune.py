@@ -41,15 +41,14 @@ CPWS = (1, 2, 4, 8)
 JPLS = (1, 2)
 EDGES = (80, 100, 125)
 DEFAULT = {"cluster_n": 4, "half": 1, "column_edge": 100, "force_block": 128,
-           "force_variant": 2, "force_cpw": 4, "force_jpl": 1}
+           "force_variant": 2, "force_cpw": 4, "force_jpl": 2}
 
 
 def valid(choice):
     """force_cpw 8 needs 4x4 clusters; several clusters per warp prefetch one
-    block ahead (variant 1 runs as 0 there; 3 is a budget for 6 blocks)."""
+    block ahead (variant 1 runs as 0 there; 3 is a budget for 6 blocks).
+    force_jpl acts with four clusters per warp and is free otherwise."""
     if choice.get("force_cpw", 1) == 8 and choice["cluster_n"] != 4:
-        return False
-    if choice.get("force_jpl", 1) == 2 and choice.get("force_cpw", 1) != 4:
         return False
     return not (choice.get("force_cpw", 1) > 1 and choice.get("force_variant", 0) == 1)
 
@@ -84,7 +83,7 @@ def tune_system(build, precision="mixed", reps=20, shapes=SHAPES, forms=FORMS, e
                                                for w in CPWS for p in JPLS):
                         c = dict(base, force_block=blk, force_variant=var, force_cpw=cpw,
                                  force_jpl=jpl)
-                        if not valid(c):
+                        if not valid(c) or (jpl == 2 and cpw != 4):
                             continue
                         apply_launch(s, c)
                         t = s.time_force(reps)
@@ -117,7 +116,8 @@ def tune_ensemble(specs, build, steps=20, rounds=2, shapes=SHAPES, forms=FORMS, 
     ensemble's throughput. ``specs`` is a list of replica descriptions with an
     ``natoms`` entry; ``build(spec, cluster_n, half, column_edge)`` returns a
     set-up mixed-precision ClusterSystem (with ``close()``). Every class starts
-    at DEFAULT; classes are visited largest (total atoms) first, each trying
+    at DEFAULT, its launch settings included (a member left untuned would run
+    another launch than the choice says); classes are visited largest (total atoms) first, each trying
     the other shapes and list forms, then the other bin sizes of its shape,
     then the other threads per block and kernel variants, with every other
     class at its current choice. A change is kept
@@ -139,6 +139,8 @@ def tune_ensemble(specs, build, steps=20, rounds=2, shapes=SHAPES, forms=FORMS, 
     def everyone():
         return [m for c in sorted(members) for m in members[c]]
 
+    for m in everyone():
+        apply_launch(m, DEFAULT)
     best = rate(everyone())
     trials = [(None, dict(DEFAULT), best)]
 
@@ -181,6 +183,8 @@ def tune_ensemble(specs, build, steps=20, rounds=2, shapes=SHAPES, forms=FORMS, 
             for val in values:
                 if val == choice[c][key]:
                     continue
+                if key == "force_jpl" and choice[c]["force_cpw"] != 4:
+                    continue  # the same launch
                 trial = dict(choice[c], **{key: val})
                 if not valid(trial):
                     continue

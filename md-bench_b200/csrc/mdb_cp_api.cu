@@ -376,7 +376,7 @@ extern "C" int mdb_cp_tune(MdbCp* ctx, const char* key, int value)
         return MDB_OK;
     }
     if (!strcmp(key, "force_jpl")) {
-        // 2: single systems with force_cpw 4
+        // 2 acts with force_cpw 4
         if (value != 1 && value != 2) return MDB_ERR_ARG;
         drop_graph(ctx);
         ctx->ty.force_jpl = value, ctx->tuned = true;

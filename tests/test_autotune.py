@@ -97,6 +97,31 @@ def test_no_change_within_noise():
     assert all(m.closed for m in log)
 
 
+def test_losing_trials_return_what_was_measured_first():
+    """Members start untuned (launch settings by size): the first measurement is
+    of the returned choice, and so is the state after every trial that lost."""
+    class Untuned(FakeMember):
+        def __init__(self, *a):
+            super().__init__(*a)
+            self.launch = {}
+
+    specs = [{"natoms": 500}] * 2 + [{"natoms": 32000}]
+    log, seen = [], []
+
+    def rate(members):
+        seen.append([(m.natoms, m.cluster_n, m.half, m.edge, dict(m.launch)) for m in members])
+        return 1.0 / len(seen)
+
+    choice, trials = AT.tune_ensemble(specs, lambda sp, n, h, e: Untuned(sp, n, h, e, log),
+                                      rate=rate)
+    for natoms, n, half, edge, launch in seen[0]:
+        assert dict(cluster_n=n, half=half, column_edge=edge, **launch) == \
+            choice[AT.size_class(natoms)]
+    # every trial changes what runs: none repeats the launch of the choice
+    assert all(s != seen[0] for s in seen[1:])
+    assert len(trials) == len(seen)
+
+
 class FakeSystem:
     """A single system whose force time the model below gives."""
 
