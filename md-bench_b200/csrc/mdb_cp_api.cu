@@ -2168,6 +2168,17 @@ static bool same_types(const Types& a, const Types& b)
     return true;
 }
 
+// A table to the device in the order of e->s, whose graphs read it. (cudaMemcpy
+// returns once pageable memory is staged, and the copy that follows on the legacy
+// stream is not ordered before a non-blocking stream's work.)
+template <class T>
+static cudaError_t ens_upload(MdbCpEnsemble* e, T* dst, const std::vector<T>& src)
+{
+    return src.empty() ? cudaSuccess
+                       : cudaMemcpyAsync(dst, src.data(), sizeof(T) * src.size(),
+                             cudaMemcpyHostToDevice, e->s);
+}
+
 // the dynamic block maps from the members' counters as the last build left
 // them (host copies in h_cnt); stream-ordered before the next graph launch
 static int ens_dyn_maps(MdbCpEnsemble* e)
@@ -2315,7 +2326,7 @@ static int ens_tables(MdbCpEnsemble* e)
             ce = cudaMallocHost((void**)&e->h_cnt_all, sizeof(int) * CP_SLOTS * n);
         if (ce == cudaSuccess) ce = cudaMalloc((void**)&e->d_flags, sizeof(int) * n);
         if (ce == cudaSuccess) ce = cudaMallocHost((void**)&e->h_flags, sizeof(int) * n);
-        if (ce == cudaSuccess) ce = cudaMemset(e->d_flags, 0, sizeof(int) * n);
+        if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_flags, 0, sizeof(int) * n, e->s);
         if (ce != cudaSuccess) return ens_fail(e, MDB_ERR_NOMEM, "ensemble tables", ce);
     }
     if (maps.size() > e->bmap_cap) {
@@ -2333,17 +2344,15 @@ static int ens_tables(MdbCpEnsemble* e)
     }
     for (int k = 0; k < n; k++) st[k].flag = e->d_flags + k;
     const char* what = "member table";
-    ce = cudaMemcpy(e->d_step, st.data(), sizeof(CpStepMember) * n, cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess)
-        ce = cudaMemcpy(e->d_force, fo.data(), sizeof(CpForceMember) * n, cudaMemcpyHostToDevice);
+    ce = ens_upload(e, e->d_step, st);
+    if (ce == cudaSuccess) ce = ens_upload(e, e->d_force, fo);
     if (ce == cudaSuccess) {
         what = "rebuild table";
-        ce = cudaMemcpy(e->d_build, bt.data(), sizeof(CpBuildMember) * n, cudaMemcpyHostToDevice);
+        ce   = ens_upload(e, e->d_build, bt);
     }
-    if (ce == cudaSuccess && !maps.empty()) {
+    if (ce == cudaSuccess) {
         what = "block maps";
-        ce   = cudaMemcpy(e->d_bmap, maps.data(), sizeof(int2) * maps.size(),
-            cudaMemcpyHostToDevice);
+        ce   = ens_upload(e, e->d_bmap, maps);
     }
     if (ce != cudaSuccess) return ens_fail(e, MDB_ERR_CUDA, what, ce);
     e->tables_ok = true;
@@ -2591,11 +2600,9 @@ static int ens_map_info(MdbCpEnsemble* e)
         if (ce != cudaSuccess) return ens_fail(e, MDB_ERR_NOMEM, "ensemble map table", ce);
     }
     if (ng > 64) return ens_fail(e, MDB_ERR_ARG, "more than 64 force groups");
-    ce = cudaMemcpy(e->d_mapinfo, info.data(), sizeof(int) * info.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess)
-        ce = cudaMemcpy(e->d_goff, goff.data(), sizeof(size_t) * goff.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess)
-        ce = cudaMemcpy(e->d_gnb, gnb.data(), sizeof(int) * gnb.size(), cudaMemcpyHostToDevice);
+    ce = ens_upload(e, e->d_mapinfo, info);
+    if (ce == cudaSuccess) ce = ens_upload(e, e->d_goff, goff);
+    if (ce == cudaSuccess) ce = ens_upload(e, e->d_gnb, gnb);
     if (ce != cudaSuccess) return ens_fail(e, MDB_ERR_CUDA, "ensemble map table", ce);
     return MDB_OK;
 }
