@@ -402,9 +402,12 @@ extern "C" int mdb_create(const MdbParams* params, MdbCtx** out)
             rc = fail(ctx, MDB_ERR_NOMEM, "device allocation", e);
             goto bad;
         }
-        cudaMemset(ctx->counters, 0, CNT_SLOTS * sizeof(int));
-        cudaMemcpy(ctx->rows_d, ctx->stencil_rows.data(), sizeof(int4) * ctx->stencil_rows.size(),
-            cudaMemcpyHostToDevice);
+        // uploads and clearings go through ctx->s: what cudaMemcpy and cudaMemset
+        // leave on the legacy stream is not ordered before a non-blocking stream
+        cudaMemsetAsync(ctx->counters, 0, CNT_SLOTS * sizeof(int), ctx->s);
+        cudaMemcpyAsync(ctx->rows_d, ctx->stencil_rows.data(),
+            sizeof(int4) * ctx->stencil_rows.size(), cudaMemcpyHostToDevice, ctx->s);
+        cudaStreamSynchronize(ctx->s); // mdb_set_atoms uses counters on the legacy stream
         if ((e = cudaGetLastError()) != cudaSuccess) {
             rc = fail(ctx, MDB_ERR_CUDA, "setup copy", e);
             goto bad;
@@ -626,12 +629,12 @@ extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const dou
         CK(dalloc(&ctx->fx, cap));
         CK(dalloc(&ctx->fy, cap));
         CK(dalloc(&ctx->fz, cap));
-        CK(cudaMemset(ctx->fx, 0, sizeof(double) * cap));
-        CK(cudaMemset(ctx->fy, 0, sizeof(double) * cap));
-        CK(cudaMemset(ctx->fz, 0, sizeof(double) * cap));
+        CK(cudaMemsetAsync(ctx->fx, 0, sizeof(double) * cap, ctx->s));
+        CK(cudaMemsetAsync(ctx->fy, 0, sizeof(double) * cap, ctx->s));
+        CK(cudaMemsetAsync(ctx->fz, 0, sizeof(double) * cap, ctx->s));
         CK(dalloc(&ctx->ghost_cnt, cap + 1));
         CK(dalloc(&ctx->ghost_off, cap + 1));
-        CK(cudaMemset(ctx->ghost_off, 0, sizeof(int) * (cap + 1)));
+        CK(cudaMemsetAsync(ctx->ghost_off, 0, sizeof(int) * (cap + 1), ctx->s));
         CK(dalloc(&ctx->numneigh, cap));
         if (ctx->p.force_field == MDB_FF_EAM && ctx->mixed) CK(dalloc(&ctx->eam_ncut, cap));
         CK(dalloc(&ctx->local_order, cap));
@@ -1178,10 +1181,12 @@ extern "C" int mdb_set_neighbor_list(MdbCtx* ctx, const int* numneigh, const int
     for (int i = 0; i < n; i++)
         for (int k = 0; k < numneigh[i]; k++)
             all[list_at(k, ctx->ld, i)] = neighbors[(size_t)i * ld + k];
-    CK(cudaStreamSynchronize(ctx->s));
-    CK(cudaMemcpy(ctx->neighbors, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->numneigh, numneigh, sizeof(int) * n, cudaMemcpyHostToDevice));
-    CK(cudaMemset(ctx->counters + CNT_NGHOST, 0, sizeof(int)));
+    cudaStream_t s = ctx->s;
+    CK(cudaMemcpyAsync(ctx->neighbors, all.data(), sizeof(int) * all.size(),
+        cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(ctx->numneigh, numneigh, sizeof(int) * n, cudaMemcpyHostToDevice, s));
+    CK(cudaMemsetAsync(ctx->counters + CNT_NGHOST, 0, sizeof(int), s));
+    CK(cudaStreamSynchronize(s));
     ctx->have_ghosts = ctx->have_list = true;
     return MDB_OK;
 }
@@ -1378,13 +1383,15 @@ extern "C" int mdb_set_eam(MdbCtx* ctx, const MdbEamTables* t)
     CK(dalloc(&ctx->eam_z2r, zr.size()));
     CK(dalloc(&ctx->eam_dens32, dens32.size()));
     CK(dalloc(&ctx->eam_pair32, pair32.size()));
-    CK(cudaMemcpy(ctx->eam_frho, fr.data(), fr.size() * sizeof(double4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->eam_rhor, rr.data(), rr.size() * sizeof(double4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->eam_z2r, zr.data(), zr.size() * sizeof(double4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->eam_dens32, dens32.data(), dens32.size() * sizeof(float4),
-        cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->eam_pair32, pair32.data(), pair32.size() * sizeof(float4),
-        cudaMemcpyHostToDevice));
+    auto upload = [ctx](void* dst, const auto& src) {
+        return cudaMemcpyAsync(dst, src.data(), src.size() * sizeof(src[0]),
+            cudaMemcpyHostToDevice, ctx->s);
+    };
+    CK(upload(ctx->eam_frho, fr));
+    CK(upload(ctx->eam_rhor, rr));
+    CK(upload(ctx->eam_z2r, zr));
+    CK(upload(ctx->eam_dens32, dens32));
+    CK(upload(ctx->eam_pair32, pair32));
     ctx->eam.nrho   = t->nrho;
     ctx->eam.nr     = t->nr;
     ctx->eam.rdr    = t->rdr;

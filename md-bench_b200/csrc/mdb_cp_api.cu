@@ -532,8 +532,9 @@ static int alloc_columns(MdbCp* ctx)
     ctx->ncl_col    = z + 2 * (size_t)mb1;
     ctx->gcol_count = z + 3 * (size_t)mb1;
     ctx->gfill      = z + 4 * (size_t)mb1;
-    if ((e = cudaMemcpy(ctx->stencil_d, ctx->stencil.data(), sizeof(int) * ctx->g.nstencil,
-             cudaMemcpyHostToDevice)) != cudaSuccess)
+    // (in the order of ctx->s, as every upload)
+    if ((e = cudaMemcpyAsync(ctx->stencil_d, ctx->stencil.data(),
+             sizeof(int) * ctx->g.nstencil, cudaMemcpyHostToDevice, ctx->s)) != cudaSuccess)
         return fail(ctx, MDB_ERR_CUDA, "stencil copy", e);
     return MDB_OK;
 }
@@ -599,7 +600,7 @@ extern "C" int mdb_cp_create(const MdbParams* params, int cluster_n, int prune_e
             rc = fail(ctx, MDB_ERR_NOMEM, "device allocation", e);
             goto bad;
         }
-        cudaMemset(ctx->cnt, 0, CP_SLOTS * sizeof(int));
+        cudaMemsetAsync(ctx->cnt, 0, CP_SLOTS * sizeof(int), ctx->s);
         if ((rc = alloc_columns(ctx)) != MDB_OK) goto bad;
     }
     *out = ctx;
