@@ -589,11 +589,12 @@ extern "C" int mdb_set_atoms(MdbCtx* ctx, int nlocal, const double* x, const dou
         int range[2];
         CK(cudaMemcpyAsync(ctx->stage_t, type, sizeof(int) * nlocal, cudaMemcpyDefault,
             cudaStreamLegacy));
-        CK(cudaMemsetAsync(ctx->counters + CNT_TYPES, 0, sizeof range, cudaStreamLegacy));
         const long long m = launch_mark();
         launch_type_range(cudaStreamLegacy, nlocal, ctx->stage_t, ctx->counters + CNT_TYPES);
         launch_account(ctx, m);
         CK(cudaMemcpy(range, ctx->counters + CNT_TYPES, sizeof range, cudaMemcpyDeviceToHost));
+        // zero again for the next check, in that stream's order
+        CK(cudaMemsetAsync(ctx->counters + CNT_TYPES, 0, sizeof range, cudaStreamLegacy));
         if (range[1]) return fail(ctx, MDB_ERR_ARG, "negative atom type");
         maxt = range[0];
     } else {

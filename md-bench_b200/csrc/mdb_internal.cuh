@@ -43,7 +43,7 @@ enum {
     CNT_MAXNEED      = 2, // largest numneigh seen when a row overflowed
     CNT_BADBIN       = 3, // atoms found outside the bin grid
     CNT_BADCELL      = 4, // mixed path: neighbour farther than two cells
-    CNT_TYPES        = 5, // and 6: the type check's two ints
+    CNT_TYPES        = 5, // and 6: the type check's two ints (zero between checks)
     CNT_SLOTS        = 8
 };
 
