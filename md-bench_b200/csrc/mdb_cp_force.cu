@@ -14,8 +14,7 @@ namespace cp {
 
 int force_blocks(int ncl_cap)
 {
-    // the FP64 kernel runs one thread per slot, the mixed one a warp per
-    // i-cluster; both size their partial-energy arrays by this count
+    // a warp per i-cluster: the largest launch, which sizes the partial energies
     long long t = (long long)ncl_cap * 32;
     return mdb_blocks(t, CP_FORCE_THREADS);
 }
@@ -201,11 +200,101 @@ __global__ void __launch_bounds__(FP64_THREADS) k_force_fp64(const int* __restri
     }
 }
 
+// Half lists of large systems, pair by pair behind the branch on the cutoff: the
+// four i atoms of a cluster then meet a j atom in the same instruction, and their
+// reactions reach one sector together. Queued, every thread is at another j atom; once
+// the force slots have left L2 that costs more than the idle threads of the branch.
+// us per launch queued / here, 4x4: 320 / 341 at 520,200 atoms, 477 / 466 at 753,768,
+// 664 / 635 at 1,048,576, 1,263 / 1,165 at 2,048,000; 4x8: 663 / 681 at 1,048,576, 1,292 /
+// 1,286 at 2,048,000. Four types: 394 / 404 at 520,200 and 810 / 758 at 1,048,576 (4x4),
+// 414 / 421 and 790 / 782 (4x8).
+template <int N, bool ENERGY>
+__global__ void __launch_bounds__(FP64_THREADS) k_force_fp64_half(const int* __restrict__ cnt,
+    const double4* __restrict__ cx, Types ty, double cutforcesq, const int* __restrict__ list,
+    int ks, int cs, const int* __restrict__ numneigh, double4* cf, double* epart)
+{
+    constexpr int M = CP_M;
+    __shared__ double s_se[MDB_MAX_TYPES], s_s3[MDB_MAX_TYPES];
+    if (threadIdx.x < MDB_MAX_TYPES) {
+        s_se[threadIdx.x] = ty.sqrt_eps[threadIdx.x];
+        s_s3[threadIdx.x] = ty.sigma3[threadIdx.x];
+    }
+    __syncthreads();
+    const int s      = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nloc   = cnt[CP_NCL] * M;
+    const double4 pi = s < nloc ? cx[s] : make_double4(0.0, 0.0, 0.0, type_bits(-1));
+    const int ti     = slot_type(pi);
+    double epot      = 0.0;
+    if (ti >= 0) { // neither past the locals nor padding
+        const int ci = s / M, a = s - ci * M;
+        const int ci_cj0 = ci / (N / M);
+        const int ai     = a + M * (ci % (N / M));
+        const double se_i = s_se[ti], s3_i = s_s3[ti];
+        const int nn      = numneigh[ci];
+        double fx = 0.0, fy = 0.0, fz = 0.0;
+        for (int k = 0; k < nn; k++) {
+            const int cj = __ldg(&list[(size_t)k * ks + (size_t)ci * cs]);
+            double fix = 0.0, fiy = 0.0, fiz = 0.0;
+#pragma unroll
+            for (int b = 0; b < N; b++) {
+                if (ci_cj0 == cj && ai >= b) continue;
+                const int sj      = cj * N + b;
+                const double4 pj  = ldg4(&cx[sj]);
+                const double delx = pi.x - pj.x;
+                const double dely = pi.y - pj.y;
+                const double delz = pi.z - pj.z;
+                const double rsq  = delx * delx + dely * dely + delz * delz;
+                if (rsq < cutforcesq) {
+                    const int tj       = max(slot_type(pj), 0);
+                    const double sig6  = s3_i * s_s3[tj];
+                    const double eps   = se_i * s_se[tj];
+                    const double sr2   = 1.0 / rsq;
+                    const double sr6   = sr2 * sr2 * sr2 * sig6;
+                    const double force = 48.0 * sr6 * (sr6 - 0.5) * sr2 * eps;
+                    if (sj < nloc) {
+                        atomicAdd(&cf[sj].x, -(delx * force));
+                        atomicAdd(&cf[sj].y, -(dely * force));
+                        atomicAdd(&cf[sj].z, -(delz * force));
+                    }
+                    fix += delx * force;
+                    fiy += dely * force;
+                    fiz += delz * force;
+                    if (ENERGY) {
+                        const double e = 4.0 * eps * sr6 * (sr6 - 1.0);
+                        epot += sj < nloc ? e : 0.5 * e;
+                    }
+                }
+            }
+            fx += fix;
+            fy += fiy;
+            fz += fiz;
+        }
+        atomicAdd(&cf[s].x, fx);
+        atomicAdd(&cf[s].y, fy);
+        atomicAdd(&cf[s].z, fz);
+    }
+    if (ENERGY) {
+        double t = block_sum(epot);
+        if (threadIdx.x == 0) epart[blockIdx.x] = t;
+    }
+}
+
+// half lists above this many i slots (ncl_cap * 4, about 1.05 times the atoms)
+static bool fp64_half_branch(int N, int uniform, int ncl_cap)
+{
+    return (long long)ncl_cap * CP_M > (N == 4 ? 11 << 16 : uniform ? 1 << 21 : 1 << 20);
+}
+
 template <int N, bool HALF, bool ENERGY>
 static void run_fp64(cudaStream_t s, int blocks, const int* cnt, const double4* cx,
     const Types& ty, double cutforcesq, const int* list, int ks, int cs, const int* numneigh,
-    double4* cf, double* epart)
+    double4* cf, double* epart, bool branch)
 {
+    if (HALF && branch) {
+        k_force_fp64_half<N, ENERGY><<<blocks, FP64_THREADS, 0, s>>>(cnt, cx, ty, cutforcesq,
+            list, ks, cs, numneigh, cf, epart);
+        return;
+    }
     k_force_fp64<4, N, HALF, ENERGY><<<blocks, FP64_THREADS, 0, s>>>(cnt, cx, ty, cutforcesq,
         list, ks, cs, numneigh, cf, epart);
 }
@@ -217,17 +306,18 @@ void launch_force_fp64(cudaStream_t s, int M, int N, int half, int energy, int n
     (void)M;
     // one thread per slot; the energy partials' size (force_blocks: ncl_cap * 32
     // threads) covers the blocks
-    const int blocks = force_fp64_blocks(ncl_cap);
+    const int blocks  = force_fp64_blocks(ncl_cap);
+    const bool branch = fp64_half_branch(N, ty.uniform, ncl_cap);
     if (N == 4) {
-        if (half) energy ? run_fp64<4, true, true>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart)
-                         : run_fp64<4, true, false>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart);
-        else energy ? run_fp64<4, false, true>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart)
-                    : run_fp64<4, false, false>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart);
+        if (half) energy ? run_fp64<4, true, true>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart, branch)
+                         : run_fp64<4, true, false>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart, branch);
+        else energy ? run_fp64<4, false, true>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart, branch)
+                    : run_fp64<4, false, false>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart, branch);
     } else {
-        if (half) energy ? run_fp64<8, true, true>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart)
-                         : run_fp64<8, true, false>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart);
-        else energy ? run_fp64<8, false, true>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart)
-                    : run_fp64<8, false, false>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart);
+        if (half) energy ? run_fp64<8, true, true>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart, branch)
+                         : run_fp64<8, true, false>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart, branch);
+        else energy ? run_fp64<8, false, true>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart, branch)
+                    : run_fp64<8, false, false>(s, blocks, cnt, cx, ty, cutforcesq, list, ks, cs, numneigh, cf, epart, branch);
     }
     g_launches++;
 }
