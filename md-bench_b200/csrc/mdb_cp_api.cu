@@ -1982,10 +1982,11 @@ extern "C" int mdb_cp_get_geometry(MdbCp* ctx, int* ints, double* dbls, int* ste
 
 // ---------------------------------------------------------------------------
 // Ensemble of independent cluster-pair systems (replicas of uneven size and
-// temperature). Every timestep of all members is one CUDA graph launch: the
-// graph forks one branch per member (each branch is that member's own kernel
-// sequence on its own buffers) and joins them, so the replicas' kernels run
-// concurrently and fill the GPU even when single replicas are small. Rebuild
+// temperature). Every timestep of all members is one CUDA graph launch. With
+// mixed members its kernels cover all members (batched); otherwise the graph
+// forks one branch per member (that member's own kernel sequence on its own
+// buffers) and joins them, so the replicas' kernels run concurrently and fill the
+// GPU even when single replicas are small. Rebuild
 // steps launch the members' rebuilds as one graph, read all their overflow
 // counters with one synchronisation, and redo only members that grew.
 struct MdbCpEnsemble {
@@ -2001,9 +2002,9 @@ struct MdbCpEnsemble {
     CpGraph g[16];
     std::vector<unsigned> gen;
     double* h_red = nullptr; // 4 doubles per member
-    // batched launches (every member mixed): the integrator, the ghost update
-    // and each force group run as one launch over all members; the members'
-    // own streams only carry the rebuild and the thermo sums
+    // batched launches (every member mixed): the integrator with the ghost
+    // update, each force group and each stage of a rebuild run as one launch over
+    // all members; the members' own streams only carry the thermo sums
     bool batched   = false;
     bool tables_ok = false;
     CpStepMember* d_step   = nullptr;
@@ -2023,9 +2024,8 @@ struct MdbCpEnsemble {
     int* h_flags = nullptr;
     // the check decided on the device (default; "check_on_host" 1: the host
     // reads the flags every step): one graph per step whose conditional nodes
-    // rebuild the members whose flag is up (the others update their ghosts);
-    // dstate = {stopped, steps run, steps with a rebuild} as for a single
-    // system
+    // rebuild the members whose flag is up; dstate = {stopped, steps run, steps
+    // with a rebuild} as for a single system
     bool check_host = false;
     int* dstate     = nullptr;
     int* h_dstate   = nullptr;
@@ -2034,8 +2034,8 @@ struct MdbCpEnsemble {
     cudaStream_t s_cap[2] = {nullptr, nullptr};
     long long chk_k[3]    = {0, 0, 0}; // kernels: fixed part, rebuild, force
     long long chk_steps = 0, chk_replays = 0;
-    // per member {M, N, force group, i-clusters per warp, force threads}, for
-    // the block maps that a rebuild inside the checked step graph refreshes
+    // per member {M, force group, i-clusters per warp, force threads}, for the
+    // block maps that a rebuild inside the checked step graph refreshes
     int* d_mapinfo = nullptr;
     size_t* d_goff = nullptr; // per force group: its region of the maps and size
     int* d_gnb     = nullptr;
@@ -2046,8 +2046,9 @@ struct MdbCpEnsemble {
         int nblocks;
         size_t off, off_dyn;
     };
-    // block maps of the integrator and the force groups that cover only the members' current clusters (the rest of each region is
-    // unused entries); refreshed from the counters after every rebuild.
+    // block maps of the integrator and the force groups that cover only the
+    // members' current clusters (the rest of each region is unused entries);
+    // refreshed from the counters after every rebuild.
     // Energy evaluations use the capacity maps, so that every energy partial
     // of a member is written.
     size_t off_integ_dyn = 0, dyn_begin = 0, dyn_end = 0;
@@ -2063,10 +2064,10 @@ struct MdbCpEnsemble {
 // step parts captured per ensemble: FI = final integration of the previous
 // step fused with the initial one of this step, I = initial only
 enum {
-    EG_PLAIN_FI, // FI, ghost update, force
-    EG_PLAIN_I,  // I, ghost update, force
-    EG_FRONT_FI, // FI, ghost update (a sample step follows with EG_SAMPLE)
-    EG_FRONT_I,  // I, ghost update
+    EG_PLAIN_FI, // FI with the ghost update, force
+    EG_PLAIN_I,  // I with the ghost update, force
+    EG_FRONT_FI, // FI with the ghost update (a sample step follows with EG_SAMPLE)
+    EG_FRONT_I,  // I with the ghost update
     EG_REB_FI,   // FI, updateSingleAtoms + wrap, rebuild, counters to the host
     EG_REB_I,    // I, the same
     EG_FORCE,    // force

@@ -27,9 +27,10 @@ int force_partial_blocks(int n) { return mdb_blocks(n > 0 ? n : 1, LJ_THREADS); 
 // Whether an FP64 system of n atoms shares an atom among 8 threads
 // (k_lj_fp64_shared): half lists at every size (29.5 -> 19.7 us per launch at
 // 47,840 atoms, 311 -> 235 at 702,464: more of their atomics are in flight), full
-// lists while a thread per atom leaves the chip idle (15.8 -> 5.6 us at 4,000, 20.5
-// -> 11.2 at 15,360, but 17.0 against 20.4 at 32,000, and 66 at 119,164 where a
-// thread per atom takes 41 at 143,748).
+// lists while a thread per atom leaves the chip idle. us per launch, a thread per atom
+// / 8 threads: 15.5 / 5.6 at 4,000 atoms, 15.5 / 11.5 at 16,384, 16.6 / 15.3 at
+// 23,328, 16.8 / 20.2 at 32,000, 39.0 / 65.6 at 119,164. They cross at about 25,000;
+// the line lies at 16,384, where the gain is still a quarter.
 static bool lj_fp64_shared(int half, int n) { return half || n <= 16384; }
 
 int lj_fp64_blocks(int half, int n)

@@ -128,7 +128,6 @@ namespace mdb {
 // ---- small device helpers ---------------------------------------------------
 __device__ __forceinline__ int type_of(const double4& p) { return (int)__double_as_longlong(p.w); }
 
-// read-only 32-byte position load as two 16-byte non-coherent loads of one sector
 // a double4 in one 256-bit read-only load (sm_100; p 32-byte aligned, as
 // every double4 array from cudaMalloc is)
 __device__ __forceinline__ double4 ldg4(const double4* p)
@@ -293,7 +292,8 @@ void launch_eam_fp64(cudaStream_t s, int energy, int nlocal,
     const double4* x, const int* numneigh, const int* neighbors, int ld, double cutforcesq,
     EamDev eam, const int* ghost_off, const int* counters, double* fp, double* fx,
     double* fy, double* fz, double* epart_rho, double* epart_pair);
-// mixed EAM: four threads per atom; xe (nlocal + ghost_cap) receives
+// mixed EAM: a thread per atom (rho_lanes 2: two in the density pass); xe
+// (nlocal + ghost_cap) receives
 // (position, F'(rho)) of every atom for the force pass; comp: two-sum
 // compensated force sums; returns the energy partials written per pass
 int launch_eam_mixed(cudaStream_t s, int energy, int comp, int rho_lanes, int nlocal,

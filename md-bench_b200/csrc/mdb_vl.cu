@@ -536,7 +536,9 @@ void launch_bin_order(cudaStream_t s, int nlocal, int nall_cap, int mbins, const
 // (2 bits per axis below the index). Bound by instructions: threads of a warp
 // differ in their runs and accepted candidates (15 of 32 threads active). 1M LJ
 // atoms 1,330 -> 913 us, 47,840 137 -> 111 us (half lists), Cu 131,072 227 -> 127
-// us, 3,960 130 -> 62 us against one branching test per candidate.
+// us, 3,960 130 -> 62 us against one branching test per candidate. The bound of 64
+// registers serves the large systems: the form before it took 974 us at 1M atoms, but
+// 99 at 47,840, which have few blocks.
 static constexpr int BL_THREADS = 128;
 static constexpr int BL_KEEP    = 15; // entries that wait before tiles are written
 static constexpr int BL_RING    = 48; // > BL_KEEP + 32 accepted of a mask
